@@ -74,14 +74,18 @@ rtb_status read_counters(rtb_context* ctx, long long* dst) {
 
 namespace rtb {
 namespace {
-__global__ void k_arm_abort(int* words, int generation) {
-  words[1] = generation;
-  words[2] = 0;
+// One launch for what every frame needs first: a small frame is a few launches long.
+__global__ void k_arm_abort(int* words, int generation, unsigned long long* work) {
+  if (threadIdx.x == 0) {
+    words[1] = generation;
+    words[2] = 0;
+  }
+  if (work) work[threadIdx.x] = 0ULL;
 }
 }  // namespace
 
-void arm_abort(rtb_context* ctx, cudaStream_t s) {
-  k_arm_abort<<<1, 1, 0, s>>>(ctx->d_abort, ctx->abort_generation.load());
+void arm_abort(rtb_context* ctx, cudaStream_t s, bool clear_work) {
+  k_arm_abort<<<1, 32, 0, s>>>(ctx->d_abort, ctx->abort_generation.load(), clear_work ? ctx->d_work : nullptr);
 }
 }  // namespace rtb
 
@@ -162,6 +166,7 @@ rtb_status rtb_context_destroy(rtb_context* ctx) {
     cudaFree(ctx->d_abort);
     cudaFree(ctx->d_stage);
     cudaFree(ctx->d_tail);
+    cudaFree(ctx->d_paths);
     cudaFree(ctx->d_wave);
     cudaFreeHost(ctx->h_pinned);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -329,7 +334,7 @@ rtb_status rtb_render_device(rtb_context* ctx, rtb_scene* scene, const rtb_camer
   Guard g(ctx);
   cudaStream_t sm = stream ? (cudaStream_t)stream : ctx->stream;
   ctx_acquire(ctx, sm);
-  arm_abort(ctx, sm);
+  arm_abort(ctx, sm, true);
   rtb_status s = render_frame(ctx, scene, camera, params, rgb_device, sm, false);
   ctx_release(ctx, sm);
   return s;
@@ -355,7 +360,7 @@ rtb_status rtb_render_rows_device(rtb_context* ctx, rtb_scene* scene, const rtb_
   Guard g(ctx);
   cudaStream_t sm = stream ? (cudaStream_t)stream : ctx->stream;
   ctx_acquire(ctx, sm);
-  arm_abort(ctx, sm);
+  arm_abort(ctx, sm, true);
   rtb_status s = render_frame(ctx, scene, camera, params, rgb_device, sm, false, first_row,
                               row_stride);
   ctx_release(ctx, sm);
@@ -373,7 +378,7 @@ rtb_status rtb_render_sample(rtb_context* ctx, rtb_scene* scene, const rtb_camer
   if (!d_rgb) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "output staging");
   cudaStream_t sm = ctx->stream;
   ctx_acquire(ctx, sm);
-  arm_abort(ctx, sm);
+  arm_abort(ctx, sm, true);
   rtb_status s = render_frame(ctx, scene, camera, params, d_rgb, sm, true);
   ctx_release(ctx, sm);
   if (s != RTB_OK) return s;

@@ -84,7 +84,7 @@ __device__ __forceinline__ void accumulate(GradTable& T, const AdjointArgs& a, i
   atomicAdd(a.grad_emission + 3 * m + 2, ge.z);
 }
 
-__global__ void __launch_bounds__(128, 6) k_adjoint(AdjointArgs a) {
+__global__ void __launch_bounds__(128, 6) k_adjoint(const __grid_constant__ AdjointArgs a) {
   __shared__ GradTable T;
   for (int i = threadIdx.x; i < kTable; i += blockDim.x) {
     T.key[i] = -1;
@@ -162,9 +162,10 @@ __global__ void __launch_bounds__(128, 6) k_adjoint(AdjointArgs a) {
         escaped = true;
         finished = true;
       } else {
-        float3 pos, n;
-        int mi;
-        hit_record(S, b, o, d, &pos, &n, &mi);
+        const float3 pos = add(o, mul(d, b.t));
+        const HitRecord hr = hit_record(S, b, o, d, pos);
+        const float3 n = hr.n;
+        const int mi = hr.material;
         float4 m0 = make_float4(0, 0, 0, 0), m1 = m0, m2 = m0;
         if (mi >= 0) {
           const float4* mp = S.materials + 4 * mi;

@@ -44,7 +44,7 @@ struct rtb_batch {
   std::vector<rtb::FramePlan*> frames;   // in the tuned order
   unsigned long long* d_queues = nullptr;  // one queue head per frame
   size_t queue_count = 0;
-  float* d_frame_tails = nullptr;          // one sample buffer per branch
+  float* d_frame_tails = nullptr;          // sample buffer and path slots of every branch
   size_t frame_tail_bytes = 0;
   cudaStream_t branch[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaEvent_t fork = nullptr, join[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -178,9 +178,10 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) k_batch(const BatchJo
         rad = add(rad, mulv(thr, J.S.background));
         finished = true;
       } else {
-        float3 pos, n;
-        int mi;
-        hit_record(J.S, b, o, d, &pos, &n, &mi);
+        const float3 pos = add(o, mul(d, b.t));
+        const HitRecord hr = hit_record(J.S, b, o, d, pos);
+        const float3 n = hr.n;
+        const int mi = hr.material;
         float4 m0 = make_float4(0, 0, 0, 0), m1 = m0, m2 = m0, m3 = m0;
         if (mi >= 0) {
           const float4* mp = J.S.materials + 4 * mi;
@@ -333,13 +334,14 @@ void free_frames(rtb_batch* B) {
   B->frames.clear();
 }
 
-// Frames mode: one planned frame per job in `order`, its queue head, and one sample buffer
-// per branch sized for the largest tail among that branch's frames.
+// Frames mode: one planned frame per job in `order`, its queue head, and per branch one
+// sample buffer and one set of path slots, each sized for the largest among that branch's
+// frames (the frames of a branch run one after the other).
 rtb_status plan_frames(rtb_context* ctx, rtb_batch* B, const std::vector<int>& order) {
   free_frames(B);
   int n = (int)order.size();
   int K = std::max(1, std::min(B->tuning.branches, n));
-  std::vector<size_t> branch_bytes(K, 0);
+  std::vector<size_t> branch_bytes(K, 0), path_bytes(K, 0);
   for (int i = 0; i < n; ++i) {
     const rtb_batch_job& j = B->jobs[order[i]];
     rtb_render_params p = j.params;
@@ -355,12 +357,15 @@ rtb_status plan_frames(rtb_context* ctx, rtb_batch* B, const std::vector<int>& o
     }
     B->frames.push_back(f);
     branch_bytes[i % K] = std::max(branch_bytes[i % K], rtb::frame_tail_bytes(f));
+    path_bytes[i % K] = std::max(path_bytes[i % K], rtb::frame_path_bytes(f));
   }
-  std::vector<size_t> off(K, 0);
+  std::vector<size_t> off(K, 0), path_off(K, 0);
   size_t total = 0;
   for (int b = 0; b < K; ++b) {
     off[b] = total;
     total += (branch_bytes[b] + 255) & ~(size_t)255;
+    path_off[b] = total;
+    total += (path_bytes[b] + 255) & ~(size_t)255;
   }
   if (total > B->frame_tail_bytes) {
     cudaFree(B->d_frame_tails);
@@ -380,7 +385,8 @@ rtb_status plan_frames(rtb_context* ctx, rtb_batch* B, const std::vector<int>& o
   }
   for (int i = 0; i < n; ++i) {
     float* tail = branch_bytes[i % K] ? (float*)((char*)B->d_frame_tails + off[i % K]) : nullptr;
-    bind_frame(B->frames[i], B->d_queues + i, tail, ctx->d_abort, ctx->d_work + 8);
+    bind_frame(B->frames[i], B->d_queues + i, tail, (char*)B->d_frame_tails + path_off[i % K], ctx->d_abort,
+               ctx->d_work + 8);
   }
   return RTB_OK;
 }

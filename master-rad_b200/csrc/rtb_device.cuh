@@ -116,7 +116,7 @@ __device__ __forceinline__ bool abort_raised(int* w) {
 }
 __device__ __forceinline__ bool abort_stopped(const int* w) { return *(volatile const int*)(w + 2) != 0; }
 
-__device__ __forceinline__ uint32_t hash_u32(uint32_t x) {
+__host__ __device__ __forceinline__ uint32_t hash_u32(uint32_t x) {
   x ^= x >> 17;
   x *= 0xed5ad4bbU;
   x ^= x >> 11;
@@ -285,25 +285,22 @@ __device__ __forceinline__ float affine_sphere_test(float4 r0, float4 r1, float4
 }
 
 // normalizedDirection (K:317-336) for a local direction whose squared length is not a
-// positive finite float: the unit direction and the scale back to the mapped parameter.
-// Out of line: rare, and kept out of the leaf test's code.  False when no direction exists.
-static __device__ __noinline__ bool degenerate_local_direction(float3 dir, float3* sd, float* pscale) {
+// positive finite float: the unit direction, and in .w the scale back to the mapped parameter
+// (0 when no direction exists).  Out of line: rare, and kept out of the leaf test's code.
+// Values in and out, no pointers: a variable whose address goes to a call lives in local
+// memory, and every use of it in the traversal loop would be a load or a store.
+static __device__ __noinline__ float4 degenerate_local_direction(float3 dir) {
   float l2 = dot(dir, dir);
-  if (isfinite(l2) && fabsf(l2 - 1.0f) <= 2.0e-6f) {
-    *sd = dir;
-    *pscale = 1.0f;
-    return true;
-  }
+  if (isfinite(l2) && fabsf(l2 - 1.0f) <= 2.0e-6f) return make_float4(dir.x, dir.y, dir.z, 1.0f);
   float scale = fmaxf(fabsf(dir.x), fmaxf(fabsf(dir.y), fabsf(dir.z)));
-  if (!(scale > 0.0f) || !isfinite(scale)) return false;
+  if (!(scale > 0.0f) || !isfinite(scale)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float3 sc = v3(dir.x / scale, dir.y / scale, dir.z / scale);
   float sl = sqrtf(dot(sc, sc));
   float dl = scale * sl;
   float inv = 1.0f / dl;
-  if (!(inv > 0.0f) || !isfinite(inv)) return false;
-  *sd = mul(sc, 1.0f / sl);
-  *pscale = inv;
-  return true;
+  if (!(inv > 0.0f) || !isfinite(inv)) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float3 sd = mul(sc, 1.0f / sl);
+  return make_float4(sd.x, sd.y, sd.z, inv);
 }
 
 // The unit-sphere part of traceAffineSphere on the mapped ray.
@@ -314,7 +311,10 @@ __device__ __forceinline__ float affine_sphere_local(const AffineRay& ar, const 
   float3 sd = ar.ld;
   float pscale = 1.0f;
   if (!(solve_a > 0.0f) || !isfinite(solve_a)) {
-    if (!degenerate_local_direction(ar.ld, &sd, &pscale)) return CUDART_INF_F;
+    const float4 g = degenerate_local_direction(ar.ld);
+    if (!(g.w > 0.0f)) return CUDART_INF_F;
+    sd = v3(g.x, g.y, g.z);
+    pscale = g.w;
     solve_a = 1.0f;
   }
   float scaled_after = after_local / pscale;
@@ -368,27 +368,26 @@ __device__ __forceinline__ float affine_box_local(const AffineRay& ar, const flo
 // ---------------------------------------------------------------- closest hit
 struct Best {
   float t;
-  int order;
   int type;   // PrimType of the winner, -1 for none
   int index;  // storage index of the winner (plane index for planes)
 };
+__device__ __forceinline__ Best no_hit() { return Best{1e30f, -1, -1}; }
 
+// Global order of a primitive (a plane's storage index is its insertion index).
 __device__ __forceinline__ int order_of(const DevScene& S, int type, int index) {
-  return S.order_base[type] + __ldg(S.orig[type] + index);
+  return S.order_base[type] + (type == kPlane ? index : __ldg(S.orig[type] + index));
 }
 
 // Offers a candidate distance: the closest hit is the lexicographic minimum of
-// (distance, global order), the contract of tracePrimitiveRef (K:772-806).
+// (distance, global order), the contract of tracePrimitiveRef (K:772-806).  The orders are
+// read only where two distances are equal.
 __device__ __forceinline__ void offer(const DevScene& S, Best& b, float t, int type, int index) {
   if (t < b.t) {
     b.t = t;
     b.type = type;
     b.index = index;
-    b.order = order_of(S, type, index);
   } else if (t == b.t && t != CUDART_INF_F) {
-    int o = order_of(S, type, index);
-    if (o < b.order) {
-      b.order = o;
+    if (b.type < 0 || order_of(S, type, index) < order_of(S, b.type, b.index)) {
       b.type = type;
       b.index = index;
     }
@@ -396,7 +395,7 @@ __device__ __forceinline__ void offer(const DevScene& S, Best& b, float t, int t
 }
 
 struct TraceCounters {
-  unsigned long long aabb, prim, type[5], internal, leaf, homo, mixed, maxstack, overflow;
+  unsigned long long rays, aabb, prim, type[5], internal, leaf, homo, mixed, maxstack, overflow;
 };
 
 template <bool METRICS>
@@ -464,191 +463,196 @@ __device__ __forceinline__ float prune_limit(float t) {
   return isfinite(t) ? fmaf(t, 1.0000015f, 1.0e-6f) : t;
 }
 
+// The exhaustive paths, out of line and by value (see degenerate_local_direction): the best
+// hit over every reference or every primitive, starting from `b`.
 template <bool METRICS>
-__device__ __noinline__ void test_all_refs(const DevScene& S, float3 o, float3 d, float dd, Best& b,
+__device__ __noinline__ Best test_all_refs(const DevScene& S, float3 o, float3 d, float dd, Best b,
                                            TraceCounters* c) {
+#pragma unroll 1
   for (int i = 0; i < S.ref_count; ++i) {
     int ref = __ldg(S.refs + i);
     test_ref<METRICS>(S, (int)((unsigned)ref >> kTypeShift), ref & kIndexMask, o, d, dd, b, c);
   }
+  return b;
 }
 
 template <bool METRICS>
-__device__ __noinline__ void test_all_primitives(const DevScene& S, float3 o, float3 d, float dd,
-                                                 Best& b, TraceCounters* c) {
+__device__ __noinline__ Best test_all_primitives(const DevScene& S, float3 o, float3 d, float dd, Best b,
+                                                 TraceCounters* c) {
+#pragma unroll 1
   for (int t = 0; t < 4; ++t)
+#pragma unroll 1
     for (int i = 0; i < S.count[t]; ++i) test_ref<METRICS>(S, t, i, o, d, dd, b, c);
+  return b;
 }
 
-// Closest hit of one ray against the resident scene (traceClosest, K:963-1020): the BVH
-// (or every bounded primitive in linear mode), then the planes.  Returns true on a hit.
+// ---- traversal state of one lane's ray
 //
-// Warp-cooperative: all 32 lanes of the warp call it together (lanes without a ray pass
-// active = false).  The traversal loop is warp-uniform -- each iteration every lane that
-// still walks processes one node: it tests both child boxes, records the leaf children it
-// reached (a lane holds up to two recorded pairs, walking on after the first), then picks
-// the next interior node; once at most kLeafPostponeLanes lanes can still walk, the
-// recorded leaves of all lanes are tested together -- and the loop condition is a warp
-// vote, so divergent lanes reconverge once per node.  Every lane
-// takes part in the votes, also where lanes hold different scenes and only some of them
-// have a tree (the batch kernel's lanes may belong to different jobs).
+// walk_node processes one node for a lane that can walk: both child boxes are tested, the
+// leaf children it reached are recorded (a lane holds up to two recorded pairs and walks on
+// after the first), and the next interior node is picked or popped.  test_recorded tests a
+// lane's recorded leaves.  The warp decides by ballots which of the two runs next, so that
+// the expensive primitive tests run with many lanes at once (leaf postponing); the prune
+// limits a lane uses while its leaves wait are from its older (farther) best hit, which
+// only visits more nodes, never fewer: the closest hit is unchanged.
 //
 // SDEPTH > 0: the first SDEPTH stack entries live in shared memory, in the caller's column
 // `ss` of an [SDEPTH][SSTRIDE] int2 array (node, entry distance bits), so that the entries
 // a traversal uses most stay out of local memory; deeper entries spill to local memory.
-template <bool METRICS, int SDEPTH = 0, int SSTRIDE = 1>
-__device__ bool trace_closest(const DevScene& S, float3 o, float3 d, bool active, Best& b,
-                              TraceCounters* c, int* overflow_flag, int2* ss = nullptr) {
-  b.t = 1e30f;
-  b.order = 0x7FFFFFFF;
-  b.type = -1;
-  b.index = -1;
-  float dd = dot(d, d);
-  const bool bvh = S.use_bvh && S.node_count > 0;
-  {
-    float3 inv = v3(d.x != 0.0f ? 1.0f / d.x : 1e30f, d.y != 0.0f ? 1.0f / d.y : 1e30f,
-                    d.z != 0.0f ? 1.0f / d.z : 1e30f);
-    int stack[kStackSize - SDEPTH];
-    float estack[kStackSize - SDEPTH];
-    int sp = 0;
-    int node = (active && bvh) ? 0 : -1;
-    bool overflow = false;
+//
+// The entries in local memory are an array of their own, outside Walk: an array indexed at
+// run time would keep the whole struct it belongs to in local memory.
+template <int SDEPTH>
+struct WalkStack {
+  int node[kStackSize - SDEPTH];
+  float entry[kStackSize - SDEPTH];
+};
+struct Walk {
+  int node;   // the next node, -1: none left
+  int sp;
+  // Recorded leaves: up to two nodes whose leaf children the ray reached, as
+  // node << 2 | (child 0 reached) | (child 1 reached) << 1; 0 for none.  The test reads the
+  // node's links again (16 bytes, in L1 as a rule), which costs less than the eight words
+  // of links would cost in registers all through the walk.
+  unsigned p0, p1;
+  int budget;
+  bool overflow;
+  __device__ __forceinline__ void begin(const DevScene& S, bool active) {
+    node = active ? 0 : -1;
+    sp = 0;
+    p0 = p1 = 0u;
+    overflow = false;
     // A tree visits each node at most once per ray; the cap only matters for malformed
     // (cyclic) caller-supplied trees, which then take the exhaustive path.
-    int budget = S.node_count + 8;
-    // Leaf postponing with speculative walking: a lane that reaches leaf children records
-    // them and walks on to its next leaf children (two recorded pairs at most, then it
-    // waits); the warp tests the recorded leaves together once at most kLeafPostponeLanes
-    // lanes can still walk, so the expensive primitive tests run with many lanes at once.
-    // The prune limits a lane uses while its leaves wait are from its older (farther) best
-    // hit, which only visits more nodes, never fewer: the closest hit is unchanged.
-    int pfirst0 = 0, pmeta0 = 0, pfirst1 = 0, pmeta1 = 0;
-    int qfirst0 = 0, qmeta0 = 0, qfirst1 = 0, qmeta1 = 0;
-    int npend = 0;
-    bool pend = false;  // this lane cannot take another leaf pair
-    while (true) {
-      pend = npend >= 2;
-      // lanes that can walk, lanes with recorded leaves (a lane that cannot walk has some)
-      const unsigned walk = __ballot_sync(0xFFFFFFFFu, node >= 0 && !pend);
-      const unsigned waiting = __ballot_sync(0xFFFFFFFFu, npend > 0);
-      if ((walk | waiting) == 0u) break;
-      if (__popc(walk) <= kLeafPostponeLanes && waiting != 0u) {
-        int c0 = npend >= 1 ? (pmeta0 & 0xFFFFFF) : 0, c1 = npend >= 1 ? (pmeta1 & 0xFFFFFF) : 0;
-        int c2 = npend >= 2 ? (qmeta0 & 0xFFFFFF) : 0, c3 = npend >= 2 ? (qmeta1 & 0xFFFFFF) : 0;
-        int e1 = c0 + c1, e2 = e1 + c2, e3 = e2 + c3;
-        for (int k = 0; k < e3; ++k) {
-          int first, meta, off;
-          if (k < c0) {
-            first = pfirst0, meta = pmeta0, off = k;
-          } else if (k < e1) {
-            first = pfirst1, meta = pmeta1, off = k - c0;
-          } else if (k < e2) {
-            first = qfirst0, meta = qmeta0, off = k - e1;
-          } else {
-            first = qfirst1, meta = qmeta1, off = k - e2;
-          }
-          int code = meta >> 24;
-          int ref = __ldg(S.refs + first + off);
-          int type = code == 4 ? (int)((unsigned)ref >> kTypeShift) : code;
-          test_ref<METRICS>(S, type, ref & kIndexMask, o, d, dd, b, c);
-        }
-        npend = 0;
-        continue;
-      }
-      if (node >= 0 && !pend) {
-        const float4* np = S.nodes + 4 * node;
-        float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2);
-        int4 n3 = __ldg(reinterpret_cast<const int4*>(np + 3));
-        float lim = prune_limit(b.t);
-        float e0 = child_entry(n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, o, inv, lim);
-        float e1 = child_entry(n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, o, inv, lim);
-        if (METRICS) {
-          c->internal++;
-          c->aabb += 2;
-        }
-        bool swap = e1 < e0;
-        float en = swap ? e1 : e0, ef = swap ? e0 : e1;
-        int ln = swap ? n3.y : n3.x, lf = swap ? n3.x : n3.y;
-        int mn = swap ? n3.w : n3.z, mf = swap ? n3.z : n3.w;
-        bool hn = en != CUDART_INF_F, hf = ef != CUDART_INF_F;
-        // Leaf children: one loop over the near leaf's references then the far leaf's.
-        // Testing the far leaf even if the near one already beats it is harmless: the
-        // closest hit is a minimum over primitives.
-        int first0 = (hn && ln < 0) ? ~ln : 0, count0 = (hn && ln < 0) ? (mn & 0xFFFFFF) : 0;
-        int first1 = (hf && lf < 0) ? ~lf : 0, count1 = (hf && lf < 0) ? (mf & 0xFFFFFF) : 0;
-        int code0 = mn >> 24, code1 = mf >> 24;
-        if (METRICS) {
-          if (count0 || (hn && ln < 0)) {
-            c->leaf++;
-            if (code0 == 4) c->mixed++; else c->homo++;
-          }
-          if (count1 || (hf && lf < 0)) {
-            c->leaf++;
-            if (code1 == 4) c->mixed++; else c->homo++;
-          }
-        }
-        if (count0 + count1 > 0) {
-          if (npend == 0) {
-            pfirst0 = first0;
-            pmeta0 = count0 | (code0 << 24);
-            pfirst1 = first1;
-            pmeta1 = count1 | (code1 << 24);
-          } else {
-            qfirst0 = first0;
-            qmeta0 = count0 | (code0 << 24);
-            qfirst1 = first1;
-            qmeta1 = count1 | (code1 << 24);
-          }
-          npend++;
-        }
-        float plim = prune_limit(b.t);
-        int next = (hn && ln >= 0) ? ln : -1;
-        if (hf && lf >= 0 && ef <= plim) {
-          if (next < 0) {
-            next = lf;
-          } else if (sp < kStackSize) {
-            if (SDEPTH > 0 && sp < SDEPTH) {
-              ss[sp * SSTRIDE] = make_int2(lf, __float_as_int(ef));
-            } else {
-              stack[sp - SDEPTH] = lf;
-              estack[sp - SDEPTH] = ef;
-            }
-            sp++;
-            if (METRICS && (unsigned long long)sp > c->maxstack) c->maxstack = sp;
-          } else {
-            overflow = true;
-          }
-        }
-        // Pop the next subtree still closer than the current hit.
-        while (next < 0 && sp > 0) {
-          --sp;
-          int sn;
-          float se;
-          if (SDEPTH > 0 && sp < SDEPTH) {
-            int2 e = ss[sp * SSTRIDE];
-            sn = e.x;
-            se = __int_as_float(e.y);
-          } else {
-            sn = stack[sp - SDEPTH];
-            se = estack[sp - SDEPTH];
-          }
-          if (se <= plim) next = sn;
-        }
-        if (--budget < 0) overflow = true;
-        node = overflow ? -1 : next;
-      }
+    budget = S.node_count + 8;
+  }
+  __device__ __forceinline__ bool can_walk() const { return node >= 0 && p1 == 0u; }
+  __device__ __forceinline__ bool waiting() const { return p0 != 0u; }
+};
+
+// The reciprocal direction of the node tests.
+__device__ __forceinline__ float3 ray_inverse(float3 d) {
+  return v3(d.x != 0.0f ? 1.0f / d.x : 1e30f, d.y != 0.0f ? 1.0f / d.y : 1e30f,
+            d.z != 0.0f ? 1.0f / d.z : 1e30f);
+}
+
+template <bool METRICS>
+__device__ __forceinline__ void test_recorded(const DevScene& S, Walk& w, float3 o, float3 d,
+                                              float dd, Best& b, TraceCounters* c) {
+  // A leaf child's first reference and count | (type code << 24), count 0 where not reached.
+  int f0 = 0, f1 = 0, f2 = 0, f3 = 0, m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+  if (w.p0 != 0u) {
+    const int4 n = __ldg(reinterpret_cast<const int4*>(S.nodes + (w.p0 & ~3u) + 3));
+    if (w.p0 & 1) f0 = ~n.x, m0 = n.z;
+    if (w.p0 & 2) f1 = ~n.y, m1 = n.w;
+  }
+  if (w.p1 != 0u) {
+    const int4 n = __ldg(reinterpret_cast<const int4*>(S.nodes + (w.p1 & ~3u) + 3));
+    if (w.p1 & 1) f2 = ~n.x, m2 = n.z;
+    if (w.p1 & 2) f3 = ~n.y, m3 = n.w;
+  }
+  const int c0 = m0 & 0xFFFFFF, c1 = m1 & 0xFFFFFF, c2 = m2 & 0xFFFFFF, c3 = m3 & 0xFFFFFF;
+  int e1 = c0 + c1, e2 = e1 + c2, e3 = e2 + c3;
+#pragma unroll 1
+  for (int k = 0; k < e3; ++k) {
+    int first, meta, off;
+    if (k < c0) {
+      first = f0, meta = m0, off = k;
+    } else if (k < e1) {
+      first = f1, meta = m1, off = k - c0;
+    } else if (k < e2) {
+      first = f2, meta = m2, off = k - e1;
+    } else {
+      first = f3, meta = m3, off = k - e2;
     }
-    if (overflow) {
-      if (overflow_flag) atomicAdd(overflow_flag, 1);
-      if (METRICS) c->overflow++;
-      test_all_refs<METRICS>(S, o, d, dd, b, c);
+    int code = meta >> 24;
+    int ref = __ldg(S.refs + first + off);
+    int type = code == 4 ? (int)((unsigned)ref >> kTypeShift) : code;
+    test_ref<METRICS>(S, type, ref & kIndexMask, o, d, dd, b, c);
+  }
+  w.p0 = w.p1 = 0u;
+}
+
+template <bool METRICS, int SDEPTH, int SSTRIDE>
+__device__ __forceinline__ void walk_node(const DevScene& S, Walk& w, WalkStack<SDEPTH>& ws, float3 o,
+                                          float3 inv, const Best& b, TraceCounters* c, int2* ss) {
+  const float4* np = S.nodes + 4 * w.node;
+  float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2);
+  int4 n3 = __ldg(reinterpret_cast<const int4*>(np + 3));
+  const float lim = prune_limit(b.t);
+  float e0 = child_entry(n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, o, inv, lim);
+  float e1 = child_entry(n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, o, inv, lim);
+  if (METRICS) {
+    c->internal++;
+    c->aabb += 2;
+  }
+  const bool h0 = e0 != CUDART_INF_F, h1 = e1 != CUDART_INF_F;
+  const int leaves = (h0 && n3.x < 0 ? 1 : 0) | (h1 && n3.y < 0 ? 2 : 0);
+  if (METRICS) {
+    if (leaves & 1) {
+      c->leaf++;
+      if (n3.z >> 24 == 4) c->mixed++; else c->homo++;
+    }
+    if (leaves & 2) {
+      c->leaf++;
+      if (n3.w >> 24 == 4) c->mixed++; else c->homo++;
     }
   }
-  if (active && !bvh) test_all_primitives<METRICS>(S, o, d, dd, b, c);
-  if (!active) return false;
-  // tracePlane, K:708-734: a plane wins only when strictly closer.
+  if (leaves) {
+    const unsigned rec = (unsigned)w.node << 2 | (unsigned)leaves;
+    if (w.p0 == 0u) w.p0 = rec; else w.p1 = rec;
+  }
+  // Interior children reached: the nearer is next, the farther goes on the stack.
+  const int i0 = h0 ? n3.x : -1, i1 = h1 ? n3.y : -1;
+  const bool swap = e1 < e0;
+  int next = swap ? i1 : i0;
+  const int far = swap ? i0 : i1;
+  if (far >= 0) {
+    if (next < 0) {
+      next = far;
+    } else if (w.sp < kStackSize) {
+      const float ef = swap ? e0 : e1;
+      if (SDEPTH > 0 && w.sp < SDEPTH) {
+        ss[w.sp * SSTRIDE] = make_int2(far, __float_as_int(ef));
+      } else {
+        ws.node[w.sp - SDEPTH] = far;
+        ws.entry[w.sp - SDEPTH] = ef;
+      }
+      w.sp++;
+      if (METRICS && (unsigned long long)w.sp > c->maxstack) c->maxstack = w.sp;
+    } else {
+      w.overflow = true;
+    }
+  }
+  // Pop the next subtree still closer than the current hit.
+  while (next < 0 && w.sp > 0) {
+    --w.sp;
+    int sn;
+    float se;
+    if (SDEPTH > 0 && w.sp < SDEPTH) {
+      int2 e = ss[w.sp * SSTRIDE];
+      sn = e.x;
+      se = __int_as_float(e.y);
+    } else {
+      sn = ws.node[w.sp - SDEPTH];
+      se = ws.entry[w.sp - SDEPTH];
+    }
+    if (se <= lim) next = sn;
+  }
+  if (--w.budget < 0) w.overflow = true;
+  w.node = w.overflow ? -1 : next;
+}
+
+// tracePlane, K:708-734: a plane wins only when strictly closer.
+template <bool METRICS>
+__device__ __forceinline__ void test_planes(const DevScene& S, float3 o, float3 d, Best& b,
+                                            TraceCounters* c) {
+  if (S.plane_count <= 0) return;
+  float4 next = __ldg(S.planes);  // one plane ahead: the loop does not wait for its loads
+#pragma unroll 1
   for (int i = 0; i < S.plane_count; ++i) {
-    float4 p = __ldg(S.planes + i);
+    const float4 p = next;
+    if (i + 1 < S.plane_count) next = __ldg(S.planes + i + 1);
     float3 pn = v3(p.x, p.y, p.z);
     float den = dot(pn, d);
     if (den == 0.0f) continue;
@@ -657,12 +661,54 @@ __device__ bool trace_closest(const DevScene& S, float3 o, float3 d, bool active
     b.t = t;
     b.type = kPlane;
     b.index = i;
-    b.order = S.order_base[kPlane] + i;
   }
   if (METRICS) {
     c->prim += S.plane_count;
     c->type[2] += S.plane_count;
   }
+}
+
+// Closest hit of one ray against the resident scene (traceClosest, K:963-1020): the BVH
+// (or every bounded primitive in linear mode), then the planes.  Returns true on a hit.
+//
+// Warp-cooperative: all 32 lanes of the warp call it together (lanes without a ray pass
+// active = false).  The traversal loop is warp-uniform -- each iteration every lane that
+// can walk processes one node; once at most kLeafPostponeLanes lanes can still walk, the
+// recorded leaves of all lanes are tested together -- and the loop condition is a warp
+// vote, so divergent lanes reconverge once per node.  Every lane takes part in the votes,
+// also where lanes hold different scenes and only some of them have a tree (the batch
+// kernel's lanes may belong to different jobs).
+template <bool METRICS, int SDEPTH = 0, int SSTRIDE = 1>
+__device__ bool trace_closest(const DevScene& S, float3 o, float3 d, bool active, Best& b,
+                              TraceCounters* c, int* overflow_flag, int2* ss = nullptr) {
+  b = no_hit();
+  float dd = dot(d, d);
+  const bool bvh = S.use_bvh && S.node_count > 0;
+  {
+    const float3 inv = ray_inverse(d);
+    Walk w;
+    WalkStack<SDEPTH> ws;
+    w.begin(S, active && bvh);
+    while (true) {
+      // lanes that can walk, lanes with recorded leaves (a lane that cannot walk has some)
+      const unsigned walk = __ballot_sync(0xFFFFFFFFu, w.can_walk());
+      const unsigned waiting = __ballot_sync(0xFFFFFFFFu, w.waiting());
+      if ((walk | waiting) == 0u) break;
+      if (__popc(walk) <= kLeafPostponeLanes && waiting != 0u) {
+        test_recorded<METRICS>(S, w, o, d, dd, b, c);
+        continue;
+      }
+      if (w.can_walk()) walk_node<METRICS, SDEPTH, SSTRIDE>(S, w, ws, o, inv, b, c, ss);
+    }
+    if (w.overflow) {
+      if (overflow_flag) atomicAdd(overflow_flag, 1);
+      if (METRICS) c->overflow++;
+      b = test_all_refs<METRICS>(S, o, d, dd, b, METRICS ? c : nullptr);
+    }
+  }
+  if (active && !bvh) b = test_all_primitives<METRICS>(S, o, d, dd, b, METRICS ? c : nullptr);
+  if (!active) return false;
+  test_planes<METRICS>(S, o, d, b, c);
   return b.type >= 0;
 }
 
@@ -686,12 +732,15 @@ __device__ __forceinline__ int plane_material(const float* p, float3 hp) {
   return (int)g[6];
 }
 
-// The full hit record of the winner: position o + d t, the reference's normal for that
-// primitive type, and its material index.
-static __device__ __noinline__ void hit_record(const DevScene& S, const Best& b, float3 o, float3 d,
-                                           float3* pos, float3* n, int* material) {
+// The full hit record of the winner: the reference's normal for that primitive type and its
+// material index; `pos` is the position o + d t.
+struct HitRecord {
+  float3 n;
+  int material;
+};
+__device__ __forceinline__ HitRecord hit_record_inline(const DevScene& S, const Best& b, float3 o, float3 d,
+                                                       float3 pos) {
   float dd = dot(d, d);
-  *pos = add(o, mul(d, b.t));
   float3 nn = v3(0.0f, 0.0f, 0.0f);
   int m = -1;
   int i = b.index;
@@ -719,14 +768,19 @@ static __device__ __noinline__ void hit_record(const DevScene& S, const Best& b,
     case kPlane: {
       float4 p = __ldg(S.planes + i);
       nn = v3(p.x, p.y, p.z);
-      m = plane_material(S.plane_full + 26 * i, *pos);
+      m = plane_material(S.plane_full + 26 * i, pos);
       break;
     }
     default:
       break;
   }
-  *n = nn;
-  *material = m;
+  return HitRecord{nn, m};
+}
+
+// Out of line for the kernels that trace and shade in one loop: kept out of its code.
+static __device__ __noinline__ HitRecord hit_record(const DevScene& S, Best b, float3 o, float3 d,
+                                                float3 pos) {
+  return hit_record_inline(S, b, o, d, pos);
 }
 
 }  // namespace rtb

@@ -41,9 +41,15 @@ struct rtb_context {
   // Per-sample radiance of the frame's last pixels (rendered one sample per lane).
   float* d_tail = nullptr;
   size_t tail_bytes = 0;
+  // Path slots of the frame kernel's blocks.
+  void* d_paths = nullptr;
+  size_t path_bytes = 0;
   // Path state of the wavefront form, grown to the largest frame rendered in that form.
   void* d_wave = nullptr;
   size_t wave_bytes = 0;
+  // Blocks per SM of each frame kernel (metrics, stack depth, form) on this context's device;
+  // 0: its attributes are not set there yet.
+  int frame_blocks[2][3][2] = {};
   int render_launches = 0;  // kernels the last render_frame launched
 };
 
@@ -78,7 +84,8 @@ inline void ctx_release(rtb_context* ctx, cudaStream_t s) {
 // Enqueues, on `s`, the write of the current abort generation as the submitted work's own
 // and the clearing of the stopped word.  Every launch of a persistent kernel is preceded by
 // it (outside any graph capture: the generation is a kernel argument).
-void arm_abort(rtb_context* ctx, cudaStream_t s);
+// With clear_work it also zeroes d_work, for render_frame.
+void arm_abort(rtb_context* ctx, cudaStream_t s, bool clear_work = false);
 
 // Status helpers.
 rtb_status fail(rtb_context* ctx, rtb_status s, const std::string& msg);
@@ -97,7 +104,7 @@ void scene_free(rtb_scene* s, cudaStream_t stream);
 
 // rtb_render.cu
 // Rows row0, row0 + row_stride, ... of the frame, packed densely into d_rgb (0, 1: the
-// whole frame).
+// whole frame).  The caller has armed the abort words and cleared d_work on `stream`.
 rtb_status render_frame(rtb_context* ctx, rtb_scene* scene, const rtb_camera* cam,
                         const rtb_render_params* p, float* d_rgb, cudaStream_t stream,
                         bool timed, int row0 = 0, int row_stride = 1);
@@ -107,8 +114,9 @@ rtb_status render_frame_wavefront(rtb_context* ctx, rtb_scene* scene, const rtb_
 // One frame's launch, planned apart from where it runs (the batch's frames mode launches
 // many into one graph).  plan_frame validates and sizes; bind_frame gives it a queue head
 // (zeroed before launch), a sample buffer of frame_tail_bytes (nullptr: no single-sample
-// tail), the abort flag and 14 counters; launch_frame enqueues its kernels and returns how
-// many.
+// tail), path slots of frame_path_bytes, the abort flag and 14 counters; launch_frame enqueues
+// its kernels and returns how many.  Frames that may run at the same time need buffers of
+// their own.
 struct FramePlan;
 FramePlan* new_frame_plan();
 void delete_frame_plan(FramePlan* f);
@@ -118,7 +126,8 @@ rtb_status plan_frame(rtb_context* ctx, rtb_scene* scene, const rtb_camera* cam,
                       const rtb_render_params* p, float* d_rgb, FramePlan* f, int row0 = 0,
                       int row_stride = 1, int tail_per_thread = 0);
 size_t frame_tail_bytes(const FramePlan* f);
-void bind_frame(FramePlan* f, unsigned long long* queue, float* tail, int* abort_flag,
+size_t frame_path_bytes(const FramePlan* f);
+void bind_frame(FramePlan* f, unsigned long long* queue, float* tail, void* paths, int* abort_flag,
                 unsigned long long* counters);
 int launch_frame(const FramePlan* f, cudaStream_t stream);
 // Closest-hit launch without a context (no counters, no allocation).

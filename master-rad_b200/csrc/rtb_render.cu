@@ -1,14 +1,14 @@
 // Path-tracing and closest-hit kernels.
 //
 // Render: one persistent launch per frame (the reference issues one launch per sample and
-// tile, GpuRayTracer.java:356-376).  Each resident thread owns one pixel at a time and runs
-// its samples in order, one path segment per loop iteration; a lane whose path ends starts
-// the next sample (or fetches the next pixel from a warp-aggregated queue) while the other
-// lanes continue, so warps stay full across uneven path lengths.  The per-pixel sum is the
-// reference's FP32 running sum over samples 0..spp-1 scaled by 1/spp after the last one
-// (GpuKernelSources.java:1284-1293), and each sample consumes the reference's random
-// stream (seed K:1231-1254, jitter and camera K:1256-1264, tracePath K:1061-1165), so the
-// image matches the reference's renderKernel bit for bit under the same arithmetic.
+// tile, GpuRayTracer.java:356-376), which takes work items from a warp-aggregated queue: a
+// whole pixel, its samples in order, or a single sample.  A path that ends is followed by its
+// pixel's next sample or the queue's next item while the others continue, so warps stay full
+// across uneven path lengths.  The per-pixel sum is the reference's FP32 running sum over
+// samples 0..spp-1 scaled by 1/spp after the last one (GpuKernelSources.java:1284-1293), and
+// each sample consumes the reference's random stream (seed K:1231-1254, jitter and camera
+// K:1256-1264, tracePath K:1061-1165), so the image matches the reference's renderKernel bit
+// for bit under the same arithmetic.
 //
 // The frame's last pixels (about four per resident thread, or all of a small frame) are
 // handed out one sample per queue item instead, so the end of the frame does not wait on
@@ -23,13 +23,18 @@ namespace {
 struct RenderArgs {
   DevScene S;
   float3 cam_pos, cam_f, cam_r, cam_u;
-  int width, height, spp, max_depth, frame_index;
-  unsigned long long frame_seed;
+  int width, height, spp, max_depth;
+  float aspect, step_x, step_y;    // width / height, 2 / width, 2 / height
+  float inv_spp;                   // 1 / spp
+  uint32_t frame_hash;             // the frame's part of every pixel's seed
+  unsigned long long spp_magic, width_magic;  // of fast_div
   float* out;
   long long pixels;                // pixels of the output (the frame, or a set of its rows)
   int row0, row_stride;            // output row k is frame row row0 + k * row_stride
   long long split;                 // pixels [split, pixels) are queued one sample per item
   long long items;                 // split + (pixels - split) * spp queue items
+  void* paths;                     // the blocks' path slots
+  int slots;                       // path slots a block uses, at most kSlotsPerBlock
   float* tail;                     // RGB of each tail item, item - split order
   unsigned long long* queue;       // work queue head
   int* abort_flag;                 // the context's abort words (abort_raised)
@@ -54,13 +59,16 @@ static __device__ __noinline__ float3 refract_dir(float3 incoming, float3 n, flo
   return normalize_safe(sub(mul(n, c1 - sq * ri), i));
 }
 
-__device__ __forceinline__ uint32_t pixel_base_seed(unsigned long long frame_seed, int frame_index,
-                                                    uint32_t pixel) {  // K:1231-1236
-  uint32_t s = hash_u32((uint32_t)(frame_seed & 0xFFFFFFFFULL));
-  s ^= hash_u32((uint32_t)(frame_seed >> 32));
-  s ^= hash_u32((uint32_t)frame_index);
-  s ^= hash_u32(pixel);
-  return hash_u32(s);
+// K:1231-1236; the part that every pixel of the frame shares is hashed on the host.
+__device__ __forceinline__ uint32_t pixel_base_seed(uint32_t frame_hash, uint32_t pixel) {
+  return hash_u32(frame_hash ^ hash_u32(pixel));
+}
+
+// n / d for 32-bit n by the divisor's magic number floor((2^64 - 1) / d) + 1 (0 for d = 1): the
+// quotient n M / 2^64 exceeds n / d by less than n / 2^64 < 1 / d, so its floor is exact.
+inline unsigned long long div_magic(unsigned d) { return ~0ULL / d + 1ULL; }
+__device__ __forceinline__ unsigned fast_div(unsigned n, unsigned long long magic) {
+  return magic ? (unsigned)__umul64hi((unsigned long long)n, magic) : n;
 }
 
 // One path segment after its closest-hit query (tracePath loop body, K:1098-1162): the
@@ -76,9 +84,10 @@ __device__ __forceinline__ bool shade_segment(const DevScene& S, bool hit, const
     rad = add(rad, mulv(thr, S.background));
     return true;
   }
-  float3 pos, n;
-  int mi;
-  hit_record(S, b, o, d, &pos, &n, &mi);
+  const float3 pos = add(o, mul(d, b.t));
+  const HitRecord hr = hit_record_inline(S, b, o, d, pos);
+  const float3 n = hr.n;
+  const int mi = hr.material;
   float4 m0 = make_float4(0, 0, 0, 0), m1 = m0, m2 = m0, m3 = m0;
   if (mi >= 0) {
     const float4* mp = S.materials + 4 * mi;
@@ -100,7 +109,10 @@ __device__ __forceinline__ bool shade_segment(const DevScene& S, bool hit, const
     float z = rand01(&rng) * 2.0f - 1.0f;
     float t = rand01(&rng) * 2.0f * CUDART_PI_F;
     float r = sqrtf(fmaxf(0.0f, 1.0f - z * z));
-    nd = add(v3(r * cosf(t), r * sinf(t), z), n);
+    // one range reduction; equal to sinf and cosf bit for bit on all 2^24 values of t
+    float st, ct2;
+    sincosf(t, &st, &ct2);
+    nd = add(v3(r * ct2, r * st, z), n);
     wc = divs(cd, pc);
   } else if (xi < wd + wr) {
     float pc = wr / sum;
@@ -120,190 +132,415 @@ __device__ __forceinline__ bool shade_segment(const DevScene& S, bool hit, const
 
 // The camera ray of sample `so` of pixel (x, y) and its random stream (renderKernel
 // prologue, K:1251-1264), for the wavefront kernels (k_render's prologue is inline).
-__device__ __forceinline__ void camera_sample(const RenderArgs& a, int x, int y, int so,
-                                              uint32_t base_seed, uint32_t& rng, float3& o,
-                                              float3& d) {
-  uint32_t seed = base_seed ^ hash_u32((uint32_t)so);
+__device__ __forceinline__ void camera_sample(const RenderArgs& a, int x, int y, int so, uint32_t& rng,
+                                              float3& o, float3& d) {
+  uint32_t seed = pixel_base_seed(a.frame_hash, (uint32_t)y * (uint32_t)a.width + (uint32_t)x) ^ hash_u32((uint32_t)so);
   seed ^= hash_u32((uint32_t)(so * 0x9E3779B9u));
   rng = hash_u32(seed);
-  const float aspect = (float)a.width / (float)a.height;
   float jx = rand01(&rng) - 0.5f;
   float jy = rand01(&rng) - 0.5f;
-  float u = ((((float)x + 0.5f) + jx) * (2.0f / (float)a.width) - 1.0f) * aspect;
-  float v = 1.0f - ((((float)y + 0.5f) + jy) * (2.0f / (float)a.height));
+  float u = ((((float)x + 0.5f) + jx) * a.step_x - 1.0f) * a.aspect;
+  float v = 1.0f - ((((float)y + 0.5f) + jy) * a.step_y);
   o = a.cam_pos;
   d = add(add(a.cam_f, mul(a.cam_r, u)), mul(a.cam_u, v));
 }
 
-// SDEPTH traversal-stack entries per thread in shared memory (16 KB a block at 16), for
-// scenes far larger than the caches: there the local-memory stack's lines compete with the
-// scene for L1 and L2.  A scene that the caches hold keeps the whole stack in local memory
-// and the caches for itself.
-#ifndef RTB_RENDER_BLOCKS_PER_SM
-#define RTB_RENDER_BLOCKS_PER_SM 8  // 64 registers a thread; 6, 7 and 9 measured slower
-#endif
-template <bool METRICS, int SDEPTH>
-__global__ void __launch_bounds__(128, RTB_RENDER_BLOCKS_PER_SM) k_render(RenderArgs a) {
-  __shared__ int2 s_stack[SDEPTH > 0 ? SDEPTH : 1][128];
+// Queue entry p as a work item: a whole pixel from its first sample, or ~(tail item), one sample.
+__device__ __forceinline__ void take_item(const RenderArgs& a, long long p, long long& item,
+                                          long long& pixel, int& so) {
+  if (p < a.split) {
+    item = pixel = p;
+    so = 0;
+  } else {
+    const unsigned t = (unsigned)(p - a.split);  // at most kMaxTailItems
+    const unsigned q = fast_div(t, a.spp_magic);
+    item = ~(long long)t;
+    pixel = a.split + q;
+    so = (int)(t - q * (unsigned)a.spp);
+  }
+}
+
+// The camera ray and random stream of sample `so` of an output pixel.
+__device__ __forceinline__ void start_sample(const RenderArgs& a, long long pixel, int so, uint32_t& rng,
+                                             float3& o, float3& d) {
+  int x, y;
+  if (a.pixels <= 0xFFFFFFFFLL) {
+    const unsigned row = fast_div((unsigned)pixel, a.width_magic);
+    x = (int)((unsigned)pixel - row * (unsigned)a.width);
+    y = (int)row;
+  } else {
+    x = (int)(pixel % a.width);
+    y = (int)(pixel / a.width);
+  }
+  camera_sample(a, x, a.row0 + y * a.row_stride, so, rng, o, d);
+}
+
+__device__ void add_counters(unsigned long long* k, const TraceCounters& c) {
+  atomicAdd(k + 0, c.rays);
+  atomicAdd(k + 1, c.aabb);
+  atomicAdd(k + 2, c.prim);
+  atomicAdd(k + 3, c.type[0]);
+  atomicAdd(k + 4, c.type[1]);
+  atomicAdd(k + 5, c.type[2]);
+  atomicAdd(k + 6, c.type[3]);
+  atomicAdd(k + 7, c.type[4]);
+  atomicAdd(k + 8, c.overflow);
+  atomicMax(k + 9, c.maxstack);
+  atomicAdd(k + 10, c.internal);
+  atomicAdd(k + 11, c.leaf);
+  atomicAdd(k + 12, c.homo);
+  atomicAdd(k + 13, c.mixed);
+}
+
+// ---- the persistent frame kernel
+//
+// Every block owns path slots in global memory, several per lane; a slot holds a path (ray,
+// throughput, radiance, random stream) and the work item it belongs to.  The block runs two
+// alternating phases over its slots:
+//
+//  trace  lanes take the slots' rays in order; when at least kRefillLanes lanes of a warp
+//         have finished their rays they store the hits and take the next ones, so a lane
+//         whose ray needs few nodes does not idle until the warp's longest ray ends;
+//  shade  every traced path is shaded, 32 per warp; a path that ends is replaced by its
+//         item's next sample or the next item of the frame's queue.
+//
+// When the queue is empty and paths end, two lists name the slots that still hold one, the
+// list that the phases read and the list that the shading writes, so that the paths that are
+// left keep full warps; until then a block's slots are all in use and need no list.
+//
+// The phases are the block's, not the warp's, for the instruction cache: the walk's loop is
+// small and the shading long and straight, and warps in both at once evict each other's
+// code (no_instruction stalls 7 per issue with a pool per warp, against 0.4 in a kernel that
+// only traces).  A block's slots are read and written once a phase, in order, mostly in L2.
+// The order in which paths are traced and shaded changes nothing in a path: its random
+// stream, its arithmetic and the sample order of a pixel's sum stay the same.
+//
+// Measured against one path a lane (k_render_small's form, as it was), where a warp's lanes wait
+// for its longest ray (9.65 active lanes, 12.56 G
+// warp instructions for 4.2 M samples of the 10k scene): 14.3 lanes, 8.45 G instructions; 10k
+// scene 1024x1024, 16 spp 68.5 -> 49.1 ms, 1M scene 1920x1080, 4 spp 56.0 -> 45.2 ms.
+//
+// A block of 1,024 threads keeps a whole SM in one phase: 10k scene 49.1 ms, with two blocks of
+// 512 52.4, with four of 256 56.8 (the same kernel's first form).
+//
+// k_render_small, in which every lane runs its own path's segments one after the other, has no
+// phases to wait for and keeps the path in registers; it is the faster one where the frame is
+// small or its rays meet next to no nodes (phases / lanes, ms): 65 spheres 256x256, 16 spp
+// 0.379 / 0.353 and 1024x1024 11.1 / 10.9, four glass spheres 1024x768, 16 spp, 24 segments
+// deep 6.21 / 4.56; but 300 mixed primitives 512x512, 16 spp 2.90 / 3.68, 10k 256x256 at 4 spp
+// 1.121 / 1.125, 8 spp 1.75 / 1.97.  So the phases take frames of kPhaseItems samples per
+// resident thread over a tree of kPhaseNodes nodes.
+constexpr int kBlock = 1024, kSmallBlock = 128;
+constexpr int kPhaseItems = 2, kPhaseNodes = 64;
+constexpr int kSlotsPerLane = 6;   // 4: 5 % slower (more phases), 8: 2 % (the slots leave L2)
+constexpr int kRefillLanes = 8;    // 4 and 12 within 1 %
+constexpr int kPoolLeafLanes = 8;  // 4 and 12 within 1 %
+
+// A path slot in global memory, by groups of 32 slots: the group's origins, directions,
+// throughputs, radiances, sums (16 bytes a slot), hits and items (8 bytes a slot).  A warp
+// that takes a group reads whole lines, and one base address serves every field.
+constexpr int kGroupBytes = 32 * 96;
+struct Slot {
+  char* p;   // the slot's 16-byte column
+  char* p8;  // its 8-byte column
+  __device__ __forceinline__ Slot(char* base, int s) {
+    char* g = base + (size_t)((unsigned)s >> 5) * kGroupBytes;
+    p = g + (s & 31) * 16;
+    p8 = g + (s & 31) * 8;
+  }
+  __device__ __forceinline__ float4& o() const { return *(float4*)p; }             // w: random stream's state
+  __device__ __forceinline__ float4& d() const { return *(float4*)(p + 512); }     // w: depth
+  __device__ __forceinline__ float4& thr() const { return *(float4*)(p + 1024); }  // w unused
+  __device__ __forceinline__ float4& rad() const { return *(float4*)(p + 1536); }  // w: sample index
+  // a whole pixel's running sum; read and written once a sample
+  __device__ __forceinline__ float4& acc() const { return *(float4*)(p + 2048); }
+  // closest bounded hit: distance, and type << 30 | index or one of the constants below
+  __device__ __forceinline__ float2& hit() const { return *(float2*)(p8 + 2560); }
+  // the work item: a whole pixel, or ~(tail item) of a single sample
+  __device__ __forceinline__ long long& item() const { return *(long long*)(p8 + 2816); }
+};
+// No hit; no traversal result (linear mode, stack overflow): the shade phase tests every
+// primitive.  Storage indices stay below kIndexMask - 1, so neither is a reference.
+constexpr int kNoRef = -1, kExhaustive = -2;
+
+__device__ __forceinline__ char* block_slots(const RenderArgs& a) {
+  return (char*)a.paths + (size_t)blockIdx.x * (((a.slots + 31) / 32) * (kGroupBytes + 256));
+}
+
+// How many slots of the block hold a path: all of them, or those of list[cur].
+struct SlotLists {
+  int count[2];
+  int head;  // the next entry to trace
+};
+__device__ __forceinline__ int* slot_list(const RenderArgs& a, char* base, int which) {
+  const int padded = (a.slots + 31) / 32 * 32;
+  return (int*)(base + (size_t)padded / 32 * kGroupBytes) + which * padded;
+}
+inline __host__ __device__ size_t block_path_bytes(int slots) {
+  return (size_t)((slots + 31) / 32) * (kGroupBytes + 2 * 32 * sizeof(int));
+}
+
+// The shade phase.  Out of line, so that the trace loop has the registers to itself.
+template <bool METRICS>
+static __device__ __noinline__ void shade_phase(const RenderArgs& a, SlotLists& L, int cur, bool first,
+                                                TraceCounters* c) {
   const DevScene& S = a.S;
+  char* const base_q = block_slots(a);
   const int lane = threadIdx.x & 31;
-  TraceCounters c{};
-  unsigned long long rays = 0;
-  // Per-lane state.
-  long long pixel = -1;
-  int x = 0, y = 0, so = 0;
-  int titem = -1;  // tail item of a single-sample lane, -1 while the lane holds a whole pixel
-  uint32_t base_seed = 0, rng = 0;
-  float3 acc = v3(0, 0, 0), thr = v3(0, 0, 0), rad = v3(0, 0, 0), o = v3(0, 0, 0), d = v3(0, 0, 0);
-  int depth = 0;
-  bool path = false;
-  bool done = false;
-  const float aspect = (float)a.width / (float)a.height;
-  while (true) {
-    // ---- fetch a pixel (warp-aggregated) for lanes that need one
-    bool need = !done && pixel < 0;
-    unsigned need_mask = __ballot_sync(0xFFFFFFFFu, need);
-    if (need_mask) {
-      unsigned long long basep = 0;
-      int leader = __ffs(need_mask) - 1;
-      if (lane == leader) {
-        basep = abort_raised(a.abort_flag) ? (unsigned long long)a.items
-                                           : atomicAdd(a.queue, (unsigned long long)__popc(need_mask));
+  const int n = L.count[cur];
+  const int* list = slot_list(a, base_q, cur);
+  int* out_list = slot_list(a, base_q, cur ^ 1);
+  for (int e0 = threadIdx.x - lane; e0 < n; e0 += kBlock) {
+    const bool in = e0 + lane < n;
+    const int s = !in ? 0 : n == a.slots ? e0 + lane : list[e0 + lane];
+    const Slot Q(base_q, s);
+    uint32_t rng = 0;
+    int depth = 0, so = -1;
+    float3 o = v3(0, 0, 0), d = v3(0, 0, 0), thr = v3(0, 0, 0), rad = v3(0, 0, 0);
+    bool finished = false, alive = in, need = first && in;
+    long long item = 0, pixel = 0;
+    if (in && !first) {
+      const float4 o4 = Q.o(), d4 = Q.d(), t4 = Q.thr(), r4 = Q.rad();
+      const float2 h2 = Q.hit();
+      o = v3(o4.x, o4.y, o4.z);
+      rng = __float_as_uint(o4.w);
+      d = v3(d4.x, d4.y, d4.z);
+      depth = __float_as_int(d4.w);
+      thr = v3(t4.x, t4.y, t4.z);
+      rad = v3(r4.x, r4.y, r4.z);
+      so = __float_as_int(r4.w);
+      const int ref = __float_as_int(h2.y);
+      Best h;
+      h.t = h2.x;
+      h.type = ref == kNoRef ? -1 : (int)((unsigned)ref >> kTypeShift);
+      h.index = ref & kIndexMask;
+      if (ref == kExhaustive) {
+        const bool bvh = S.use_bvh && S.node_count > 0;
+        if (METRICS && bvh) c->overflow++;
+        h = bvh ? test_all_refs<METRICS>(S, o, d, dot(d, d), no_hit(), c)
+                : test_all_primitives<METRICS>(S, o, d, dot(d, d), no_hit(), c);
       }
-      basep = __shfl_sync(0xFFFFFFFFu, basep, leader);
-      if (need) {
-        long long p = (long long)basep + __popc(need_mask & ((1u << lane) - 1u));
-        if (p >= a.items) {
-          done = true;
+      if (METRICS) c->rays++;
+      test_planes<METRICS>(S, o, d, h, c);
+      finished = shade_segment(S, h.type >= 0, h, o, d, thr, rad, rng, depth, a.max_depth);
+    }
+    if (finished) {
+      item = pixel = Q.item();
+      if (item < 0) {
+        float* t = a.tail + 3 * (size_t)~item;
+        t[0] = rad.x;
+        t[1] = rad.y;
+        t[2] = rad.z;
+        need = true;
+      } else {
+        float3 acc = rad;
+        if (so > 0) {
+          const float4 a4 = Q.acc();
+          acc = add(v3(a4.x, a4.y, a4.z), rad);
+        }
+        so++;
+        if (so == a.spp) {
+          acc = mul(acc, a.inv_spp);
+          float* out = a.out + 3 * item;
+          out[0] = acc.x;
+          out[1] = acc.y;
+          out[2] = acc.z;
+          need = true;
         } else {
-          if (p < a.split) {
-            so = 0;
-            titem = -1;
-          } else {
-            titem = (int)(p - a.split);
-            so = (int)((unsigned)titem % (unsigned)a.spp);
-            p = a.split + (long long)((unsigned)titem / (unsigned)a.spp);
-          }
-          pixel = p;
-          x = (int)(p % a.width);
-          y = a.row0 + (int)(p / a.width) * a.row_stride;
-          base_seed = pixel_base_seed(a.frame_seed, a.frame_index,
-                                      (uint32_t)y * (uint32_t)a.width + (uint32_t)x);
+          Q.acc() = make_float4(acc.x, acc.y, acc.z, 0.0f);
         }
       }
     }
-    if (__all_sync(0xFFFFFFFFu, done)) break;
+    // An abort ends every path at its sample's end: pixels with samples left stay unwritten.
+    if (__any_sync(0xFFFFFFFFu, finished || need) && abort_raised(a.abort_flag) && (finished || need))
+      alive = finished = need = false;
+    // ---- fetch an item (warp-aggregated) for slots that need one
+    const unsigned need_mask = __ballot_sync(0xFFFFFFFFu, need);
+    if (need_mask) {
+      unsigned long long basep = 0;
+      const int leader = __ffs(need_mask) - 1;
+      if (lane == leader) basep = atomicAdd(a.queue, (unsigned long long)__popc(need_mask));
+      basep = __shfl_sync(0xFFFFFFFFu, basep, leader);
+      if (need) {
+        const long long p = (long long)basep + __popc(need_mask & ((1u << lane) - 1u));
+        finished = alive = p < a.items;
+        take_item(a, p, item, pixel, so);
+        if (alive) Q.item() = item;
+      }
+    }
     // ---- start a sample (renderKernel prologue, K:1251-1264)
-    if (!done && !path) {
-      uint32_t seed = base_seed ^ hash_u32((uint32_t)so);
-      seed ^= hash_u32((uint32_t)(so * 0x9E3779B9u));
-      rng = hash_u32(seed);
-      float jx = rand01(&rng) - 0.5f;
-      float jy = rand01(&rng) - 0.5f;
-      float u = ((((float)x + 0.5f) + jx) * (2.0f / (float)a.width) - 1.0f) * aspect;
-      float v = 1.0f - ((((float)y + 0.5f) + jy) * (2.0f / (float)a.height));
-      o = a.cam_pos;
-      d = add(add(a.cam_f, mul(a.cam_r, u)), mul(a.cam_u, v));
+    if (alive) {
+      if (finished) {
+        start_sample(a, pixel, so, rng, o, d);
+        thr = v3(1.0f, 1.0f, 1.0f);
+        rad = v3(0.0f, 0.0f, 0.0f);
+        depth = 0;
+      }
+      Q.o() = make_float4(o.x, o.y, o.z, __uint_as_float(rng));
+      Q.d() = make_float4(d.x, d.y, d.z, __int_as_float(depth));
+      Q.thr() = make_float4(thr.x, thr.y, thr.z, 0.0f);
+      Q.rad() = make_float4(rad.x, rad.y, rad.z, __int_as_float(so));
+    }
+    const unsigned alive_mask = __ballot_sync(0xFFFFFFFFu, alive);
+    int base = 0;
+    if (lane == 0 && alive_mask) base = atomicAdd(&L.count[cur ^ 1], __popc(alive_mask));
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    if (alive) out_list[base + __popc(alive_mask & ((1u << lane) - 1u))] = s;
+  }
+}
+
+template <bool METRICS, int SDEPTH>
+__global__ void __launch_bounds__(kBlock, 1) k_render(const __grid_constant__ RenderArgs a) {
+  extern __shared__ int2 s_stack[];  // [SDEPTH][kBlock]
+  __shared__ SlotLists L;
+  const DevScene& S = a.S;
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  TraceCounters c{};
+  if (threadIdx.x == 0) {
+    L.count[0] = a.slots;
+    L.count[1] = 0;
+  }
+  int cur = 0;
+  bool first = true;
+  while (true) {
+    __syncthreads();
+    shade_phase<METRICS>(a, L, cur, first, METRICS ? &c : nullptr);
+    first = false;
+    if (threadIdx.x == 0) L.head = 0;
+    __syncthreads();
+    if (threadIdx.x == 0) L.count[cur] = 0;
+    cur ^= 1;
+    const int n = L.count[cur];
+    if (n == 0) break;
+    // ---- trace phase
+    char* const base_q = block_slots(a);
+    const int* list = slot_list(a, base_q, cur);
+    const bool bvh = S.use_bvh && S.node_count > 0;
+    int slot = -1;
+    float3 o = v3(0, 0, 0), d = v3(0, 0, 0), inv = v3(0, 0, 0);
+    float dd = 0.0f;
+    Best b = no_hit();
+    Walk w;
+    WalkStack<SDEPTH> ws;
+    w.begin(S, false);
+    bool more = true;  // warp-uniform: slots may be left to take
+    while (true) {
+      const unsigned walk = __ballot_sync(0xFFFFFFFFu, w.can_walk());
+      const unsigned waiting = __ballot_sync(0xFFFFFFFFu, w.waiting());
+      const unsigned busy = walk | waiting;
+      const int idle = 32 - __popc(busy);
+      if (busy == 0u || (more && idle >= kRefillLanes)) {
+        const bool free_lane = !(busy >> lane & 1u);
+        if (free_lane && slot >= 0) {
+          const int ref = !bvh || w.overflow ? kExhaustive
+                          : b.type < 0       ? kNoRef
+                                             : (int)((unsigned)b.type << kTypeShift | (unsigned)b.index);
+          Slot(base_q, slot).hit() = make_float2(b.t, __int_as_float(ref));
+          slot = -1;
+        }
+        if (!more) break;
+        int next = 0;
+        if (lane == 0) next = atomicAdd(&L.head, idle);
+        next = __shfl_sync(0xFFFFFFFFu, next, 0);
+        more = next + idle < n;
+        const int e = next + __popc(~busy & below);
+        if (free_lane && e < n) {
+          slot = n == a.slots ? e : list[e];
+          const Slot Q(base_q, slot);
+          const float4 o4 = Q.o(), d4 = Q.d();
+          o = v3(o4.x, o4.y, o4.z);
+          d = v3(d4.x, d4.y, d4.z);
+          inv = ray_inverse(d);
+          dd = dot(d, d);
+          b = no_hit();
+          w.begin(S, bvh);
+        }
+        continue;
+      }
+      if (__popc(walk) <= kPoolLeafLanes && waiting != 0u) {
+        test_recorded<METRICS>(S, w, o, d, dd, b, METRICS ? &c : nullptr);
+        continue;
+      }
+      if (w.can_walk())
+        walk_node<METRICS, SDEPTH, kBlock>(S, w, ws, o, inv, b, METRICS ? &c : nullptr, s_stack + threadIdx.x);
+    }
+  }
+  if (METRICS) add_counters(a.counters, c);
+}
+
+// Each lane holds one item at a time: a whole pixel, its samples in order, or a single sample.
+template <bool METRICS, int SDEPTH>
+__global__ void __launch_bounds__(kSmallBlock, 1024 / kSmallBlock) k_render_small(const __grid_constant__ RenderArgs a) {
+  extern __shared__ int2 s_stack[];  // [SDEPTH][kSmallBlock]
+  const DevScene& S = a.S;
+  const int lane = threadIdx.x & 31;
+  if (a.max_depth <= 0) {  // every sample is black
+    for (long long p = (long long)blockIdx.x * kSmallBlock + threadIdx.x; p < 3 * a.pixels;
+         p += (long long)gridDim.x * kSmallBlock)
+      a.out[p] = 0.0f;
+    return;
+  }
+  TraceCounters c{};
+  long long item = 0, pixel = 0;
+  int so = 0, depth = 0;
+  uint32_t rng = 0;
+  float3 acc = v3(0, 0, 0), thr = v3(0, 0, 0), rad = v3(0, 0, 0), o = v3(0, 0, 0), d = v3(0, 0, 0);
+  bool alive = true, need = true, start = true;
+  while (true) {
+    // ---- fetch an item (warp-aggregated) for lanes that need one
+    const unsigned need_mask = __ballot_sync(0xFFFFFFFFu, need);
+    if (need_mask) {
+      unsigned long long basep = 0;
+      const int leader = __ffs(need_mask) - 1;
+      if (lane == leader)
+        basep = abort_raised(a.abort_flag) ? (unsigned long long)a.items
+                                           : atomicAdd(a.queue, (unsigned long long)__popc(need_mask));
+      basep = __shfl_sync(0xFFFFFFFFu, basep, leader);
+      if (need) {
+        const long long p = (long long)basep + __popc(need_mask & ((1u << lane) - 1u));
+        alive = p < a.items;
+        need = false;
+        take_item(a, p, item, pixel, so);
+      }
+      if (!__any_sync(0xFFFFFFFFu, alive)) break;
+    }
+    if (alive && start) {
+      start_sample(a, pixel, so, rng, o, d);
       thr = v3(1.0f, 1.0f, 1.0f);
       rad = v3(0.0f, 0.0f, 0.0f);
       depth = 0;
-      path = a.max_depth > 0;
+      start = false;
     }
-    // ---- one path segment (tracePath loop body, K:1098-1162)
-    bool finished = !done && !path;  // max_depth == 0: the sample is black
-    bool tracing = !done && path;
     Best b;
-    bool hit = trace_closest<METRICS, SDEPTH, 128>(S, o, d, tracing, b, &c, nullptr,
-                                                  &s_stack[0][threadIdx.x]);
-    if (tracing) {
-      if (METRICS) rays++;
-      if (!hit) {
-        rad = add(rad, mulv(thr, S.background));
-        finished = true;
-      } else {
-        float3 pos, n;
-        int mi;
-        hit_record(S, b, o, d, &pos, &n, &mi);
-        float4 m0 = make_float4(0, 0, 0, 0), m1 = m0, m2 = m0, m3 = m0;
-        if (mi >= 0) {
-          const float4* mp = S.materials + 4 * mi;
-          m0 = __ldg(mp);
-          m1 = __ldg(mp + 1);
-          m2 = __ldg(mp + 2);
-          m3 = __ldg(mp + 3);
-        }
-        float3 cd = v3(m0.x, m0.y, m0.z), cr = v3(m1.x, m1.y, m1.z), ct = v3(m2.x, m2.y, m2.z);
-        rad = add(rad, mulv(thr, v3(m3.x, m3.y, m3.z)));
-        float3 inc = neg(d);
-        float wd = luminance(cd), wr = luminance(cr), wt = luminance(ct);
-        float sum = wd + wr + wt;
-        if (sum <= 0.0f) {
-          finished = true;
+    const bool hit = trace_closest<METRICS, SDEPTH, kSmallBlock>(S, o, d, alive, b, METRICS ? &c : nullptr, nullptr,
+                                                                  s_stack + threadIdx.x);
+    if (alive) {
+      if (METRICS) c.rays++;
+      if (shade_segment(S, hit, b, o, d, thr, rad, rng, depth, a.max_depth)) {
+        start = true;
+        if (item < 0) {
+          float* t = a.tail + 3 * (size_t)~item;
+          t[0] = rad.x;
+          t[1] = rad.y;
+          t[2] = rad.z;
+          need = true;
         } else {
-          float xi = rand01(&rng) * sum;
-          float3 nd, wc;
-          if (xi < wd) {
-            float pc = wd / sum;
-            float z = rand01(&rng) * 2.0f - 1.0f;
-            float t = rand01(&rng) * 2.0f * CUDART_PI_F;
-            float r = sqrtf(fmaxf(0.0f, 1.0f - z * z));
-            nd = add(v3(r * cosf(t), r * sinf(t), z), n);
-            wc = divs(cd, pc);
-          } else if (xi < wd + wr) {
-            float pc = wr / sum;
-            nd = reflect_dir(n, inc);
-            wc = divs(cr, pc);
-          } else {
-            float pc = wt / sum;
-            nd = refract_dir(inc, n, m0.w);
-            wc = divs(ct, pc);
+          acc = so == 0 ? rad : add(acc, rad);
+          so++;
+          if (so == a.spp) {
+            acc = mul(acc, a.inv_spp);
+            float* out = a.out + 3 * item;
+            out[0] = acc.x;
+            out[1] = acc.y;
+            out[2] = acc.z;
+            need = true;
           }
-          o = add(pos, mul(nd, kEps));
-          thr = mulv(thr, wc);
-          d = nd;
-          depth++;
-          if (depth >= a.max_depth) finished = true;
         }
       }
     }
-    if (finished && titem >= 0) {
-      path = false;
-      float* t = a.tail + 3 * (size_t)titem;
-      t[0] = rad.x;
-      t[1] = rad.y;
-      t[2] = rad.z;
-      pixel = -1;
-    } else if (finished) {
-      path = false;
-      acc = so == 0 ? rad : add(acc, rad);
-      so++;
-      if (so == a.spp) {
-        acc = mul(acc, 1.0f / (float)a.spp);
-        float* out = a.out + 3 * pixel;
-        out[0] = acc.x;
-        out[1] = acc.y;
-        out[2] = acc.z;
-        pixel = -1;
-      }
-    }
   }
-  if (METRICS) {
-    unsigned long long* k = a.counters;
-    atomicAdd(k + 0, rays);
-    atomicAdd(k + 1, c.aabb);
-    atomicAdd(k + 2, c.prim);
-    atomicAdd(k + 3, c.type[0]);
-    atomicAdd(k + 4, c.type[1]);
-    atomicAdd(k + 5, c.type[2]);
-    atomicAdd(k + 6, c.type[3]);
-    atomicAdd(k + 7, c.type[4]);
-    atomicAdd(k + 8, c.overflow);
-    atomicMax(k + 9, c.maxstack);
-    atomicAdd(k + 10, c.internal);
-    atomicAdd(k + 11, c.leaf);
-    atomicAdd(k + 12, c.homo);
-    atomicAdd(k + 13, c.mixed);
-  }
+  if (METRICS) add_counters(a.counters, c);
 }
 
 // One thread per tail pixel: the in-order FP32 sum of its samples, scaled as in k_render.
@@ -325,7 +562,7 @@ __global__ void __launch_bounds__(256) k_sum_tail(const float* __restrict__ tail
 }
 
 template <bool METRICS>
-__global__ void __launch_bounds__(256) k_trace(DevScene S, const float* rays, int n, int* flags,
+__global__ void __launch_bounds__(256) k_trace(const __grid_constant__ DevScene S, const float* rays, int n, int* flags,
                                                float* dist, int* order, int* mat, float* normal,
                                                unsigned long long* counters) {
   int r = blockIdx.x * blockDim.x + threadIdx.x;
@@ -340,12 +577,16 @@ __global__ void __launch_bounds__(256) k_trace(DevScene S, const float* rays, in
   Best b;
   bool hit = trace_closest<METRICS>(S, o, d, active, b, &c, nullptr);
   if (!active) return;
-  float3 pos, nn = v3(0, 0, 0);
+  float3 nn = v3(0, 0, 0);
   int mi = -1;
-  if (hit) hit_record(S, b, o, d, &pos, &nn, &mi);
+  if (hit) {
+    const HitRecord hr = hit_record(S, b, o, d, add(o, mul(d, b.t)));
+    nn = hr.n;
+    mi = hr.material;
+  }
   flags[r] = hit ? 1 : 0;
   dist[r] = hit ? b.t : CUDART_INF_F;
-  order[r] = hit ? b.order : -1;
+  order[r] = hit ? order_of(S, b.type, b.index) : -1;
   mat[r] = hit ? mi : -1;
   normal[3 * (size_t)r] = nn.x;
   normal[3 * (size_t)r + 1] = nn.y;
@@ -367,8 +608,6 @@ __global__ void __launch_bounds__(256) k_trace(DevScene S, const float* rays, in
     atomicAdd(counters + 13, c.mixed);
   }
 }
-
-int g_render_blocks_per_sm[2][3] = {{0, 0, 0}, {0, 0, 0}};
 
 // Scenes whose traversal data (nodes, references, primitive records) exceed this many bytes
 // use the shared-memory stack: on the 1M-primitive scene (about 150 MB) it was 5 % faster,
@@ -420,9 +659,7 @@ __global__ void __launch_bounds__(256) k_wf_start(RenderArgs a, WaveState W, int
   }
   uint32_t rng;
   float3 o, d;
-  camera_sample(a, x, y, so,
-                pixel_base_seed(a.frame_seed, a.frame_index, (uint32_t)y * (uint32_t)a.width + (uint32_t)x),
-                rng, o, d);
+  camera_sample(a, x, y, so, rng, o, d);
   W.o[p] = make_float4(o.x, o.y, o.z, 0.0f);
   W.d[p] = make_float4(d.x, d.y, d.z, 0.0f);
   W.thr[p] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(rng));
@@ -431,7 +668,7 @@ __global__ void __launch_bounds__(256) k_wf_start(RenderArgs a, WaveState W, int
 }
 
 template <int SDEPTH>
-__global__ void __launch_bounds__(128, RTB_RENDER_BLOCKS_PER_SM) k_wf_trace(RenderArgs a, WaveState W,
+__global__ void __launch_bounds__(128, 8) k_wf_trace(const __grid_constant__ RenderArgs a, WaveState W,
                                                                            int cur) {
   __shared__ int2 s_stack[SDEPTH > 0 ? SDEPTH : 1][128];
   const int n = W.count[cur];
@@ -455,7 +692,7 @@ __global__ void __launch_bounds__(128, RTB_RENDER_BLOCKS_PER_SM) k_wf_trace(Rend
   }
 }
 
-__global__ void __launch_bounds__(256) k_wf_shade(RenderArgs a, WaveState W, int so, int cur) {
+__global__ void __launch_bounds__(256) k_wf_shade(const __grid_constant__ RenderArgs a, WaveState W, int so, int cur) {
   const int n = W.count[cur];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -504,6 +741,7 @@ struct FramePlan {
   RenderArgs a;
   int metrics = 0;
   int shared_stack = 0;       // k_render's SDEPTH: 0, 8 or kSharedStackDepth
+  int block = 0;              // kBlock: k_render, kSmallBlock: k_render_small
   long long resident = 0;     // threads of a full-occupancy grid
   long long tail_pixels = 0;  // the frame's last pixels, queued one sample per item
   long long grid = 0;
@@ -511,20 +749,33 @@ struct FramePlan {
 
 namespace {
 
-const void* render_kernel(int metrics, int shared_stack) {
-  if (shared_stack == kSharedStackDepth)
-    return metrics ? (const void*)k_render<true, kSharedStackDepth>
-                   : (const void*)k_render<false, kSharedStackDepth>;
-  if (shared_stack == 8)
-    return metrics ? (const void*)k_render<true, 8> : (const void*)k_render<false, 8>;
-  return metrics ? (const void*)k_render<true, 0> : (const void*)k_render<false, 0>;
+template <bool METRICS, int SDEPTH>
+const void* render_kernel_of(int block) {
+  return block == kBlock ? (const void*)k_render<METRICS, SDEPTH> : (const void*)k_render_small<METRICS, SDEPTH>;
 }
 
-int frame_blocks_per_sm(int metrics, int shared_stack) {
-  int& bps = g_render_blocks_per_sm[metrics][shared_stack == 0 ? 0 : shared_stack == 8 ? 1 : 2];
+const void* render_kernel(int metrics, int shared_stack, int block) {
+  if (shared_stack == kSharedStackDepth)
+    return metrics ? render_kernel_of<true, kSharedStackDepth>(block)
+                   : render_kernel_of<false, kSharedStackDepth>(block);
+  if (shared_stack == 8) return metrics ? render_kernel_of<true, 8>(block) : render_kernel_of<false, 8>(block);
+  return metrics ? render_kernel_of<true, 0>(block) : render_kernel_of<false, 0>(block);
+}
+
+size_t stack_smem(int shared_stack, int block) { return (size_t)shared_stack * block * sizeof(int2); }
+
+int frame_blocks_per_sm(rtb_context* ctx, int metrics, int shared_stack, int block) {
+  int& bps = ctx->frame_blocks[metrics][shared_stack == 0 ? 0 : shared_stack == 8 ? 1 : 2][block == kBlock];
   if (bps == 0) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, render_kernel(metrics, shared_stack), 128, 0);
+    const void* kernel = render_kernel(metrics, shared_stack, block);
+    const size_t smem = stack_smem(shared_stack, block);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, block, smem);
     if (bps < 1) bps = 1;
+    // Loads the sum's code now: loaded at its first launch, behind a running frame, it would
+    // hold up an abort request until the frame ends.
+    cudaFuncAttributes loaded;
+    cudaFuncGetAttributes(&loaded, (const void*)k_sum_tail);
   }
   return bps;
 }
@@ -539,8 +790,19 @@ void set_tail(FramePlan* f, long long tail_pixels) {
   f->tail_pixels = tail_pixels;
   a.split = a.pixels - tail_pixels;
   a.items = a.split + tail_pixels * a.spp;
-  long long want = (a.items + 127) / 128;
-  f->grid = std::min<long long>(f->resident / 128, want);
+  const long long blocks = f->resident / f->block;
+  a.slots = 0;
+  if (f->block == kSmallBlock) {
+    f->grid = std::min<long long>(blocks, (a.items + kSmallBlock - 1) / kSmallBlock);
+    return;
+  }
+  // Path slots per block: kSlotsPerLane a lane on large frames; where the frame's items fill
+  // them only a few times, the number that divides them into equal rounds (a last round of a
+  // few slots costs nearly a whole one).
+  const long long most = kSlotsPerLane * kBlock;
+  const long long rounds = (a.items + blocks * most - 1) / (blocks * most);
+  a.slots = (int)std::min(most, std::max<long long>(32, (a.items + blocks * rounds - 1) / (blocks * rounds)));
+  f->grid = std::min<long long>(blocks, (a.items + a.slots - 1) / a.slots);
 }
 
 }  // namespace
@@ -565,9 +827,15 @@ rtb_status plan_frame(rtb_context* ctx, rtb_scene* scene, const rtb_camera* cam,
   a.width = p->width;
   a.height = p->height;
   a.spp = p->samples_per_frame;
+  a.aspect = (float)a.width / (float)a.height;  // IEEE quotients, the same on host and device
+  a.step_x = 2.0f / (float)a.width;
+  a.step_y = 2.0f / (float)a.height;
+  a.inv_spp = 1.0f / (float)a.spp;
+  a.spp_magic = div_magic((unsigned)a.spp);
+  a.width_magic = div_magic((unsigned)a.width);
   a.max_depth = p->max_depth;
-  a.frame_index = p->frame_index;
-  a.frame_seed = p->frame_seed;
+  a.frame_hash = hash_u32((uint32_t)(p->frame_seed & 0xFFFFFFFFULL)) ^
+                 hash_u32((uint32_t)(p->frame_seed >> 32)) ^ hash_u32((uint32_t)p->frame_index);
   if (row0 < 0 || row0 >= p->height || row_stride < 1)
     return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "first row must be in [0, height) and the stride positive");
   a.out = d_rgb;
@@ -581,11 +849,16 @@ rtb_status plan_frame(rtb_context* ctx, rtb_scene* scene, const rtb_camera* cam,
     return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "shared_stack_entries must be 0, -1, 8 or 16");
   f->shared_stack = se == 0 ? (traversal_bytes(a.S) > kSharedStackSceneBytes ? kSharedStackDepth : 0)
                   : se < 0 ? 0 : se;
-  f->resident = (long long)ctx->sm_count * frame_blocks_per_sm(f->metrics, f->shared_stack) * 128;
+  f->block = a.max_depth > 0 && a.S.use_bvh && a.S.node_count >= kPhaseNodes &&
+                     a.pixels * a.spp >= (long long)kPhaseItems * 1024 * ctx->sm_count
+                 ? kBlock
+                 : kSmallBlock;
+  f->resident = (long long)ctx->sm_count * frame_blocks_per_sm(ctx, f->metrics, f->shared_stack, f->block) * f->block;
   // Tail: about four pixels per resident thread are split into single samples.
   double per_thread = tail_per_thread > 0 ? (double)tail_per_thread : RTB_TAIL_FACTOR;
   long long tail_pixels = std::min<long long>(a.pixels, (long long)(per_thread * f->resident));
-  set_tail(f, std::min<long long>(tail_pixels, kMaxTailItems / a.spp));
+  // A pixel of one sample is its own item, and a black frame has none.
+  set_tail(f, a.max_depth > 0 && a.spp > 1 ? std::min<long long>(tail_pixels, kMaxTailItems / a.spp) : 0);
   return RTB_OK;
 }
 
@@ -593,33 +866,25 @@ size_t frame_tail_bytes(const FramePlan* f) {
   return (size_t)f->tail_pixels * f->a.spp * 3 * sizeof(float);
 }
 
-void bind_frame(FramePlan* f, unsigned long long* queue, float* tail, int* abort_flag,
+size_t frame_path_bytes(const FramePlan* f) {
+  return f->block == kBlock ? (size_t)f->grid * block_path_bytes(f->a.slots) : 0;
+}
+
+void bind_frame(FramePlan* f, unsigned long long* queue, float* tail, void* paths, int* abort_flag,
                 unsigned long long* counters) {
-  if (!tail) set_tail(f, 0);  // no buffer: every pixel keeps its samples in one lane
+  if (!tail) set_tail(f, 0);  // no buffer: every pixel keeps its samples in one slot
   f->a.queue = queue;
   f->a.tail = tail;
+  f->a.paths = paths;
   f->a.abort_flag = abort_flag;
   f->a.counters = counters;
 }
 
 int launch_frame(const FramePlan* f, cudaStream_t stream) {
   const RenderArgs& a = f->a;
-  if (f->shared_stack == kSharedStackDepth) {
-    if (f->metrics)
-      k_render<true, kSharedStackDepth><<<(unsigned)f->grid, 128, 0, stream>>>(a);
-    else
-      k_render<false, kSharedStackDepth><<<(unsigned)f->grid, 128, 0, stream>>>(a);
-  } else if (f->shared_stack == 8) {
-    if (f->metrics)
-      k_render<true, 8><<<(unsigned)f->grid, 128, 0, stream>>>(a);
-    else
-      k_render<false, 8><<<(unsigned)f->grid, 128, 0, stream>>>(a);
-  } else {
-    if (f->metrics)
-      k_render<true, 0><<<(unsigned)f->grid, 128, 0, stream>>>(a);
-    else
-      k_render<false, 0><<<(unsigned)f->grid, 128, 0, stream>>>(a);
-  }
+  void* args[] = {const_cast<RenderArgs*>(&a)};
+  cudaLaunchKernel(render_kernel(f->metrics, f->shared_stack, f->block), dim3((unsigned)f->grid), dim3(f->block), args,
+                   stack_smem(f->shared_stack, f->block), stream);
   if (f->tail_pixels == 0) return 1;
   k_sum_tail<<<(unsigned)((f->tail_pixels + 255) / 256), 256, 0, stream>>>(
       a.tail, a.out, a.split, (int)f->tail_pixels, a.spp, a.abort_flag);
@@ -635,21 +900,25 @@ rtb_status render_frame(rtb_context* ctx, rtb_scene* scene, const rtb_camera* ca
   FramePlan f;
   rtb_status s = plan_frame(ctx, scene, cam, p, d_rgb, &f, row0, row_stride);
   if (s != RTB_OK) return s;
-  size_t tail_bytes = frame_tail_bytes(&f);
-  if (tail_bytes > ctx->tail_bytes) {
-    cudaStreamSynchronize(stream);  // the previous frame's sum may still read the buffer
-    cudaFree(ctx->d_tail);
-    ctx->d_tail = nullptr;
-    ctx->tail_bytes = 0;
-    if (cudaMalloc(&ctx->d_tail, tail_bytes) == cudaSuccess) {
-      ctx->tail_bytes = tail_bytes;
-    } else {
+  // The previous frame may still use a buffer that has to grow.
+  auto grow = [stream](auto** buf, size_t* have, size_t want) {
+    if (want <= *have) return true;
+    cudaStreamSynchronize(stream);
+    cudaFree(*buf);
+    *buf = nullptr;
+    *have = 0;
+    if (cudaMalloc(buf, want) != cudaSuccess) {
       cudaGetLastError();
-      ctx->d_tail = nullptr;
+      *buf = nullptr;
+      return false;
     }
-  }
-  bind_frame(&f, ctx->d_work, ctx->d_tail, ctx->d_abort, ctx->d_work + 8);
-  cudaMemsetAsync(ctx->d_work, 0, 32 * sizeof(unsigned long long), stream);
+    *have = want;
+    return true;
+  };
+  const bool tail_ok = grow(&ctx->d_tail, &ctx->tail_bytes, frame_tail_bytes(&f));
+  if (!grow(&ctx->d_paths, &ctx->path_bytes, frame_path_bytes(&f)))
+    return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "path slots");
+  bind_frame(&f, ctx->d_work, tail_ok ? ctx->d_tail : nullptr, ctx->d_paths, ctx->d_abort, ctx->d_work + 8);
   if (timed) cudaEventRecord(ctx->ev0, stream);
   ctx->render_launches = launch_frame(&f, stream);
   if (timed) cudaEventRecord(ctx->ev1, stream);
