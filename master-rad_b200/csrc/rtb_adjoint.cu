@@ -18,234 +18,347 @@
 #include <algorithm>
 
 #include "rtb_internal.h"
+#include "rtb_paths.cuh"
 
 namespace rtb {
 namespace {
 
 constexpr int kTable = 512;       // shared-memory gradient entries per block
 constexpr int kMaxVertices = 32;  // max_depth limit of the renderer
+constexpr long long kMaxVertexBytes = 256LL << 20;  // of the phases' paths
 
 struct AdjointArgs {
-  DevScene S;
-  float3 cam_pos, cam_f, cam_r, cam_u;
-  int width, height, spp, max_depth, frame_index;
-  unsigned long long frame_seed;
+  RenderArgs r;          // scene, camera, sizes, queue, path slots
   const float* adjoint;  // dLoss/dI, 3 floats per pixel
   float* grad_albedo;    // 3 per material
   float* grad_emission;  // 3 per material
-  long long pixels;
-  unsigned long long* queue;
-  int* abort_flag;  // the context's abort words (abort_raised)
+  float4* vertices;      // k_adjoint: the slots' path vertices, see PathVertices
+  long long samples;     // of the frame
 };
-
-__device__ __forceinline__ float luminance(float3 c) {  // K:181-183
-  return c.x * 0.212655f + c.y * 0.715158f + c.z * 0.072187f;
-}
-__device__ __forceinline__ float3 reflect_dir(float3 n, float3 i) {  // K:1022-1024
-  return sub(mul(n, 2.0f * dot(i, n)), i);
-}
-static __device__ __noinline__ float3 refract_dir(float3 incoming, float3 n, float eta) {  // K:1026-1039
-  float3 i = normalize_safe(incoming);
-  float c1 = dot(i, n);
-  float ri = (c1 >= 0.0f) ? eta : -1.0f / eta;
-  float inv_ri2 = 1.0f / (ri * ri);
-  float c2 = 1.0f - (1.0f - c1 * c1) * inv_ri2;
-  if (c2 <= 0.0f) return normalize_safe(reflect_dir(n, i));
-  float sq = sqrtf(c2);
-  return normalize_safe(sub(mul(n, c1 - sq * ri), i));
-}
 
 struct GradTable {
   int key[kTable];
   float val[kTable][6];
 };
 
-__device__ __forceinline__ void accumulate(GradTable& T, const AdjointArgs& a, int m, float3 ga,
-                                           float3 ge) {
-  unsigned h = ((unsigned)m * 2654435761u) & (kTable - 1);
-  for (int probe = 0; probe < 8; ++probe) {
-    int slot = (h + probe) & (kTable - 1);
-    int k = atomicCAS(&T.key[slot], -1, m);
-    if (k == -1 || k == m) {
-      atomicAdd(&T.val[slot][0], ga.x);
-      atomicAdd(&T.val[slot][1], ga.y);
-      atomicAdd(&T.val[slot][2], ga.z);
-      atomicAdd(&T.val[slot][3], ge.x);
-      atomicAdd(&T.val[slot][4], ge.y);
-      atomicAdd(&T.val[slot][5], ge.z);
-      return;
-    }
-  }
-  atomicAdd(a.grad_albedo + 3 * m, ga.x);
-  atomicAdd(a.grad_albedo + 3 * m + 1, ga.y);
-  atomicAdd(a.grad_albedo + 3 * m + 2, ga.z);
-  atomicAdd(a.grad_emission + 3 * m, ge.x);
-  atomicAdd(a.grad_emission + 3 * m + 1, ge.y);
-  atomicAdd(a.grad_emission + 3 * m + 2, ge.z);
-}
-
-__global__ void __launch_bounds__(128, 6) k_adjoint(const __grid_constant__ AdjointArgs a) {
-  __shared__ GradTable T;
+__device__ __forceinline__ void clear_table(GradTable& T) {
   for (int i = threadIdx.x; i < kTable; i += blockDim.x) {
     T.key[i] = -1;
     for (int k = 0; k < 6; ++k) T.val[i][k] = 0.0f;
   }
-  __syncthreads();
-  const DevScene& S = a.S;
+}
+
+// Adds the table to the gradients and empties it; between barriers.
+__device__ __forceinline__ void flush_table(GradTable& T, const AdjointArgs& a) {
+  for (int i = threadIdx.x; i < kTable; i += blockDim.x) {
+    const int m = T.key[i];
+    if (m < 0) continue;
+    for (int k = 0; k < 3; ++k) {
+      if (T.val[i][k] != 0.0f) atomicAdd(a.grad_albedo + 3 * m + k, T.val[i][k]);
+      if (T.val[i][3 + k] != 0.0f) atomicAdd(a.grad_emission + 3 * m + k, T.val[i][3 + k]);
+      T.val[i][k] = T.val[i][3 + k] = 0.0f;
+    }
+    T.key[i] = -1;
+  }
+}
+
+// The albedo gradient is zero wherever the path met no light afterwards: nothing is added then.
+__device__ __forceinline__ void accumulate(GradTable& T, const AdjointArgs& a, int m, float3 ga, float3 ge) {
+  float* pa = a.grad_albedo + 3 * m;
+  float* pe = a.grad_emission + 3 * m;
+  unsigned h = ((unsigned)m * 2654435761u) & (kTable - 1);
+  for (int probe = 0; probe < 8; ++probe) {
+    int slot = (h + probe) & (kTable - 1);
+    int k = *(volatile int*)&T.key[slot];
+    if (k == -1) k = atomicCAS(&T.key[slot], -1, m);
+    if (k == -1 || k == m) {
+      pa = &T.val[slot][0];
+      pe = &T.val[slot][3];
+      break;
+    }
+  }
+  if (ga.x != 0.0f || ga.y != 0.0f || ga.z != 0.0f) {
+    atomicAdd(pa, ga.x);
+    atomicAdd(pa + 1, ga.y);
+    atomicAdd(pa + 2, ga.z);
+  }
+  atomicAdd(pe, ge.x);
+  atomicAdd(pe + 1, ge.y);
+  atomicAdd(pe + 2, ge.z);
+}
+
+__device__ __forceinline__ float warp_sum(float v) {
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
+  return v;
+}
+
+// accumulate() for the lanes with `valid` set, all 32 lanes calling it.  Walls and lights are hit by
+// many lanes at once, and adds to one shared word run one after the other: the materials that
+// most lanes share are summed over the warp first, at most two of them.
+__device__ __forceinline__ void accumulate_warp(GradTable& T, const AdjointArgs& a, bool valid, int m, float3 ga,
+                                                float3 ge) {
+  for (int round = 0; round < 2; ++round) {
+    const unsigned peers = __match_any_sync(0xFFFFFFFFu, valid ? m : -1);
+    const int share = valid ? __popc(peers) : 0;
+    const int most = __reduce_max_sync(0xFFFFFFFFu, share);
+    if (most < 6) break;
+    const int leader = __ffs(__ballot_sync(0xFFFFFFFFu, share == most)) - 1;
+    const int common = __shfl_sync(0xFFFFFFFFu, m, leader);
+    const bool in = valid && m == common;
+    float3 sa = v3(0, 0, 0);
+    if (__any_sync(0xFFFFFFFFu, in && (ga.x != 0.0f || ga.y != 0.0f || ga.z != 0.0f)))
+      sa = v3(warp_sum(in ? ga.x : 0.0f), warp_sum(in ? ga.y : 0.0f), warp_sum(in ? ga.z : 0.0f));
+    const float3 se = v3(warp_sum(in ? ge.x : 0.0f), warp_sum(in ? ge.y : 0.0f), warp_sum(in ? ge.z : 0.0f));
+    if ((int)(threadIdx.x & 31) == leader) accumulate(T, a, common, sa, se);
+    valid = valid && !in;
+  }
+  if (valid) accumulate(T, a, m, ga, ge);
+}
+
+// The vertices of a block's paths: (throughput, 1 / p or 0) and (lobe weight, material), by
+// vertex, then slot.
+struct PathVertices {
+  float4* v;
+  int slots;
+  __device__ __forceinline__ PathVertices(const AdjointArgs& a)
+      : v(a.vertices + (size_t)blockIdx.x * a.r.slots * a.r.max_depth * 2), slots(a.r.slots) {}
+  __device__ __forceinline__ float4& thr(int k, int s) const { return v[(size_t)(2 * k) * slots + s]; }
+  __device__ __forceinline__ float4& w(int k, int s) const { return v[(size_t)(2 * k + 1) * slots + s]; }
+};
+
+// Queue entry p: a sample of a pixel.
+__device__ __forceinline__ void sample_item(const AdjointArgs& a, long long p, long long& pixel, int& so) {
+  if (a.samples <= 0xFFFFFFFFLL) {
+    const unsigned q = fast_div((unsigned)p, a.r.spp_magic);
+    pixel = q;
+    so = (int)((unsigned)p - q * (unsigned)a.r.spp);
+  } else {
+    pixel = p / a.r.spp;
+    so = (int)(p % a.r.spp);
+  }
+}
+
+__device__ __forceinline__ float3 pixel_adjoint(const AdjointArgs& a, long long pixel) {
+  const float* ap = a.adjoint + 3 * pixel;
+  return v3(ap[0] * a.r.inv_spp, ap[1] * a.r.inv_spp, ap[2] * a.r.inv_spp);
+}
+
+// The shade phase of the replay: every traced path gets its vertex, and a path that ends is
+// walked backward into the gradients and replaced by the queue's next sample.
+static __device__ __noinline__ void replay_phase(const AdjointArgs& a, GradTable& T, SlotLists& L, int cur,
+                                                 bool first) {
+  const DevScene& S = a.r.S;
+  char* const base_q = block_slots(a.r);
+  const PathVertices V(a);
   const int lane = threadIdx.x & 31;
-  long long pixel = -1;
-  int x = 0, y = 0, so = 0;
-  uint32_t base_seed = 0, rng = 0;
-  float3 adj = v3(0, 0, 0), thr = v3(0, 0, 0), o = v3(0, 0, 0), d = v3(0, 0, 0);
-  int depth = 0;
-  bool path = false, done = false;
+  const int n = L.count[cur];
+  const int* list = slot_list(a.r, base_q, cur);
+  int* out_list = slot_list(a.r, base_q, cur ^ 1);
+  for (int e0 = threadIdx.x - lane; e0 < n; e0 += kBlock) {
+    const bool in = e0 + lane < n;
+    const int s = !in ? 0 : n == a.r.slots ? e0 + lane : list[e0 + lane];
+    const Slot Q(base_q, s);
+    uint32_t rng = 0;
+    int depth = 0, nv = 0;
+    float3 o = v3(0, 0, 0), d = v3(0, 0, 0), thr = v3(0, 0, 0), adj = v3(0, 0, 0), li = v3(0, 0, 0);
+    bool alive = in, finished = first && in;
+    if (in && !first) {
+      const float4 o4 = Q.o(), d4 = Q.d(), t4 = Q.thr();
+      o = v3(o4.x, o4.y, o4.z);
+      rng = __float_as_uint(o4.w);
+      d = v3(d4.x, d4.y, d4.z);
+      depth = nv = __float_as_int(d4.w);
+      thr = v3(t4.x, t4.y, t4.z);
+      const Best h = slot_hit<false>(S, Q.hit(), o, d, nullptr);
+      if (h.type < 0) {
+        li = S.background;
+        finished = true;
+      } else {
+        const Vertex v = hit_vertex(S, h, o, d);
+        float3 wc = v3(0.0f, 0.0f, 0.0f);
+        float pc = 1.0f;
+        bool diffuse = false;
+        finished = !scatter(v, o, d, rng, wc, pc, diffuse);
+        // 1 / p of 0: no albedo gradient through this vertex
+        V.thr(depth, s) = make_float4(thr.x, thr.y, thr.z, diffuse ? 1.0f / pc : 0.0f);
+        V.w(depth, s) = make_float4(wc.x, wc.y, wc.z, __int_as_float(v.material));
+        nv = depth + 1;
+        if (!finished) {
+          thr = mulv(thr, wc);
+          depth++;
+          finished = depth >= a.r.max_depth;
+        }
+      }
+      if (finished) adj = pixel_adjoint(a, Q.item());
+    }
+    // ---- backward over the vertices of the paths that ended
+    if (__any_sync(0xFFFFFFFFu, finished && nv > 0)) {
+      for (int k = __reduce_max_sync(0xFFFFFFFFu, finished ? nv : 0) - 1; k >= 0; --k) {
+        const bool mine = finished && k < nv;
+        int m = -1;
+        float3 ga = v3(0, 0, 0), base = v3(0, 0, 0);
+        if (mine) {
+          const float4 t4 = V.thr(k, s), w4 = V.w(k, s);
+          m = __float_as_int(w4.w);
+          float3 e = v3(0.0f, 0.0f, 0.0f);
+          if (m >= 0) {
+            const float4 m3 = __ldg(S.materials + 4 * m + 3);
+            e = v3(m3.x, m3.y, m3.z);
+            base = mulv(adj, v3(t4.x, t4.y, t4.z));
+            ga = mul(mulv(base, li), t4.w);
+          }
+          li = add(e, mulv(v3(w4.x, w4.y, w4.z), li));
+        }
+        accumulate_warp(T, a, mine && m >= 0, m, ga, base);
+      }
+    }
+    // ---- the queue's next sample (warp-aggregated)
+    const unsigned need_mask = __ballot_sync(0xFFFFFFFFu, finished);
+    if (need_mask) {
+      unsigned long long basep = 0;
+      const int leader = __ffs(need_mask) - 1;
+      if (lane == leader)
+        basep = abort_raised(a.r.abort_flag) ? (unsigned long long)a.samples
+                                             : atomicAdd(a.r.queue, (unsigned long long)__popc(need_mask));
+      basep = __shfl_sync(0xFFFFFFFFu, basep, leader);
+      if (finished) {
+        const long long p = (long long)basep + __popc(need_mask & ((1u << lane) - 1u));
+        alive = p < a.samples;
+        if (alive) {
+          long long pixel;
+          int so;
+          sample_item(a, p, pixel, so);
+          start_sample(a.r, pixel, so, rng, o, d);
+          thr = v3(1.0f, 1.0f, 1.0f);
+          depth = 0;
+          Q.item() = pixel;
+        }
+      }
+    }
+    if (alive) {
+      Q.o() = make_float4(o.x, o.y, o.z, __uint_as_float(rng));
+      Q.d() = make_float4(d.x, d.y, d.z, __int_as_float(depth));
+      Q.thr() = make_float4(thr.x, thr.y, thr.z, 0.0f);
+    }
+    const unsigned alive_mask = __ballot_sync(0xFFFFFFFFu, alive);
+    int at = 0;
+    if (lane == 0 && alive_mask) at = atomicAdd(&L.count[cur ^ 1], __popc(alive_mask));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    if (alive) out_list[at + __popc(alive_mask & ((1u << lane) - 1u))] = s;
+  }
+}
+
+// The replay in the frame kernel's two phases.  The gradients of a block meet in a shared
+// table that is added to the global ones every kFlushPhases phases, so that no partial sum grows
+// longer than in one pass over a small share of the frame.
+constexpr int kFlushPhases = 8;
+__global__ void __launch_bounds__(kBlock, 1) k_adjoint(const __grid_constant__ AdjointArgs a) {
+  __shared__ SlotLists L;
+  __shared__ GradTable T;
+  clear_table(T);
+  if (threadIdx.x == 0) {
+    L.count[0] = a.r.slots;
+    L.count[1] = 0;
+  }
+  int cur = 0, phase = 0;
+  while (true) {
+    __syncthreads();
+    replay_phase(a, T, L, cur, phase == 0);
+    __syncthreads();
+    const int n = L.count[cur ^ 1];
+    if (threadIdx.x == 0) {
+      L.count[cur] = 0;
+      begin_trace(a.r, L, cur ^ 1);
+    }
+    cur ^= 1;
+    __syncthreads();
+    if (++phase % kFlushPhases == 0 || n == 0) flush_table(T, a);
+    if (n == 0) break;
+    trace_phase<false, 0>(a.r, L, &L.head, nullptr, nullptr);
+  }
+}
+
+// One path a lane, for what the phases are not faster at (see use_phases).
+__global__ void __launch_bounds__(128, 6) k_adjoint_small(const __grid_constant__ AdjointArgs a) {
+  __shared__ GradTable T;
+  clear_table(T);
+  __syncthreads();
+  const DevScene& S = a.r.S;
+  const int lane = threadIdx.x & 31;
+  long long pixel = 0;
+  uint32_t rng = 0;
+  float3 thr = v3(0, 0, 0), o = v3(0, 0, 0), d = v3(0, 0, 0);
+  bool alive = a.r.max_depth > 0, finished = true;
+  int nv = 0;
   // Vertex stack of the current sample.
   int vm[kMaxVertices];
   float3 vthr[kMaxVertices], vw[kMaxVertices];
   float vinvp[kMaxVertices];
-  int nv = 0;
-  bool escaped = false;
-  const float aspect = (float)a.width / (float)a.height;
   while (true) {
-    bool need = !done && pixel < 0;
-    unsigned need_mask = __ballot_sync(0xFFFFFFFFu, need);
+    const unsigned need_mask = __ballot_sync(0xFFFFFFFFu, alive && finished);
     if (need_mask) {
       unsigned long long basep = 0;
-      int leader = __ffs(need_mask) - 1;
+      const int leader = __ffs(need_mask) - 1;
       if (lane == leader)
-        basep = abort_raised(a.abort_flag) ? (unsigned long long)a.pixels
-                                           : atomicAdd(a.queue, (unsigned long long)__popc(need_mask));
+        basep = abort_raised(a.r.abort_flag) ? (unsigned long long)a.samples
+                                             : atomicAdd(a.r.queue, (unsigned long long)__popc(need_mask));
       basep = __shfl_sync(0xFFFFFFFFu, basep, leader);
-      if (need) {
-        long long p = (long long)basep + __popc(need_mask & ((1u << lane) - 1u));
-        if (p >= a.pixels) {
-          done = true;
-        } else {
-          pixel = p;
-          x = (int)(p % a.width);
-          y = (int)(p / a.width);
-          so = 0;
-          uint32_t s = hash_u32((uint32_t)(a.frame_seed & 0xFFFFFFFFULL));
-          s ^= hash_u32((uint32_t)(a.frame_seed >> 32));
-          s ^= hash_u32((uint32_t)a.frame_index);
-          s ^= hash_u32((uint32_t)y * (uint32_t)a.width + (uint32_t)x);
-          base_seed = hash_u32(s);
-          float inv_spp = 1.0f / (float)a.spp;
-          const float* ap = a.adjoint + 3 * p;
-          adj = v3(ap[0] * inv_spp, ap[1] * inv_spp, ap[2] * inv_spp);
+      if (alive && finished) {
+        const long long p = (long long)basep + __popc(need_mask & ((1u << lane) - 1u));
+        alive = p < a.samples;
+        if (alive) {
+          int so;
+          sample_item(a, p, pixel, so);
+          start_sample(a.r, pixel, so, rng, o, d);
+          thr = v3(1.0f, 1.0f, 1.0f);
+          nv = 0;
+          finished = false;
         }
       }
     }
-    if (__all_sync(0xFFFFFFFFu, done)) break;
-    if (!done && !path) {  // replay the sample's camera ray (K:1251-1264)
-      uint32_t seed = base_seed ^ hash_u32((uint32_t)so);
-      seed ^= hash_u32((uint32_t)(so * 0x9E3779B9u));
-      rng = hash_u32(seed);
-      float jx = rand01(&rng) - 0.5f;
-      float jy = rand01(&rng) - 0.5f;
-      float u = ((((float)x + 0.5f) + jx) * (2.0f / (float)a.width) - 1.0f) * aspect;
-      float v = 1.0f - ((((float)y + 0.5f) + jy) * (2.0f / (float)a.height));
-      o = a.cam_pos;
-      d = add(add(a.cam_f, mul(a.cam_r, u)), mul(a.cam_u, v));
-      thr = v3(1.0f, 1.0f, 1.0f);
-      depth = 0;
-      nv = 0;
-      escaped = false;
-      path = a.max_depth > 0;
-    }
-    bool finished = !done && !path;
-    bool tracing = !done && path;
+    if (!__any_sync(0xFFFFFFFFu, alive)) break;
     Best b;
-    bool hit = trace_closest<false>(S, o, d, tracing, b, nullptr, nullptr);
-    if (tracing) {
+    const bool hit = trace_closest<false>(S, o, d, alive, b, nullptr, nullptr);
+    float3 li = v3(0.0f, 0.0f, 0.0f);
+    if (alive) {
       if (!hit) {
-        escaped = true;
+        li = S.background;
         finished = true;
       } else {
-        const float3 pos = add(o, mul(d, b.t));
-        const HitRecord hr = hit_record(S, b, o, d, pos);
-        const float3 n = hr.n;
-        const int mi = hr.material;
-        float4 m0 = make_float4(0, 0, 0, 0), m1 = m0, m2 = m0;
-        if (mi >= 0) {
-          const float4* mp = S.materials + 4 * mi;
-          m0 = __ldg(mp);
-          m1 = __ldg(mp + 1);
-          m2 = __ldg(mp + 2);
-        }
-        float3 cd = v3(m0.x, m0.y, m0.z), cr = v3(m1.x, m1.y, m1.z), ct = v3(m2.x, m2.y, m2.z);
-        float3 inc = neg(d);
-        float wd = luminance(cd), wr = luminance(cr), wt = luminance(ct);
-        float sum = wd + wr + wt;
-        vm[nv] = mi;
+        const Vertex v = hit_vertex(S, b, o, d);
+        float3 wc = v3(0.0f, 0.0f, 0.0f);
+        float pc = 1.0f;
+        bool diffuse = false;
+        finished = !scatter(v, o, d, rng, wc, pc, diffuse);
+        vm[nv] = v.material;
         vthr[nv] = thr;
-        vw[nv] = v3(0.0f, 0.0f, 0.0f);
-        vinvp[nv] = 0.0f;  // 0: no albedo gradient through this vertex
-        if (sum <= 0.0f) {
-          finished = true;
-        } else {
-          float xi = rand01(&rng) * sum;
-          float3 nd, wc;
-          if (xi < wd) {
-            float pc = wd / sum;
-            float z = rand01(&rng) * 2.0f - 1.0f;
-            float t = rand01(&rng) * 2.0f * CUDART_PI_F;
-            float r = sqrtf(fmaxf(0.0f, 1.0f - z * z));
-            nd = add(v3(r * cosf(t), r * sinf(t), z), n);
-            wc = divs(cd, pc);
-            vinvp[nv] = 1.0f / pc;
-          } else if (xi < wd + wr) {
-            float pc = wr / sum;
-            nd = reflect_dir(n, inc);
-            wc = divs(cr, pc);
-          } else {
-            float pc = wt / sum;
-            nd = refract_dir(inc, n, m0.w);
-            wc = divs(ct, pc);
-          }
-          vw[nv] = wc;
-          o = add(pos, mul(nd, kEps));
-          thr = mulv(thr, wc);
-          d = nd;
-          depth++;
-          if (depth >= a.max_depth) finished = true;
-        }
+        vw[nv] = wc;
+        vinvp[nv] = diffuse ? 1.0f / pc : 0.0f;  // 0: no albedo gradient through this vertex
         nv++;
+        if (!finished) {
+          thr = mulv(thr, wc);
+          finished = nv >= a.r.max_depth;
+        }
       }
     }
-    if (finished) {
-      path = false;
-      if (nv > 0) {
-        // Backward over the sample's vertices.
-        float3 li = escaped ? S.background : v3(0.0f, 0.0f, 0.0f);
-        for (int k = nv - 1; k >= 0; --k) {
-          int m = vm[k];
-          float3 e = v3(0.0f, 0.0f, 0.0f);
-          if (m >= 0) {
-            float4 m3 = __ldg(S.materials + 4 * m + 3);
-            e = v3(m3.x, m3.y, m3.z);
-            float3 base = mulv(adj, vthr[k]);
-            float3 ga = mul(mulv(base, li), vinvp[k]);
-            accumulate(T, a, m, ga, base);
-          }
-          li = add(e, mulv(vw[k], li));
+    if (alive && finished) {
+      // Backward over the sample's vertices.
+      const float3 adj = pixel_adjoint(a, pixel);
+      for (int k = nv - 1; k >= 0; --k) {
+        int m = vm[k];
+        float3 e = v3(0.0f, 0.0f, 0.0f);
+        if (m >= 0) {
+          float4 m3 = __ldg(S.materials + 4 * m + 3);
+          e = v3(m3.x, m3.y, m3.z);
+          float3 base = mulv(adj, vthr[k]);
+          accumulate(T, a, m, mul(mulv(base, li), vinvp[k]), base);
         }
+        li = add(e, mulv(vw[k], li));
       }
-      so++;
-      if (so == a.spp) pixel = -1;
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < kTable; i += blockDim.x) {
-    int m = T.key[i];
-    if (m < 0) continue;
-    atomicAdd(a.grad_albedo + 3 * m, T.val[i][0]);
-    atomicAdd(a.grad_albedo + 3 * m + 1, T.val[i][1]);
-    atomicAdd(a.grad_albedo + 3 * m + 2, T.val[i][2]);
-    atomicAdd(a.grad_emission + 3 * m, T.val[i][3]);
-    atomicAdd(a.grad_emission + 3 * m + 1, T.val[i][4]);
-    atomicAdd(a.grad_emission + 3 * m + 2, T.val[i][5]);
-  }
+  flush_table(T, a);
 }
 
 __global__ void k_repack_materials(const float* raw, int n, float4* out) {
@@ -299,36 +412,43 @@ static rtb_status render_backward(rtb_context* ctx, rtb_scene* scene, const rtb_
     return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "GPU full-path depth must be in [0, 32]");
   cudaStream_t sm = stream ? stream : ctx->stream;
   ctx_acquire(ctx, sm);
-  AdjointArgs a;
-  a.S = scene->dev;
-  a.S.use_bvh = (p->use_bvh && scene->has_bvh) ? 1 : 0;
-  a.cam_pos = make_float3(cam->position[0], cam->position[1], cam->position[2]);
-  a.cam_f = make_float3(cam->forward[0], cam->forward[1], cam->forward[2]);
-  a.cam_r = make_float3(cam->right[0], cam->right[1], cam->right[2]);
-  a.cam_u = make_float3(cam->up[0], cam->up[1], cam->up[2]);
-  a.width = p->width;
-  a.height = p->height;
-  a.spp = p->samples_per_frame;
-  a.max_depth = p->max_depth;
-  a.frame_index = p->frame_index;
-  a.frame_seed = p->frame_seed;
+  AdjointArgs a{};
+  a.r = frame_args(scene, cam, p);
   a.adjoint = adjoint_device;
   a.grad_albedo = grad_albedo_device;
   a.grad_emission = grad_emission_device;
-  a.pixels = (long long)p->width * p->height;
-  a.queue = ctx->d_work;
-  a.abort_flag = ctx->d_abort;
+  a.samples = a.r.pixels * a.r.spp;
+  a.r.queue = ctx->d_work;
+  a.r.abort_flag = ctx->d_abort;
+  const bool phases = use_phases(a.r, ctx->sm_count);
+  long long grid = ctx->sm_count;
+  if (phases) {
+    // As many slots as a frame has (set_tail in rtb_render.cu), in equal rounds, but vertices of
+    // kMaxVertexBytes at most.
+    const long long vertex = 2 * sizeof(float4) * a.r.max_depth;
+    const long long most = std::max<long long>(
+        kBlock, std::min<long long>(kSlotsPerLane * kBlock, kMaxVertexBytes / (vertex * grid) / kBlock * kBlock));
+    const long long rounds = (a.samples + grid * most - 1) / (grid * most);
+    a.r.slots = (int)std::min(most, (a.samples + grid * rounds - 1) / (grid * rounds));
+    const size_t path_bytes = ((size_t)grid * block_path_bytes(a.r.slots) + 255) & ~(size_t)255;
+    if (!ctx_grow(&ctx->d_paths, &ctx->path_bytes, path_bytes + (size_t)(grid * a.r.slots * vertex), sm))
+      return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "path slots");
+    a.r.paths = ctx->d_paths;
+    a.vertices = (float4*)((char*)ctx->d_paths + path_bytes);
+  }
   size_t gbytes = (size_t)scene->dev.material_count * 3 * sizeof(float);
-  cudaMemsetAsync(ctx->d_work, 0, sizeof(unsigned long long), sm);
-  arm_abort(ctx, sm);
+  arm_abort(ctx, sm, true);
   cudaMemsetAsync(grad_albedo_device, 0, gbytes, sm);
   cudaMemsetAsync(grad_emission_device, 0, gbytes, sm);
-  int bps = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, (const void*)k_adjoint, 128, 0);
-  if (bps < 1) bps = 1;
-  long long grid = std::min<long long>((long long)ctx->sm_count * bps, (a.pixels + 127) / 128);
   cudaEventRecord(ctx->ev0, sm);
-  k_adjoint<<<(unsigned)std::max<long long>(1, grid), 128, 0, sm>>>(a);
+  if (phases) {
+    k_adjoint<<<(unsigned)grid, kBlock, 0, sm>>>(a);
+  } else {
+    int bps = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, (const void*)k_adjoint_small, 128, 0);
+    grid = std::min<long long>(grid * std::max(bps, 1), (a.samples + 127) / 128);
+    k_adjoint_small<<<(unsigned)std::max<long long>(1, grid), 128, 0, sm>>>(a);
+  }
   cudaEventRecord(ctx->ev1, sm);
   ctx_release(ctx, sm);
   cudaError_t e = cudaGetLastError();

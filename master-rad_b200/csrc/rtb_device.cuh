@@ -366,12 +366,23 @@ __device__ __forceinline__ float affine_box_local(const AffineRay& ar, const flo
 }
 
 // ---------------------------------------------------------------- closest hit
+// The closest bounded hit so far: its distance and its reference word (type << 30 | storage
+// index), kNoRef for none.  One word less than a Best in the walk's registers.
+constexpr int kNoRef = -1;  // storage indices stay below kIndexMask, so no reference is -1
+struct Hit {
+  float t;
+  int ref;
+};
+__device__ __forceinline__ Hit no_hit() { return Hit{1e30f, kNoRef}; }
+
 struct Best {
   float t;
   int type;   // PrimType of the winner, -1 for none
   int index;  // storage index of the winner (plane index for planes)
 };
-__device__ __forceinline__ Best no_hit() { return Best{1e30f, -1, -1}; }
+__device__ __forceinline__ Best best_of(Hit h) {
+  return Best{h.t, h.ref == kNoRef ? -1 : (int)((unsigned)h.ref >> kTypeShift), h.ref & kIndexMask};
+}
 
 // Global order of a primitive (a plane's storage index is its insertion index).
 __device__ __forceinline__ int order_of(const DevScene& S, int type, int index) {
@@ -381,16 +392,15 @@ __device__ __forceinline__ int order_of(const DevScene& S, int type, int index) 
 // Offers a candidate distance: the closest hit is the lexicographic minimum of
 // (distance, global order), the contract of tracePrimitiveRef (K:772-806).  The orders are
 // read only where two distances are equal.
-__device__ __forceinline__ void offer(const DevScene& S, Best& b, float t, int type, int index) {
+__device__ __forceinline__ void offer(const DevScene& S, Hit& b, float t, int ref) {
   if (t < b.t) {
     b.t = t;
-    b.type = type;
-    b.index = index;
+    b.ref = ref;
   } else if (t == b.t && t != CUDART_INF_F) {
-    if (b.type < 0 || order_of(S, type, index) < order_of(S, b.type, b.index)) {
-      b.type = type;
-      b.index = index;
-    }
+    if (b.ref == kNoRef ||
+        order_of(S, (int)((unsigned)ref >> kTypeShift), ref & kIndexMask) <
+            order_of(S, (int)((unsigned)b.ref >> kTypeShift), b.ref & kIndexMask))
+      b.ref = ref;
   }
 }
 
@@ -399,8 +409,9 @@ struct TraceCounters {
 };
 
 template <bool METRICS>
-__device__ __forceinline__ void test_ref(const DevScene& S, int type, int idx, float3 o, float3 d,
-                                         float dd, Best& b, TraceCounters* c) {
+__device__ __forceinline__ void test_ref(const DevScene& S, int ref, float3 o, float3 d, float dd, Hit& b,
+                                         TraceCounters* c) {
+  const int type = (int)((unsigned)ref >> kTypeShift), idx = ref & kIndexMask;
   float t;
   float3 dummy;
   if (type == kSphere) {
@@ -440,7 +451,7 @@ __device__ __forceinline__ void test_ref(const DevScene& S, int type, int idx, f
     c->prim++;
     c->type[type == kSphere ? 0 : type == kBox ? 1 : type == kAffineSphere ? 3 : 4]++;
   }
-  offer(S, b, t, type, idx);
+  offer(S, b, t, ref);
 }
 
 // Child-box entry distance for the node test.  (lo - o) * inv carries at most ~3 ulp
@@ -458,31 +469,29 @@ __device__ __forceinline__ float child_entry(float lox, float hix, float loy, fl
   return tn <= tf ? tn : CUDART_INF_F;
 }
 
-// Conservative prune limit for the current best distance, K:746-748 / 889-891.
-__device__ __forceinline__ float prune_limit(float t) {
-  return isfinite(t) ? fmaf(t, 1.0000015f, 1.0e-6f) : t;
-}
+// Conservative prune limit for the current best distance, K:746-748 / 889-891 (at most
+// no_hit's 1e30, so always finite).
+__device__ __forceinline__ float prune_limit(float t) { return fmaf(t, 1.0000015f, 1.0e-6f); }
 
 // The exhaustive paths, out of line and by value (see degenerate_local_direction): the best
 // hit over every reference or every primitive, starting from `b`.
 template <bool METRICS>
-__device__ __noinline__ Best test_all_refs(const DevScene& S, float3 o, float3 d, float dd, Best b,
+__device__ __noinline__ Hit test_all_refs(const DevScene& S, float3 o, float3 d, float dd, Hit b,
                                            TraceCounters* c) {
 #pragma unroll 1
   for (int i = 0; i < S.ref_count; ++i) {
-    int ref = __ldg(S.refs + i);
-    test_ref<METRICS>(S, (int)((unsigned)ref >> kTypeShift), ref & kIndexMask, o, d, dd, b, c);
+    test_ref<METRICS>(S, __ldg(S.refs + i), o, d, dd, b, c);
   }
   return b;
 }
 
 template <bool METRICS>
-__device__ __noinline__ Best test_all_primitives(const DevScene& S, float3 o, float3 d, float dd, Best b,
+__device__ __noinline__ Hit test_all_primitives(const DevScene& S, float3 o, float3 d, float dd, Hit b,
                                                  TraceCounters* c) {
 #pragma unroll 1
   for (int t = 0; t < 4; ++t)
 #pragma unroll 1
-    for (int i = 0; i < S.count[t]; ++i) test_ref<METRICS>(S, t, i, o, d, dd, b, c);
+    for (int i = 0; i < S.count[t]; ++i) test_ref<METRICS>(S, (int)((unsigned)t << kTypeShift) | i, o, d, dd, b, c);
   return b;
 }
 
@@ -515,19 +524,18 @@ struct Walk {
   // node's links again (16 bytes, in L1 as a rule), which costs less than the eight words
   // of links would cost in registers all through the walk.
   unsigned p0, p1;
+  // A tree visits each node at most once per ray; the cap only matters for malformed (cyclic)
+  // caller-supplied trees, which then take the exhaustive path, as does a full stack: negative.
   int budget;
-  bool overflow;
   __device__ __forceinline__ void begin(const DevScene& S, bool active) {
     node = active ? 0 : -1;
     sp = 0;
     p0 = p1 = 0u;
-    overflow = false;
-    // A tree visits each node at most once per ray; the cap only matters for malformed
-    // (cyclic) caller-supplied trees, which then take the exhaustive path.
     budget = S.node_count + 8;
   }
   __device__ __forceinline__ bool can_walk() const { return node >= 0 && p1 == 0u; }
   __device__ __forceinline__ bool waiting() const { return p0 != 0u; }
+  __device__ __forceinline__ bool overflow() const { return budget < 0; }
 };
 
 // The reciprocal direction of the node tests.
@@ -537,45 +545,37 @@ __device__ __forceinline__ float3 ray_inverse(float3 d) {
 }
 
 template <bool METRICS>
-__device__ __forceinline__ void test_recorded(const DevScene& S, Walk& w, float3 o, float3 d,
-                                              float dd, Best& b, TraceCounters* c) {
-  // A leaf child's first reference and count | (type code << 24), count 0 where not reached.
-  int f0 = 0, f1 = 0, f2 = 0, f3 = 0, m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+__device__ __forceinline__ void test_recorded(const DevScene& S, Walk& w, float3 o, float3 d, Hit& b,
+                                              TraceCounters* c) {
+  const float dd = dot(d, d);
+  // A leaf child's first reference and its count, 0 where the ray did not reach it.
+  int f0 = 0, f1 = 0, f2 = 0, f3 = 0, c0 = 0, c1 = 0, c2 = 0, c3 = 0;
   if (w.p0 != 0u) {
     const int4 n = __ldg(reinterpret_cast<const int4*>(S.nodes + (w.p0 & ~3u) + 3));
-    if (w.p0 & 1) f0 = ~n.x, m0 = n.z;
-    if (w.p0 & 2) f1 = ~n.y, m1 = n.w;
+    if (w.p0 & 1) f0 = ~n.x, c0 = n.z & 0xFFFFFF;
+    if (w.p0 & 2) f1 = ~n.y, c1 = n.w & 0xFFFFFF;
   }
   if (w.p1 != 0u) {
     const int4 n = __ldg(reinterpret_cast<const int4*>(S.nodes + (w.p1 & ~3u) + 3));
-    if (w.p1 & 1) f2 = ~n.x, m2 = n.z;
-    if (w.p1 & 2) f3 = ~n.y, m3 = n.w;
+    if (w.p1 & 1) f2 = ~n.x, c2 = n.z & 0xFFFFFF;
+    if (w.p1 & 2) f3 = ~n.y, c3 = n.w & 0xFFFFFF;
   }
-  const int c0 = m0 & 0xFFFFFF, c1 = m1 & 0xFFFFFF, c2 = m2 & 0xFFFFFF, c3 = m3 & 0xFFFFFF;
-  int e1 = c0 + c1, e2 = e1 + c2, e3 = e2 + c3;
+  // Reference k of the lane's leaves lies at at + k, `at` by the leaf that k falls into.
+  const int e1 = c0 + c1, e2 = e1 + c2, e3 = e2 + c3;
+  f1 -= c0;
+  f2 -= e1;
+  f3 -= e2;
 #pragma unroll 1
   for (int k = 0; k < e3; ++k) {
-    int first, meta, off;
-    if (k < c0) {
-      first = f0, meta = m0, off = k;
-    } else if (k < e1) {
-      first = f1, meta = m1, off = k - c0;
-    } else if (k < e2) {
-      first = f2, meta = m2, off = k - e1;
-    } else {
-      first = f3, meta = m3, off = k - e2;
-    }
-    int code = meta >> 24;
-    int ref = __ldg(S.refs + first + off);
-    int type = code == 4 ? (int)((unsigned)ref >> kTypeShift) : code;
-    test_ref<METRICS>(S, type, ref & kIndexMask, o, d, dd, b, c);
+    const int at = k < c0 ? f0 : k < e1 ? f1 : k < e2 ? f2 : f3;
+    test_ref<METRICS>(S, __ldg(S.refs + at + k), o, d, dd, b, c);
   }
   w.p0 = w.p1 = 0u;
 }
 
 template <bool METRICS, int SDEPTH, int SSTRIDE>
 __device__ __forceinline__ void walk_node(const DevScene& S, Walk& w, WalkStack<SDEPTH>& ws, float3 o,
-                                          float3 inv, const Best& b, TraceCounters* c, int2* ss) {
+                                          float3 inv, const Hit& b, TraceCounters* c, int2* ss) {
   const float4* np = S.nodes + 4 * w.node;
   float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2);
   int4 n3 = __ldg(reinterpret_cast<const int4*>(np + 3));
@@ -621,7 +621,7 @@ __device__ __forceinline__ void walk_node(const DevScene& S, Walk& w, WalkStack<
       w.sp++;
       if (METRICS && (unsigned long long)w.sp > c->maxstack) c->maxstack = w.sp;
     } else {
-      w.overflow = true;
+      w.budget = 0;  // negative below
     }
   }
   // Pop the next subtree still closer than the current hit.
@@ -639,8 +639,7 @@ __device__ __forceinline__ void walk_node(const DevScene& S, Walk& w, WalkStack<
     }
     if (se <= lim) next = sn;
   }
-  if (--w.budget < 0) w.overflow = true;
-  w.node = w.overflow ? -1 : next;
+  w.node = --w.budget < 0 ? -1 : next;
 }
 
 // tracePlane, K:708-734: a plane wins only when strictly closer.
@@ -681,8 +680,7 @@ __device__ __forceinline__ void test_planes(const DevScene& S, float3 o, float3 
 template <bool METRICS, int SDEPTH = 0, int SSTRIDE = 1>
 __device__ bool trace_closest(const DevScene& S, float3 o, float3 d, bool active, Best& b,
                               TraceCounters* c, int* overflow_flag, int2* ss = nullptr) {
-  b = no_hit();
-  float dd = dot(d, d);
+  Hit h = no_hit();
   const bool bvh = S.use_bvh && S.node_count > 0;
   {
     const float3 inv = ray_inverse(d);
@@ -695,18 +693,19 @@ __device__ bool trace_closest(const DevScene& S, float3 o, float3 d, bool active
       const unsigned waiting = __ballot_sync(0xFFFFFFFFu, w.waiting());
       if ((walk | waiting) == 0u) break;
       if (__popc(walk) <= kLeafPostponeLanes && waiting != 0u) {
-        test_recorded<METRICS>(S, w, o, d, dd, b, c);
+        test_recorded<METRICS>(S, w, o, d, h, c);
         continue;
       }
-      if (w.can_walk()) walk_node<METRICS, SDEPTH, SSTRIDE>(S, w, ws, o, inv, b, c, ss);
+      if (w.can_walk()) walk_node<METRICS, SDEPTH, SSTRIDE>(S, w, ws, o, inv, h, c, ss);
     }
-    if (w.overflow) {
+    if (w.overflow()) {
       if (overflow_flag) atomicAdd(overflow_flag, 1);
       if (METRICS) c->overflow++;
-      b = test_all_refs<METRICS>(S, o, d, dd, b, METRICS ? c : nullptr);
+      h = test_all_refs<METRICS>(S, o, d, dot(d, d), h, METRICS ? c : nullptr);
     }
   }
-  if (active && !bvh) b = test_all_primitives<METRICS>(S, o, d, dd, b, METRICS ? c : nullptr);
+  if (active && !bvh) h = test_all_primitives<METRICS>(S, o, d, dot(d, d), h, METRICS ? c : nullptr);
+  b = best_of(h);
   if (!active) return false;
   test_planes<METRICS>(S, o, d, b, c);
   return b.type >= 0;

@@ -91,6 +91,24 @@ void arm_abort(rtb_context* ctx, cudaStream_t s, bool clear_work = false);
 rtb_status fail(rtb_context* ctx, rtb_status s, const std::string& msg);
 rtb_status cuda_fail(rtb_context* ctx, cudaError_t e, const char* what);
 
+// Grows a context's device buffer to `want` bytes; `stream`'s work may still use the old one.
+// False, with no buffer, where the memory is not there.
+template <typename T>
+inline bool ctx_grow(T** buf, size_t* have, size_t want, cudaStream_t stream) {
+  if (want <= *have) return true;
+  cudaStreamSynchronize(stream);
+  cudaFree(*buf);
+  *buf = nullptr;
+  *have = 0;
+  if (cudaMalloc(buf, want) != cudaSuccess) {
+    cudaGetLastError();
+    *buf = nullptr;
+    return false;
+  }
+  *have = want;
+  return true;
+}
+
 // Device staging buffer of at least `bytes` (grown on demand, owned by the context).
 void* stage(rtb_context* ctx, size_t bytes);
 void* pinned(rtb_context* ctx, size_t bytes);
