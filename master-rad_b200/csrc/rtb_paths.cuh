@@ -20,7 +20,7 @@ struct RenderArgs {
   long long split;                 // pixels [split, pixels) are queued one sample per item
   long long items;                 // split + (pixels - split) * spp queue items
   void* paths;                     // the blocks' path slots
-  int slots;                       // path slots a block uses, at most kSlotsPerBlock
+  int slots;                       // path slots a block uses; k_render_small: lanes a warp uses
   float* tail;                     // RGB of each tail item, item - split order
   unsigned long long* queue;       // work queue head
   int* abort_flag;                 // the context's abort words (abort_raised)
