@@ -54,6 +54,10 @@ long long ns_since(Clock::time_point t0) {
   return std::chrono::duration_cast<std::chrono::nanoseconds>(Clock::now() - t0).count();
 }
 
+// Results up to this size come back by way of pinned staging: a 64x36 image (28 KB) or 4,000
+// rays; beyond it the second copy costs what the first saves.
+constexpr size_t kPinnedCopyBytes = 256 << 10;
+
 struct Guard {
   rtb_context* ctx;
   std::lock_guard<std::mutex> lock;
@@ -299,21 +303,31 @@ rtb_status rtb_trace_replay(rtb_context* ctx, rtb_scene* scene, const float* ray
   int* d_m = (int*)(sb + o);
   o += al(n * 4);
   float* d_n = (float*)(sb + o);
+  // Few rays go through pinned staging, one copy each way: a copy to or from pageable memory
+  // costs some 10 us of its own, and there are six.
+  const size_t rays_bytes = al(n * 24), hits_bytes = bytes - rays_bytes;
+  char* host = bytes <= kPinnedCopyBytes ? (char*)pinned(ctx, kPinnedCopyBytes) : nullptr;
   cudaStream_t sm = ctx->stream;
   ctx_acquire(ctx, sm);
-  cudaMemcpyAsync(d_rays, rays, n * 24, cudaMemcpyHostToDevice, sm);
+  if (host) memcpy(host, rays, n * 24);
+  cudaMemcpyAsync(d_rays, host ? (const void*)host : rays, n * 24, cudaMemcpyHostToDevice, sm);
   cudaEventRecord(ctx->ev0, sm);
   rtb_status s = trace_rays(ctx, scene, d_rays, ray_count, use_bvh, collect_metrics, d_f, d_t, d_o, d_m, d_n, sm);
   if (s != RTB_OK) return s;
   cudaEventRecord(ctx->ev1, sm);
-  cudaMemcpyAsync(hit_flags, d_f, n * 4, cudaMemcpyDeviceToHost, sm);
-  cudaMemcpyAsync(hit_distances, d_t, n * 4, cudaMemcpyDeviceToHost, sm);
-  cudaMemcpyAsync(hit_orders, d_o, n * 4, cudaMemcpyDeviceToHost, sm);
-  cudaMemcpyAsync(hit_materials, d_m, n * 4, cudaMemcpyDeviceToHost, sm);
-  cudaMemcpyAsync(hit_normals, d_n, n * 12, cudaMemcpyDeviceToHost, sm);
+  void* to[5] = {hit_flags, hit_distances, hit_orders, hit_materials, hit_normals};
+  const void* from[5] = {d_f, d_t, d_o, d_m, d_n};
+  if (host) {
+    cudaMemcpyAsync(host + rays_bytes, sb + rays_bytes, hits_bytes, cudaMemcpyDeviceToHost, sm);
+  } else {
+    for (int k = 0; k < 5; ++k)
+      cudaMemcpyAsync(to[k], from[k], n * (k < 4 ? 4 : 12), cudaMemcpyDeviceToHost, sm);
+  }
   ctx_release(ctx, sm);
   cudaError_t e = cudaStreamSynchronize(sm);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "trace replay");
+  if (host)
+    for (int k = 0; k < 5; ++k) memcpy(to[k], host + ((const char*)from[k] - sb), n * (k < 4 ? 4 : 12));
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
   ctx->last = rtb_frame_stats{};
@@ -382,15 +396,23 @@ rtb_status rtb_render_sample(rtb_context* ctx, rtb_scene* scene, const rtb_camer
   rtb_status s = render_frame(ctx, scene, camera, params, d_rgb, sm, true);
   ctx_release(ctx, sm);
   if (s != RTB_OK) return s;
+  // The stopped word and a small image come back by way of pinned staging in the frame's own
+  // stream, behind it, so that the host waits once; a large image is copied in place.
+  char* host = (char*)pinned(ctx, kPinnedCopyBytes);
+  const bool small = host && bytes <= kPinnedCopyBytes - 256;
+  int aborted = 0;  // abort word [2]: the kernel stopped fetching work
+  cudaMemcpyAsync(host ? (int*)host : &aborted, ctx->d_abort + 2, sizeof(int), cudaMemcpyDeviceToHost, sm);
+  if (small) cudaMemcpyAsync(host + 256, d_rgb, bytes, cudaMemcpyDeviceToHost, sm);
   cudaError_t e = cudaEventSynchronize(ctx->ev1);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "render");
-  int aborted = 0;  // abort word [2]: the kernel stopped fetching work
-  cudaMemcpy(&aborted, ctx->d_abort + 2, sizeof(int), cudaMemcpyDeviceToHost);
+  auto tc = Clock::now();
+  if (!small) e = cudaMemcpyAsync(rgb, d_rgb, bytes, cudaMemcpyDeviceToHost, sm);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(sm);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "image read-back");
+  if (small) memcpy(rgb, host + 256, bytes);
+  if (host) aborted = *(const int*)host;
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  auto tc = Clock::now();
-  e = cudaMemcpy(rgb, d_rgb, bytes, cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "image read-back");
   rtb_frame_stats st{};
   st.copy_ns = ns_since(tc);
   st.kernel_ns = (long long)(ms * 1e6);

@@ -350,11 +350,12 @@ class GpuRayTracer:
         ctx = self._require()
         res = self.ensure_scene_resident(scene, bvh)
         n = ray_count
-        flags = np.zeros(n, np.int32)
-        dist = np.zeros(n, np.float32)
-        order = np.zeros(n, np.int32)
-        mat = np.zeros(n, np.int32)
-        nrm = np.zeros(3 * n, np.float32)
+        # every element is written by the call
+        flags = np.empty(n, np.int32)
+        dist = np.empty(n, np.float32)
+        order = np.empty(n, np.int32)
+        mat = np.empty(n, np.int32)
+        nrm = np.empty(3 * n, np.float32)
         ctx.check(ctx.lib.rtb_trace_replay(ctx.handle, res.handle, N.fptr(rays), n,
                                            1 if self.bvh_traversal else 0,
                                            1 if collect_metrics else 0, N.iptr(flags),
