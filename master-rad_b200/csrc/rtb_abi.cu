@@ -198,7 +198,7 @@ rtb_status rtb_scene_upload(rtb_context* ctx, const rtb_scene_desc* desc, const 
   Guard g(ctx);
   auto t0 = Clock::now();
   ctx_acquire(ctx, ctx->stream);
-  rtb_status s = scene_create(ctx, desc, bvh, nullptr, nullptr, 0, nullptr, 0, nullptr, 0, out);
+  rtb_status s = scene_create(ctx, desc, bvh, nullptr, out);
   ctx_release(ctx, ctx->stream);
   if (s == RTB_OK) ctx->last.upload_ns = ns_since(t0);
   return s;

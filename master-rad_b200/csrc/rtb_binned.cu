@@ -558,7 +558,7 @@ rtb_status build_bvh_binned(rtb_context* ctx, const rtb_scene_desc* desc, const 
   if (st != RTB_OK) return st;
   if (stats) *stats = rtb_bvh_stats{};
   if (c.total == 0) {
-    rtb_status s = scene_create(ctx, desc, nullptr, nullptr, nullptr, 0, nullptr, 0, nullptr, 0, out);
+    rtb_status s = scene_create(ctx, desc, nullptr, nullptr, out);
     if (stats) stats->leaf_size = cfg->leaf_size;
     return s;
   }
@@ -587,7 +587,6 @@ rtb_status build_bvh_binned(rtb_context* ctx, const rtb_scene_desc* desc, const 
   int* lscan = W.alloc<int>(n);
   int* active = W.alloc<int>(cap);
   int* next_active = W.alloc<int>(cap);
-  int* all_nodes = W.alloc<int>(cap);
   // node counter, next count, stats {leaves, min occupancy, max occupancy, max depth},
   // next large count, partition errors
   int* counters = W.alloc<int>(8);
@@ -617,7 +616,6 @@ rtb_status build_bvh_binned(rtb_context* ctx, const rtb_scene_desc* desc, const 
   cudaMemcpyAsync(N.end, h_re, roots * 4, cudaMemcpyHostToDevice, sm);
   cudaMemcpyAsync(X.slot_of, h_slot.data(), roots * 4, cudaMemcpyHostToDevice, sm);
   cudaMemcpyAsync(active, h_init.data(), roots * 4, cudaMemcpyHostToDevice, sm);
-  cudaMemcpyAsync(all_nodes, h_init.data(), roots * 4, cudaMemcpyHostToDevice, sm);
   cudaMemcpyAsync(counters, h_counters, sizeof(h_counters), cudaMemcpyHostToDevice, sm);
   cudaMemsetAsync(N.order_axis, 0, (size_t)roots * 4, sm);
   cudaMemsetAsync(N.depth, 0, (size_t)roots * 4, sm);
@@ -632,10 +630,8 @@ rtb_status build_bvh_binned(rtb_context* ctx, const rtb_scene_desc* desc, const 
   S.lambda = c.lambda;
   for (int q = 0; q < 4; ++q) S.measured[q] = c.measured[q];
 
-  std::vector<int> level_begin = {0};
   int k = roots, level = 0, total_nodes = roots;
   while (k > 0) {
-    level_begin.push_back(level_begin.back() + k);
     if (large > 0) {
       k_init_acc<<<blocks((long long)large * 96), 256, 0, sm>>>(acc, gbins, large);
       k_node_acc<<<blocks(n), 256, 0, sm>>>(P, idx, key, level_of, level, X.slot_of, n, acc);
@@ -660,10 +656,7 @@ rtb_status build_bvh_binned(rtb_context* ctx, const rtb_scene_desc* desc, const 
     if (e != cudaSuccess) return cuda_fail(ctx, e, "binned BVH build level");
     if (h[7] != 0) return fail(ctx, RTB_ERR_DEVICE_CHECK, "binned BVH partition disagrees with its bins");
     int next = h[1];
-    if (next > 0) {
-      cudaMemcpyAsync(all_nodes + total_nodes, next_active, (size_t)next * 4, cudaMemcpyDeviceToDevice, sm);
-      std::swap(active, next_active);
-    }
+    if (next > 0) std::swap(active, next_active);
     total_nodes += next;
     large = h[6];
     k = next;
@@ -671,8 +664,7 @@ rtb_status build_bvh_binned(rtb_context* ctx, const rtb_scene_desc* desc, const 
   }
   IdxSet I;
   for (int a = 0; a < 3; ++a) I.a[a] = idx;
-  return finish_build(ctx, desc, cfg, W, c, P, I, N, all_nodes, level_begin, roots, total_nodes,
-                      counters, out, stats);
+  return finish_build(ctx, desc, cfg, W, c, in, P, I, N, roots, total_nodes, counters, out, stats);
 }
 
 }  // namespace rtb

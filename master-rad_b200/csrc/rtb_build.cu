@@ -890,54 +890,6 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
   }
 }
 
-// Nodes per depth, then all nodes listed level by level (the finishing passes walk them;
-// the order inside a level is free, every node of a level being independent of the
-// others).  Both passes count in shared memory first, a warp's lanes of equal depth
-// together, so that each block adds once per depth to the few global counters instead of
-// once per node; depths from kDepthShared up go to the global counters directly.
-constexpr int kDepthShared = 256;
-
-__global__ void __launch_bounds__(256) k_depth_hist(const Nodes N, int count, int* hist) {
-  __shared__ int sh[kDepthShared];
-  for (int i = threadIdx.x; i < kDepthShared; i += blockDim.x) sh[i] = 0;
-  __syncthreads();
-  const int node = blockIdx.x * blockDim.x + threadIdx.x;
-  const int d = node < count ? N.depth[node] : -1;
-  const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
-  if (d >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) {
-    if (d < kDepthShared) atomicAdd(sh + d, __popc(peers));
-    else atomicAdd(hist + d, __popc(peers));
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < kDepthShared; i += blockDim.x)
-    if (sh[i]) atomicAdd(hist + i, sh[i]);
-}
-
-__global__ void __launch_bounds__(256) k_depth_scatter(const Nodes N, int count, int* cursor,
-                                                       int* all_nodes) {
-  __shared__ int cnt[kDepthShared], base[kDepthShared];
-  for (int i = threadIdx.x; i < kDepthShared; i += blockDim.x) cnt[i] = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int node = blockIdx.x * blockDim.x + threadIdx.x;
-  const int d = node < count ? N.depth[node] : -1;
-  const unsigned peers = __match_any_sync(0xFFFFFFFFu, d);
-  const int leader = __ffs(peers) - 1;
-  int local = -1;  // rank among the block's nodes of depth d
-  if (d >= 0 && d < kDepthShared) {
-    int first = 0;
-    if (lane == leader) first = atomicAdd(cnt + d, __popc(peers));
-    local = first;
-  }
-  local = __shfl_sync(0xFFFFFFFFu, local, leader) + __popc(peers & ((1u << lane) - 1u));
-  __syncthreads();
-  for (int i = threadIdx.x; i < kDepthShared; i += blockDim.x)
-    if (cnt[i]) base[i] = atomicAdd(cursor + i, cnt[i]);
-  __syncthreads();
-  if (d >= kDepthShared) all_nodes[atomicAdd(cursor + d, 1)] = node;
-  else if (d >= 0) all_nodes[base[d] + local] = node;
-}
-
 // Leaf-or-split decision per active node (GpuScene.java:1424-1447).
 __global__ void k_decide(const Prims P, IdxSet I, Nodes N, const int* active, int k,
                          const double* best_cost, const long long* best_flat, const Box* node_box,
@@ -1210,7 +1162,7 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
     return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "rotationPasses must be positive.");
   if (stats) *stats = rtb_bvh_stats{};
   if (c.total == 0) {
-    rtb_status s = scene_create(ctx, desc, nullptr, nullptr, nullptr, 0, nullptr, 0, nullptr, 0, out);
+    rtb_status s = scene_create(ctx, desc, nullptr, nullptr, out);
     if (stats) stats->leaf_size = cfg->leaf_size;
     return s;
   }
@@ -1254,7 +1206,6 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   double* best_bound = W.alloc<double>(cap);
   int* lists = W.alloc<int>(2);  // small count, failed count
   int* sub_roots = W.alloc<int>(cap);  // nodes whose subtrees k_subtrees builds
-  int* depth_hist = W.alloc<int>(cap + 1);
   unsigned char* side = W.alloc<unsigned char>(n);
   int* flags = W.alloc<int>(3 * (size_t)n);  // left flags of the three axis orders
   int* lscan = W.alloc<int>(3 * (size_t)n);
@@ -1265,7 +1216,6 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   int* tkeys2 = W.alloc<int>(n);
   int* active = W.alloc<int>(cap);
   int* next_active = W.alloc<int>(cap);
-  int* all_nodes = W.alloc<int>(cap);
   double* best_cost = W.alloc<double>(cap);
   long long* best_flat = W.alloc<long long>(cap);
   int* arg_counts = W.alloc<int>(cap);
@@ -1331,7 +1281,6 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   TypeWeights tw;
   for (int t = 0; t < 4; ++t) tw.w[t] = c.weighted ? 1.0 + c.lambda * (c.measured[t] - 1.0) : 1.0;
   int sequential_nodes = 0;
-  std::vector<int> level_begin = {0};
   int k = (int)h_big.size(), level = 0, total_nodes = roots;
   const dim3 seg_grid(nc, 3), carry_grid(3, 2);
   // split costs of every position on all three axes (and the level's node bounds)
@@ -1436,7 +1385,7 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
     k = next;
     level++;
   }
-  // ---- the subtrees below the level loop, then every node listed by depth
+  // ---- the subtrees below the level loop
   {
     int h[8];
     cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, sm);
@@ -1450,22 +1399,12 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "BVH subtrees");
     total_nodes = h[0];
-    int depths = h[5] + 1;
-    if (total_nodes < 1 || total_nodes > cap || depths < 1 || depths > cap)
-      return fail(ctx, RTB_ERR_DEVICE_CHECK, "BVH node count out of range");
-    cudaMemsetAsync(depth_hist, 0, (size_t)depths * 4, sm);
-    k_depth_hist<<<blocks(total_nodes), 256, 0, sm>>>(N, total_nodes, depth_hist);
-    std::vector<int> hist(depths);
-    cudaMemcpyAsync(hist.data(), depth_hist, (size_t)depths * 4, cudaMemcpyDeviceToHost, sm);
-    e = cudaStreamSynchronize(sm);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "BVH depth histogram");
-    level_begin.assign(1, 0);
-    for (int d = 0; d < depths; ++d) level_begin.push_back(level_begin.back() + hist[d]);
-    cudaMemcpyAsync(depth_hist, level_begin.data(), (size_t)depths * 4, cudaMemcpyHostToDevice, sm);
-    k_depth_scatter<<<blocks(total_nodes), 256, 0, sm>>>(N, total_nodes, depth_hist, all_nodes);
+    if (total_nodes < 1 || total_nodes > cap) return fail(ctx, RTB_ERR_DEVICE_CHECK, "BVH node count out of range");
   }
   int rotation_count = 0;
   if (rotate) {
+    std::vector<int> level_begin;
+    int* all_nodes = W.alloc<int>(cap);
     double* rcost = W.alloc<double>(cap);
     int* rot = W.alloc<int>(2);
     if (!W.ok) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "BVH rotation workspace");
@@ -1497,8 +1436,7 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
     cudaMemcpyAsync(counters + 5, &depth, 4, cudaMemcpyHostToDevice, sm);
     cudaStreamSynchronize(sm);
   }
-  rtb_status fs = finish_build(ctx, desc, cfg, W, c, P, I, N, all_nodes, level_begin, roots, total_nodes,
-                               counters, out, stats);
+  rtb_status fs = finish_build(ctx, desc, cfg, W, c, in, P, I, N, roots, total_nodes, counters, out, stats);
   if (fs == RTB_OK && stats) {
     stats->rotation_count = rotation_count;
     stats->sequential_nodes = sequential_nodes;

@@ -134,9 +134,9 @@ struct Nodes {
   int* split_pos;
   Box* bounds;
   int* size;
-  int* pre;
+  int* parent;  // -1 at a root
+  int* visits;  // of the bottom-up pass
   int* rsize;   // primitive references under the node
-  int* rfirst;  // the node's first reference in preorder (leaf ranges after rotations)
   double* sah[3];   // generalized, uniform, weighted
 };
 
@@ -190,78 +190,113 @@ __global__ void k_update_keys(const Nodes N, const int* level_of, int level, int
   key[j] = j < N.start[node] + N.split_pos[node] ? N.left[node] : N.right[node];
 }
 
-// Bottom-up subtree sizes and SAH statistics (GpuScene.java:810-838) over one level.
-__global__ void k_bottom_up(const Prims P, IdxSet I, Nodes N, const int* nodes, int k,
-                            double traversal) {
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= k) return;
-  int node = nodes[g];
-  if (N.leaf[node]) {
-    N.size[node] = 1;
-    N.rsize[node] = N.end[node] - N.start[node];
-    double c0 = 0.0, c1 = 0.0, c2 = 0.0;
-    for (int j = N.start[node]; j < N.end[node]; ++j) {
-      int p = current_prim(I.a, N.order_axis[node], j);
-      c0 = c0 + P.w[p];
-      c1 = c1 + 1.0;
-      c2 = c2 + P.measured[p];
-    }
-    N.sah[0][node] = c0;
-    N.sah[1][node] = c1;
-    N.sah[2][node] = c2;
-    return;
-  }
-  int l = N.left[node], r = N.right[node];
-  N.size[node] = 1 + N.size[l] + N.size[r];
-  N.rsize[node] = N.rsize[l] + N.rsize[r];
-  double area = surface_area(N.bounds[node]);
-  double al = surface_area(N.bounds[l]), ar = surface_area(N.bounds[r]);
-  for (int m = 0; m < 3; ++m) {
-    double v;
-    if (!(area > 0.0)) {
-      v = N.sah[m][l] + N.sah[m][r];
-    } else {
-      double x = al / area * N.sah[m][l];
-      double y = ar / area * N.sah[m][r];
-      v = (traversal + x) + y;
-    }
-    N.sah[m][node] = v;
-  }
-}
+// ---- finishing passes: three launches over all nodes, whatever the tree's depth (a launch per
+// level took 34 launches of some 5 us each at 10k primitives, 58 at 1M)
 
-__global__ void k_preorder(Nodes N, const int* nodes, int k) {
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= k) return;
-  int node = nodes[g];
-  if (N.leaf[node]) return;
-  int l = N.left[node];
-  N.pre[l] = N.pre[node] + 1;
-  N.rfirst[l] = N.rfirst[node];
-  N.rfirst[N.right[node]] = N.rfirst[node] + N.rsize[l];
-  N.pre[N.right[node]] = N.pre[node] + 1 + N.size[l];
-}
-
-// Flattened reference layout (flattenBvh / leafKind, GpuScene.java:772-808).
-__global__ void k_flatten(const Prims P, IdxSet I, const Nodes N, int count, float* node_bounds,
-                          int* node_data, int* refs) {
+__global__ void k_parents(Nodes N, int count, int roots) {
   int node = blockIdx.x * blockDim.x + threadIdx.x;
   if (node >= count) return;
-  int at = N.pre[node];
+  if (node < roots) N.parent[node] = -1;
+  N.visits[node] = 0;
+  if (N.leaf[node]) return;
+  N.parent[N.left[node]] = node;
+  N.parent[N.right[node]] = node;
+}
+
+// Subtree sizes and SAH statistics (GpuScene.java:810-838): every leaf's thread climbs, and of
+// a node's two children the one that arrives last goes on with the node, whose values are the
+// same expression of both children's whichever that is.  The children's values pass between
+// SMs: written before a fence and the visit, read past the L1 cache after it.
+__global__ void k_bottom_up(const Prims P, IdxSet I, Nodes N, int count, double traversal) {
+  int node = blockIdx.x * blockDim.x + threadIdx.x;
+  if (node >= count || !N.leaf[node]) return;
+  N.size[node] = 1;
+  N.rsize[node] = N.end[node] - N.start[node];
+  double c0 = 0.0, c1 = 0.0, c2 = 0.0;
+  for (int j = N.start[node]; j < N.end[node]; ++j) {
+    int p = current_prim(I.a, N.order_axis[node], j);
+    c0 = c0 + P.w[p];
+    c1 = c1 + 1.0;
+    c2 = c2 + P.measured[p];
+  }
+  N.sah[0][node] = c0;
+  N.sah[1][node] = c1;
+  N.sah[2][node] = c2;
+  while ((node = N.parent[node]) >= 0) {
+    __threadfence();
+    if (atomicAdd(N.visits + node, 1) == 0) return;
+    __threadfence();
+    const int l = N.left[node], r = N.right[node];
+    N.size[node] = 1 + __ldcg(N.size + l) + __ldcg(N.size + r);
+    N.rsize[node] = __ldcg(N.rsize + l) + __ldcg(N.rsize + r);
+    const double area = surface_area(N.bounds[node]);
+    const double al = surface_area(N.bounds[l]), ar = surface_area(N.bounds[r]);
+    for (int m = 0; m < 3; ++m) {
+      const double sl = __ldcg(N.sah[m] + l), sr = __ldcg(N.sah[m] + r);
+      double v;
+      if (!(area > 0.0)) {
+        v = sl + sr;
+      } else {
+        double x = al / area * sl;
+        double y = ar / area * sr;
+        v = (traversal + x) + y;
+      }
+      N.sah[m][node] = v;
+    }
+  }
+}
+
+// What the host reads back of a finished build.
+struct BuildResult {
+  double sah[4][3];  // per root
+};
+
+// The flattened reference layout (flattenBvh / leafKind, GpuScene.java:772-808).  A node's preorder
+// index and first reference are sums over the path to its root: one for every step down, the
+// left sibling's sizes for every step to the right, the earlier trees' sizes at the root.  A full
+// binary tree of s nodes has (s + 1) / 2 leaves, so the same walk gives an interior node's rank
+// among the interior nodes.
+__global__ void k_flatten(const Prims P, IdxSet I, const Nodes N, int count, int roots, float* node_bounds,
+                          int* node_data, int* refs, int* ranks, int* root_out, BuildResult* result) {
+  const int node = blockIdx.x * blockDim.x + threadIdx.x;
+  if (node >= count) return;
+  int at = 0, f = 0, leaves = 0, c = node;
+  for (int p = N.parent[c]; p >= 0; c = p, p = N.parent[c]) {
+    const int l = N.left[p];
+    at += 1;
+    if (c != l) {
+      const int size = N.size[l];
+      at += size;
+      leaves += (size + 1) >> 1;
+      f += N.rsize[l];
+    }
+  }
+  for (int r = 0; r < c; ++r) {  // c is the root now, and the roots are the first nodes
+    const int size = N.size[r];
+    at += size;
+    leaves += (size + 1) >> 1;
+    f += N.rsize[r];
+  }
+  if (node < roots) {
+    root_out[node] = at;
+    for (int m = 0; m < 3; ++m) result->sah[node][m] = N.sah[m][node];
+  }
   Box b = N.bounds[node];
   for (int k = 0; k < 3; ++k) {
     node_bounds[6 * (size_t)at + k] = b.mn[k];
     node_bounds[6 * (size_t)at + 3 + k] = b.mx[k];
   }
   int* d = node_data + 4 * (size_t)at;
+  ranks[at] = at - leaves;
   if (!N.leaf[node]) {
-    d[0] = N.pre[N.left[node]];
-    d[1] = N.pre[N.right[node]];
+    d[0] = at + 1;
+    d[1] = at + 1 + N.size[N.left[node]];
     d[2] = -1;
     d[3] = 0;
     return;
   }
   // references in preorder of the leaves (after rotations that differs from array order)
-  int s = N.start[node], e = N.end[node], f = N.rfirst[node];
+  int s = N.start[node], e = N.end[node];
   int t0 = -1;
   bool mixed = false;
   for (int j = s; j < e; ++j) {
@@ -387,9 +422,9 @@ inline Nodes alloc_nodes(Workspace& W, int cap) {
   N.split_pos = W.alloc<int>(cap);
   N.bounds = W.alloc<Box>(cap);
   N.size = W.alloc<int>(cap);
-  N.pre = W.alloc<int>(cap);
+  N.parent = W.alloc<int>(cap);
+  N.visits = W.alloc<int>(cap);
   N.rsize = W.alloc<int>(cap);
-  N.rfirst = W.alloc<int>(cap);
   for (int m = 0; m < 3; ++m) N.sah[m] = W.alloc<double>(cap);
   return N;
 }
@@ -414,60 +449,47 @@ inline int root_ranges(const BuildCfg& c, bool per_type, int* rs, int* re) {
   return roots;
 }
 
-// Bottom-up sizes and SAH statistics, preorder indices, the flattened arrays and the
-// resident scene.  all_nodes lists the nodes level by level (level_begin offsets);
-// counters + 2 holds {leaves, min occupancy, max occupancy, max depth}.
+// Sizes and SAH statistics, the flattened arrays and the resident scene.  counters + 2 holds
+// {leaves, min occupancy, max occupancy, max depth}.
 inline rtb_status finish_build(rtb_context* ctx, const rtb_scene_desc* desc, const rtb_build_config* cfg,
-                               Workspace& W, const BuildCfg& c, const Prims& P, const IdxSet& I,
-                               const Nodes& N, const int* all_nodes, const std::vector<int>& level_begin,
-                               int roots, int total_nodes, const int* counters, rtb_scene** out,
-                               rtb_bvh_stats* stats) {
+                               Workspace& W, const BuildCfg& c, const PrimInputs& in, const Prims& P,
+                               const IdxSet& I, const Nodes& N, int roots, int total_nodes, const int* counters,
+                               rtb_scene** out, rtb_bvh_stats* stats) {
   cudaStream_t sm = ctx->stream;
   const int n = c.total;
-  for (int L = (int)level_begin.size() - 2; L >= 0; --L) {
-    int b = level_begin[L], cnt = level_begin[L + 1] - b;
-    k_bottom_up<<<blocks(cnt, 128), 128, 0, sm>>>(P, I, N, all_nodes + b, cnt, c.traversal);
-  }
-  // Tree roots in order: preorder index = sizes of the previous trees.
-  std::vector<int> h_size(roots), h_rsize(roots);
-  for (int r = 0; r < roots; ++r) cudaMemcpyAsync(&h_size[r], N.size + r, 4, cudaMemcpyDeviceToHost, sm);
-  for (int r = 0; r < roots; ++r) cudaMemcpyAsync(&h_rsize[r], N.rsize + r, 4, cudaMemcpyDeviceToHost, sm);
-  double h_sah[4][3];
-  for (int r = 0; r < roots; ++r)
-    for (int m = 0; m < 3; ++m) cudaMemcpyAsync(&h_sah[r][m], N.sah[m] + r, 8, cudaMemcpyDeviceToHost, sm);
-  cudaError_t e = cudaStreamSynchronize(sm);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "BVH sizes");
-  std::vector<int> h_pre(roots), h_rfirst(roots);
-  int acc = 0;
-  for (int r = 0; r < roots; ++r) {
-    h_pre[r] = acc;
-    acc += h_size[r];
-    h_rfirst[r] = r ? h_rfirst[r - 1] + h_rsize[r - 1] : 0;
-  }
-  cudaMemcpyAsync(N.pre, h_pre.data(), roots * 4, cudaMemcpyHostToDevice, sm);
-  cudaMemcpyAsync(N.rfirst, h_rfirst.data(), roots * 4, cudaMemcpyHostToDevice, sm);
-  for (int L = 0; L + 1 < (int)level_begin.size(); ++L) {
-    int b = level_begin[L], cnt = level_begin[L + 1] - b;
-    k_preorder<<<blocks(cnt, 128), 128, 0, sm>>>(N, all_nodes + b, cnt);
-  }
   float* o_nb = W.alloc<float>((size_t)total_nodes * 6);
   int* o_nd = W.alloc<int>((size_t)total_nodes * 4);
+  int* o_rank = W.alloc<int>(total_nodes);
   int* o_refs = W.alloc<int>(n);
   int* o_roots = W.alloc<int>(4);
+  BuildResult* o_result = W.alloc<BuildResult>(1);
   if (!W.ok) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "BVH output");
-  k_flatten<<<blocks(total_nodes, 128), 128, 0, sm>>>(P, I, N, total_nodes, o_nb, o_nd, o_refs);
-  cudaMemcpyAsync(o_roots, h_pre.data(), roots * 4, cudaMemcpyHostToDevice, sm);
+  k_parents<<<blocks(total_nodes), 256, 0, sm>>>(N, total_nodes, roots);
+  k_bottom_up<<<blocks(total_nodes, 128), 128, 0, sm>>>(P, I, N, total_nodes, c.traversal);
+  k_flatten<<<blocks(total_nodes, 128), 128, 0, sm>>>(P, I, N, total_nodes, roots, o_nb, o_nd, o_refs, o_rank,
+                                                      o_roots, o_result);
   cudaEventRecord(ctx->ev1, sm);
-  int h_stats[4];
-  cudaMemcpyAsync(h_stats, counters + 2, sizeof(h_stats), cudaMemcpyDeviceToHost, sm);
-  e = cudaStreamSynchronize(sm);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "BVH flatten");
+  // Read back through pinned memory, so that the host goes on; scene_create waits for the stream.
+  struct Back {
+    int stats[4];
+    BuildResult result;
+  };
+  Back* back = (Back*)pinned(ctx, sizeof(Back));
+  if (!back) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "pinned staging");
+  cudaMemcpyAsync(back->stats, counters + 2, sizeof(back->stats), cudaMemcpyDeviceToHost, sm);
+  cudaMemcpyAsync(&back->result, o_result, sizeof(BuildResult), cudaMemcpyDeviceToHost, sm);
+  BuiltTree tree{o_nb, o_nd, total_nodes, o_refs, n, o_roots, roots, o_rank, (total_nodes - roots) / 2, in.sph, in.box};
+  rtb_status s = scene_create(ctx, desc, nullptr, &tree, out);
+  if (s != RTB_OK) return s;
+  const int* h_stats = back->stats;
+  const BuildResult& h_result = back->result;
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  if (total_nodes != 2 * h_stats[0] - roots)
+  if (total_nodes != 2 * h_stats[0] - roots) {
+    scene_free(*out, sm);
+    *out = nullptr;
     return fail(ctx, RTB_ERR_DEVICE_CHECK, "A binary BVH forest must contain 2 * leafCount - rootCount nodes.");
-  rtb_status s = scene_create(ctx, desc, nullptr, o_nb, o_nd, total_nodes, o_refs, n, o_roots, roots, out);
-  if (s != RTB_OK) return s;
+  }
   if (stats) {
     stats->node_count = total_nodes;
     stats->root_count = roots;
@@ -479,9 +501,9 @@ inline rtb_status finish_build(rtb_context* ctx, const rtb_scene_desc* desc, con
     stats->max_leaf_occupancy = h_stats[2];
     double g = 0.0, u = 0.0, w = 0.0;
     for (int r = 0; r < roots; ++r) {
-      u = u + h_sah[r][1];
-      w = w + h_sah[r][2];
-      g = g + h_sah[r][0];
+      u = u + h_result.sah[r][1];
+      w = w + h_result.sah[r][2];
+      g = g + h_result.sah[r][0];
     }
     stats->generalized_sah_cost = g;
     stats->uniform_sah_cost = u;

@@ -114,10 +114,26 @@ void* stage(rtb_context* ctx, size_t bytes);
 void* pinned(rtb_context* ctx, size_t bytes);
 
 // rtb_scene.cu
+// A tree that a builder made on the device, in the reference's flattened layout, with what the
+// builder knows of it: every interior node's rank among the interior nodes in preorder and their
+// number, that every primitive is referenced once, and the uploaded spheres and boxes.
+struct BuiltTree {
+  const float* node_bounds;
+  const int* node_data;
+  int node_count;
+  const int* refs;
+  int ref_count;
+  const int* roots;
+  int root_count;
+  const int* ranks;
+  int interior;
+  const float* spheres;
+  const float* boxes;
+};
+// The resident scene, with a caller's tree, a builder's, or none.  Returns with the context's
+// stream finished.
 rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* desc, const rtb_bvh_desc* host_bvh,
-                        const float* d_node_bounds, const int* d_node_data, int node_count,
-                        const int* d_refs, int ref_count, const int* d_roots, int root_count,
-                        rtb_scene** out);
+                        const BuiltTree* built, rtb_scene** out);
 void scene_free(rtb_scene* s, cudaStream_t stream);
 
 // rtb_render.cu

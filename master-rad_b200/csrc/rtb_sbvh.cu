@@ -440,7 +440,7 @@ rtb_status build_bvh_sbvh(rtb_context* ctx, const rtb_scene_desc* desc, const rt
   if (stats) *stats = rtb_bvh_stats{};
   auto t0 = std::chrono::steady_clock::now();
   if (c.total == 0) {
-    rtb_status s = scene_create(ctx, desc, nullptr, nullptr, nullptr, 0, nullptr, 0, nullptr, 0, out);
+    rtb_status s = scene_create(ctx, desc, nullptr, nullptr, out);
     if (stats) stats->leaf_size = cfg->leaf_size;
     return s;
   }
@@ -541,7 +541,7 @@ rtb_status build_bvh_sbvh(rtb_context* ctx, const rtb_scene_desc* desc, const rt
     return fail(ctx, RTB_ERR_DEVICE_CHECK, "SBVH flattening is incomplete");
   int root = 0;
   rtb_bvh_desc hb{nb.data(), nd.data(), count, orefs.data(), nrefs, &root, 1};
-  rtb_status s = scene_create(ctx, desc, &hb, nullptr, nullptr, 0, nullptr, 0, nullptr, 0, out);
+  rtb_status s = scene_create(ctx, desc, &hb, nullptr, out);
   if (s != RTB_OK) return s;
   if (stats) {
     stats->node_count = count;

@@ -121,7 +121,7 @@ __global__ void k_ref_remap(const int* refs, int n, const int* ranks, int* refs_
   int ref = refs[j];
   int t = (int)((unsigned)ref >> kTypeShift);
   int idx = ref & kIndexMask;
-  int s = ranks[t * (size_t)n + j];
+  int s = ranks[t * (size_t)n + j] - base[t];
   orig_of_new[base[t] + s] = idx;
   refs_out[j] = (int)((unsigned)t << kTypeShift) | s;
 }
@@ -267,8 +267,7 @@ void scene_free(rtb_scene* s, cudaStream_t stream) {
 }
 
 rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* d, const rtb_bvh_desc* hb,
-                        const float* d_nb, const int* d_nd, int node_count, const int* d_refs,
-                        int ref_count, const int* d_roots, int root_count, rtb_scene** out) {
+                        const BuiltTree* built, rtb_scene** out) {
   if (!d || !out) return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "scene description is required");
   const int cnt[6] = {d->sphere_count, d->box_count, d->plane_count, d->affine_sphere_count,
                       d->affine_box_count, d->material_count};
@@ -287,10 +286,14 @@ rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* d, const rtb_bvh
         (hb->primitive_ref_count > 0 && !hb->primitive_refs) ||
         (hb->root_count > 0 && !hb->root_indices))
       return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "invalid BVH description");
-    node_count = hb->node_count;
-    ref_count = hb->primitive_ref_count;
-    root_count = hb->root_count;
   }
+  const float* d_nb = built ? built->node_bounds : nullptr;
+  const int* d_nd = built ? built->node_data : nullptr;
+  const int* d_refs = built ? built->refs : nullptr;
+  const int* d_roots = built ? built->roots : nullptr;
+  const int node_count = hb ? hb->node_count : built ? built->node_count : 0;
+  const int ref_count = hb ? hb->primitive_ref_count : built ? built->ref_count : 0;
+  const int root_count = hb ? hb->root_count : built ? built->root_count : 0;
   bool has_bvh = node_count > 0 && ref_count > 0 && root_count > 0;
   if (has_bvh && (long long)node_count > 2LL * ref_count + 8)
     return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "BVH has more nodes than a binary tree over its references");
@@ -300,7 +303,9 @@ rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* d, const rtb_bvh
   // ---- staging: raw packed arrays (+ host BVH) in one device buffer
   Arena st;
   size_t raw_off[6];
-  for (int k = 0; k < 6; ++k) raw_off[k] = st.take<float>((size_t)cnt[k] * fpr[k]);
+  // a builder has uploaded the spheres and boxes already
+  const float* uploaded[6] = {built ? built->spheres : nullptr, built ? built->boxes : nullptr};
+  for (int k = 0; k < 6; ++k) raw_off[k] = st.take<float>(uploaded[k] ? 0 : (size_t)cnt[k] * fpr[k]);
   size_t hb_off[4] = {0, 0, 0, 0};
   if (hb && has_bvh) {
     hb_off[0] = st.take<float>((size_t)node_count * 6);
@@ -317,14 +322,16 @@ rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* d, const rtb_bvh
   {
     int* dummy = nullptr;
     cub::DeviceScan::ExclusiveSum(nullptr, scan_tmp_bytes, dummy, dummy,
-                                  4 * std::max(ref_count, std::max(node_count, 1)));
+                                  4LL * std::max(ref_count, std::max(node_count, 1)));
   }
   size_t tmp_off = st.take<char>(scan_tmp_bytes);
   char* sb = (char*)stage(ctx, st.off);
   if (!sb) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "staging allocation failed");
   cudaStream_t sm = ctx->stream;
+  const float* raw[6];
+  for (int k = 0; k < 6; ++k) raw[k] = uploaded[k] ? uploaded[k] : (const float*)(sb + raw_off[k]);
   for (int k = 0; k < 6; ++k)
-    if (cnt[k] > 0)
+    if (cnt[k] > 0 && !uploaded[k])
       cudaMemcpyAsync(sb + raw_off[k], src[k], (size_t)cnt[k] * fpr[k] * 4, cudaMemcpyHostToDevice, sm);
   if (hb && has_bvh) {
     cudaMemcpyAsync(sb + hb_off[0], hb->node_bounds, (size_t)node_count * 24, cudaMemcpyHostToDevice, sm);
@@ -371,14 +378,18 @@ rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* d, const rtb_bvh
     h_meta[5 + t] = b;
     h_meta[9 + t] = b;
   }
-  // Interior-node count is needed for the node array size; compute it on the device.
+  // The interior nodes' ranks, and their number for the node array's size: a builder's, or
+  // computed on the device.
   int* iflag = (int*)(sb + iflag_off);
-  int* irank = (int*)(sb + ranks_off);  // reused below only after the node conversion
+  const int* irank = (const int*)(sb + ranks_off);  // reused below only after the node conversion
   cudaMemcpyAsync(err, h_meta, sizeof(h_meta), cudaMemcpyHostToDevice, sm);
-  if (has_bvh) {
+  if (has_bvh && built) {
+    irank = built->ranks;
+    interior = built->interior;
+  } else if (has_bvh) {
     k_interior_flags<<<blocks(node_count), 256, 0, sm>>>(d_nd, node_count, iflag);
     size_t tb = scan_tmp_bytes;
-    cub::DeviceScan::ExclusiveSum(sb + tmp_off, tb, iflag, irank, node_count, sm);
+    cub::DeviceScan::ExclusiveSum(sb + tmp_off, tb, iflag, (int*)(sb + ranks_off), node_count, sm);
     int last_flag = 0, last_rank = 0;
     cudaMemcpyAsync(&last_flag, iflag + node_count - 1, 4, cudaMemcpyDeviceToHost, sm);
     cudaMemcpyAsync(&last_rank, irank + node_count - 1, 4, cudaMemcpyDeviceToHost, sm);
@@ -422,28 +433,30 @@ rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* d, const rtb_bvh
     k_ref_flags<<<blocks(ref_count), 256, 0, sm>>>(d_refs, ref_count, d_counts, flags, seen,
                                                     d_seen_base, err);
     int herr = 0;
-    cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, sm);
-    e = cudaStreamSynchronize(sm);
-    if (e != cudaSuccess) {
-      scene_free(s, sm);
-      return cuda_fail(ctx, e, "BVH reference check");
-    }
-    if (herr & 1) {
-      scene_free(s, sm);
-      return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "BVH reference index out of range");
-    }
-    if (herr & (4 | 8)) {
-      scene_free(s, sm);
-      return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "BVH node child or leaf range out of range");
-    }
-    // A permutation needs every primitive referenced exactly once (no duplicates).
-    permute = !(herr & 2) && ref_count == nbounded;
-    if (permute) {
-      for (int t = 0; t < 4; ++t) {
-        size_t tb = scan_tmp_bytes;
-        cub::DeviceScan::ExclusiveSum(sb + tmp_off, tb, flags + (size_t)t * ref_count,
-                                      ranks + (size_t)t * ref_count, ref_count, sm);
+    if (!built) {
+      cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, sm);
+      e = cudaStreamSynchronize(sm);
+      if (e != cudaSuccess) {
+        scene_free(s, sm);
+        return cuda_fail(ctx, e, "BVH reference check");
       }
+      if (herr & 1) {
+        scene_free(s, sm);
+        return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "BVH reference index out of range");
+      }
+      if (herr & (4 | 8)) {
+        scene_free(s, sm);
+        return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "BVH node child or leaf range out of range");
+      }
+    }
+    // A permutation needs every primitive referenced exactly once (no duplicates), as a builder
+    // does.
+    permute = built || (!(herr & 2) && ref_count == nbounded);
+    if (permute) {
+      // One scan over the four types' flags, one type after the other: a reference's sum is its
+      // rank among its type's plus the number of primitives of the types before, base[type].
+      size_t tb = scan_tmp_bytes;
+      cub::DeviceScan::ExclusiveSum(sb + tmp_off, tb, flags, ranks, 4LL * ref_count, sm);
       k_ref_remap<<<blocks(ref_count), 256, 0, sm>>>(d_refs, ref_count, ranks, (int*)(A + o_refs),
                                                       oon, d_base);
     } else {
@@ -456,31 +469,31 @@ rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* d, const rtb_bvh
   int* orig = (int*)(A + o_orig);
   int base[4] = {h_meta[9], h_meta[10], h_meta[11], h_meta[12]};
   if (nprim[0])
-    k_pack_spheres<<<blocks(nprim[0]), 256, 0, sm>>>((const float*)(sb + raw_off[0]), nprim[0],
+    k_pack_spheres<<<blocks(nprim[0]), 256, 0, sm>>>(raw[0], nprim[0],
                                                       permute ? oon + base[0] : nullptr,
                                                       (float4*)(A + o_sph), mat + base[0], orig + base[0],
                                                       cnt[5], err);
   if (nprim[1])
-    k_pack_boxes<<<blocks(nprim[1]), 256, 0, sm>>>((const float*)(sb + raw_off[1]), nprim[1],
+    k_pack_boxes<<<blocks(nprim[1]), 256, 0, sm>>>(raw[1], nprim[1],
                                                     permute ? oon + base[1] : nullptr,
                                                     (float4*)(A + o_box), mat + base[1], orig + base[1],
                                                     cnt[5], err);
   if (nprim[2])
-    k_pack_affine<<<blocks(nprim[2]), 256, 0, sm>>>((const float*)(sb + raw_off[3]), nprim[2],
+    k_pack_affine<<<blocks(nprim[2]), 256, 0, sm>>>(raw[3], nprim[2],
                                                      permute ? oon + base[2] : nullptr,
                                                      (float4*)(A + o_asp), (float*)(A + o_asn),
                                                      mat + base[2], orig + base[2], cnt[5], err);
   if (nprim[3])
-    k_pack_affine<<<blocks(nprim[3]), 256, 0, sm>>>((const float*)(sb + raw_off[4]), nprim[3],
+    k_pack_affine<<<blocks(nprim[3]), 256, 0, sm>>>(raw[4], nprim[3],
                                                      permute ? oon + base[3] : nullptr,
                                                      (float4*)(A + o_abx), (float*)(A + o_abn),
                                                      mat + base[3], orig + base[3], cnt[5], err);
   if (cnt[2])
-    k_pack_planes<<<blocks(cnt[2]), 256, 0, sm>>>((const float*)(sb + raw_off[2]), cnt[2],
+    k_pack_planes<<<blocks(cnt[2]), 256, 0, sm>>>(raw[2], cnt[2],
                                                    (float4*)(A + o_pl), (float*)(A + o_plf),
                                                    cnt[5], err);
   if (cnt[5])
-    k_pack_materials<<<blocks(cnt[5]), 256, 0, sm>>>((const float*)(sb + raw_off[5]), cnt[5],
+    k_pack_materials<<<blocks(cnt[5]), 256, 0, sm>>>(raw[5], cnt[5],
                                                       (float4*)(A + o_mt));
   int herr = 0;
   cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, sm);
