@@ -664,7 +664,7 @@ rtb_status build_bvh_binned(rtb_context* ctx, const rtb_scene_desc* desc, const 
   }
   IdxSet I;
   for (int a = 0; a < 3; ++a) I.a[a] = idx;
-  return finish_build(ctx, desc, cfg, W, c, in, P, I, N, roots, total_nodes, counters, out, stats);
+  return finish_build(ctx, desc, cfg, W, c, in, P, I, N, roots, total_nodes, total_nodes, counters, out, stats);
 }
 
 }  // namespace rtb

@@ -597,22 +597,41 @@ __global__ void k_argmin_flat(int blocks_total, const double* part_cost, const l
   if (part_cost[b] == best_cost[g]) atomicMin(best_flat + g, part_flat[b]);
 }
 
-// ---- whole subtrees of at most kSubtreeSize primitives, one warp each
+// ---- node ids
 //
-// The recursion of BvhBuildState.build (GpuScene.java:1424-1447) below such a node runs in
-// one warp, depth first, with the node's three axis orders in shared memory: per node and
-// axis the suffix boxes and weights (weights summed one by one in the reference's order,
-// the same additions as its loop), then the prefix pass evaluating every split's cost in the
-// reference's expression order, the first minimum over (axis, position), the leaf rule in
-// the node's current order, and a stable partition of the other two axis orders.  Every
-// number is the one the level loop would compute for the same node; the subtree only saves
-// the per-level passes over all primitives (scans, gathers, argmin blocks) that dominate
-// the deep levels.
-constexpr int kSubtreeSize = kSeqNodeSize;
+// A split puts a boundary between two positions that no other split of the tree uses, so the
+// children of a node split at position q are nodes roots + 2 q and the next: ids need no counter.
+// They are sparse; N.leaf is -1 where there is no node.
+__device__ __forceinline__ int child_id(int roots, int split) { return roots + 2 * split; }
+
+// ---- whole subtrees of at most kSubtreeSize primitives, one block each
+//
+// The recursion of BvhBuildState.build (GpuScene.java:1424-1447) below such a node, depth first,
+// with the node's three axis orders in shared memory: per node and axis the suffix boxes and
+// weights (weights summed one by one in the reference's order, the same additions as its loop),
+// then the prefix pass evaluating every split's cost in the reference's expression order, the
+// first minimum over (axis, position), the leaf rule in the node's current order, and a stable
+// partition of the other two axis orders.  Every number is the one the level loop would compute
+// for the same node; the subtree only saves the per-level passes over all primitives (scans,
+// gathers, argmin blocks) that dominate the deep levels.
+//
+// k_subtrees builds the nodes of more than kWarpNode primitives, one block of three warps a
+// subtree and one warp an axis; what is left, nodes of at most kWarpNode, is listed for
+// k_small_subtrees, where one warp builds all below one of them with no barrier.  Of at most
+// kPackNode primitives the three axes share the warp, eight lanes each: most nodes of a tree are
+// that small, and as the block's they were mostly idle lanes and barriers.  10k primitives: 950 ->
+// 94 + 68 us, with the ids above (a split took a round trip to a global counter) and centroids
+// from the staged boxes; the whole build 2.60 -> 1.65 ms, of 1M 14.9 -> 11.5 ms.
+// k_small_subtrees' blocks are single warps so that every branch lies on a value that the compiler
+// knows is the same in all lanes (read from shared memory at one address): where it does not,
+// each shuffle gets a branch of its own, and the same code inside the three-warp block took 1.6 ms.
+constexpr int kSubtreeSize = 512;  // 256: one level-loop round more, 10k 1.69 against 1.65 ms, 1M 11.7 against 11.5
 constexpr int kSubtreeThreads = 96;  // one warp per axis
+constexpr int kWarpNode = 32, kPackNode = 8;
 #ifndef RTB_SUBTREE_BLOCKS_PER_SM
-#define RTB_SUBTREE_BLOCKS_PER_SM 9  // 22.8 KB of shared memory and <= 72 registers each
+#define RTB_SUBTREE_BLOCKS_PER_SM 5  // 37 KB of shared memory and 80 registers each
 #endif
+constexpr int kSmallBlocksPerSm = 32;
 
 struct SubtreeSmem {
   // The subtree's primitives get local slots 0..M-1 (axis 0's order at the root); the
@@ -627,11 +646,22 @@ struct SubtreeSmem {
     double sterm[3][kSubtreeSize];  // per axis: suffix area x suffix weight of the current node
     int tmp[3][kSubtreeSize];       // per axis: partition scratch
   };
-  int4 stack[kSubtreeSize];     // pending nodes, depth first: node, start, end,
-                                // depth << 2 | (order axis + 1)
+  // Pending nodes, disjoint ranges of more than kWarpNode positions: node, start, end,
+  // depth << 2 | (order axis + 1).
+  int4 stack[kSubtreeSize / kWarpNode];
   double best_cost[3];
-  long long best_flat[3];
-  int sp, child;
+  int best_flat[3];
+  int sp;
+};
+
+struct SmallSmem {
+  Box lbox[kWarpNode];  // by slot, as in SubtreeSmem
+  double lw[kWarpNode];
+  int gid[kWarpNode];
+  int idx[3][kWarpNode];
+  unsigned char lside[kWarpNode];
+  int4 stack[kWarpNode];
+  int leaf, flat;
 };
 
 __device__ __forceinline__ Box empty_box() {
@@ -686,21 +716,233 @@ __device__ __forceinline__ double warp_sequential_sum(double w, double& acc, int
   return mine;
 }
 
-__device__ __forceinline__ bool lex_less(double c, long long f, double bc, long long bf) {
+__device__ __forceinline__ bool lex_less(double c, int f, double bc, int bf) {
   return c < bc || (c == bc && f < bf);
 }
 
-// One block of three warps per subtree root: warp a sweeps axis a of the current node,
-// the block takes the first minimum over the three axes' winners, and the warps of the two
-// other axes partition their orders.  Every decision is computed identically by all threads
-// (or broadcast through shared memory), so the block's barriers are uniform.
+// A staged primitive's centroid, as k_prims computes it from the same bounds.
+__device__ __forceinline__ double box_centroid(const Box& b, int axis) {
+  return ((double)b.mn[axis] + (double)b.mx[axis]) * 0.5;
+}
+
+// Splits of a node of m <= W positions on the axis of this lane's group of W lanes: the best
+// (cost, axis * m + position) of the group's positions in *best and *flat, lane by lane, and the
+// node's bounds.  W = 8: groups 0..2 are the axes, group 3 has none (axis < 0).
+template <int W>
+__device__ __forceinline__ Box group_sweep(const SmallSmem& sm, int axis, int lo, int m, double traversal,
+                                           double* best, int* flat) {
+  const int i = (int)(threadIdx.x & 31) & (W - 1);
+  const bool in = i < m && axis >= 0;
+  const int slot = in ? sm.idx[axis][lo + i] : 0;
+  Box pre = in ? sm.lbox[slot] : empty_box();
+  Box suf = pre;
+  const double w = in ? sm.lw[slot] : 0.0;
+  // suffix sums from the last position down (GpuScene.java:1476-1480) and prefix sums (1470-1475),
+  // two chains of additions side by side; positions from m up carry 0, which changes no sum
+  double sw = 0.0, pw = 0.0, down = 0.0, up = 0.0;
+  const int steps = W == 8 ? 8 : (m + 3) & ~3;
+#pragma unroll
+  for (int g0 = 0; g0 < W; g0 += 4) {
+    if (W > 8 && g0 >= steps) break;
+    double vu[4], vd[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      vu[q] = __shfl_sync(0xFFFFFFFFu, w, g0 + q, W);
+      vd[q] = __shfl_sync(0xFFFFFFFFu, w, steps - 1 - g0 - q, W);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      up = up + vu[q];
+      pw = g0 + q == i - 1 ? up : pw;  // of the positions before i
+      down = down + vd[q];
+      sw = steps - 1 - g0 - q == i ? down : sw;
+    }
+  }
+#pragma unroll
+  for (int off = 1; off < W; off <<= 1) {
+    Box u, d;
+    for (int k = 0; k < 3; ++k) {
+      u.mn[k] = __shfl_up_sync(0xFFFFFFFFu, pre.mn[k], off, W);
+      u.mx[k] = __shfl_up_sync(0xFFFFFFFFu, pre.mx[k], off, W);
+      d.mn[k] = __shfl_down_sync(0xFFFFFFFFu, suf.mn[k], off, W);
+      d.mx[k] = __shfl_down_sync(0xFFFFFFFFu, suf.mx[k], off, W);
+    }
+    if (i >= off) pre = BoxUnion()(pre, u);
+    if (i + off < W) suf = BoxUnion()(suf, d);
+  }
+  const Box node = warp_bcast(suf, 0);  // group 0's first suffix: everything
+  Box left;
+  for (int k = 0; k < 3; ++k) {
+    left.mn[k] = __shfl_up_sync(0xFFFFFFFFu, pre.mn[k], 1, W);
+    left.mx[k] = __shfl_up_sync(0xFFFFFFFFu, pre.mx[k], 1, W);
+  }
+  *best = CUDART_INF;
+  *flat = 0x7FFFFFFF;
+  if (in && i > 0) {
+    const int f = sm.idx[axis][lo], l = sm.idx[axis][lo + m - 1];
+    if (box_centroid(sm.lbox[l], axis) - box_centroid(sm.lbox[f], axis) > 1.0e-12) {
+      const double node_a = surface_area(node) * traversal;
+      const double bl = surface_area(left) * pw;
+      const double d = surface_area(suf) * sw;
+      *best = (node_a + bl) + d;
+      *flat = axis * m + i;
+    }
+  }
+  return node;
+}
+
+// The leaf rule's sequential weight sum, in the node's current order (GpuScene.java:1435-1441).
+template <class Smem>
+__device__ __forceinline__ double order_weight(const Smem& sm, const Prims& P, int oa, int s, int lo, int m) {
+  double sum = 0.0;
+  for (int j = 0; j < m; ++j) sum = sum + (oa < 0 ? P.w[s + j] : sm.lw[sm.idx[oa][lo + j]]);
+  return sum;
+}
+
+struct LeafStats {
+  int leaves, min_occ, max_occ, max_depth;
+  __device__ __forceinline__ void add(int m, int depth) {
+    leaves++;
+    min_occ = min(min_occ, m);
+    max_occ = max(max_occ, m);
+    max_depth = max(max_depth, depth);
+  }
+};
+
+// A split node's record and its children's, by one thread.
+__device__ __forceinline__ void write_split(const Nodes& N, int node, int l, int axis, int pos, int s, int e,
+                                            int depth) {
+  const int r = l + 1;
+  N.leaf[node] = 0;
+  N.left[node] = l;
+  N.right[node] = r;
+  N.split_axis[node] = axis;
+  N.split_pos[node] = pos;
+  N.start[l] = s;
+  N.end[l] = s + pos;
+  N.start[r] = s + pos;
+  N.end[r] = e;
+  N.order_axis[l] = N.order_axis[r] = axis;
+  N.depth[l] = N.depth[r] = depth + 1;
+}
+
+// Everything below each listed node of at most kWarpNode primitives, a warp (the block) a node,
+// depth first.
+__global__ void __launch_bounds__(32, kSmallBlocksPerSm) k_small_subtrees(const Prims P, IdxSet I, Nodes N,
+                                                                         const int4* list, const int* count,
+                                                                         int roots, int leaf_size,
+                                                                         double traversal, int* stats) {
+  __shared__ SmallSmem sm;
+  const int lane = threadIdx.x;
+  LeafStats st{0, 0x7FFFFFFF, 0, 0};
+  const int listed = *count;
+  for (int k = blockIdx.x; k < listed; k += gridDim.x) {
+    int4 en = list[k];
+    const int rs = en.y, M = en.z - en.y;
+    {
+      int p[3];
+      for (int a = 0; a < 3; ++a) p[a] = lane < M ? I.a[a][rs + lane] : -1 - a;
+      if (lane < M) {
+        sm.gid[lane] = p[0];
+        sm.lbox[lane] = P.box[p[0]];
+        sm.lw[lane] = P.w[p[0]];
+        sm.idx[0][lane] = lane;
+      }
+      int s1 = 0, s2 = 0;
+      for (int j = 0; j < M; ++j) {
+        const int q = __shfl_sync(0xFFFFFFFFu, p[0], j);
+        s1 = q == p[1] ? j : s1;
+        s2 = q == p[2] ? j : s2;
+      }
+      if (lane < M) sm.idx[1][lane] = s1, sm.idx[2][lane] = s2;
+    }
+    __syncwarp();
+    int sp = 0;
+    while (true) {
+      const int node = en.x, s = en.y, e = en.z, m = e - s, lo = s - rs;
+      const int oa = (en.w & 3) - 1, depth = en.w >> 2;
+      double best = CUDART_INF;
+      int flat = 0x7FFFFFFF;
+      Box nb;
+      if (m == 1) {
+        nb = sm.lbox[sm.idx[0][lo]];
+      } else if (m <= kPackNode) {
+        nb = group_sweep<kPackNode>(sm, lane < 24 ? lane >> 3 : -1, lo, m, traversal, &best, &flat);
+      } else {
+        for (int a = 0; a < 3; ++a) {
+          double c;
+          int f;
+          nb = group_sweep<32>(sm, a, lo, m, traversal, &c, &f);
+          if (lex_less(c, f, best, flat)) best = c, flat = f;
+        }
+      }
+      if (m > 1) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+          const double oc = __shfl_xor_sync(0xFFFFFFFFu, best, off);
+          const int of = __shfl_xor_sync(0xFFFFFFFFu, flat, off);
+          if (lex_less(oc, of, best, flat)) best = oc, flat = of;
+        }
+      }
+      if (lane == 0) {
+        int leaf = m == 1 || best == CUDART_INF;
+        if (!leaf && m <= leaf_size && !(best < surface_area(nb) * order_weight(sm, P, oa, s, lo, m))) leaf = 1;
+        sm.leaf = leaf;
+        sm.flat = flat;
+        N.bounds[node] = nb;
+        N.split_axis[node] = -1;
+        if (leaf) {
+          N.leaf[node] = 1;
+          st.add(m, depth);
+        }
+      }
+      __syncwarp();
+      if (sm.leaf) {
+        if (sp == 0) break;
+        en = sm.stack[--sp];
+        __syncwarp();
+        continue;
+      }
+      const int axis = sm.flat / m, pos = sm.flat - axis * m;
+      const int l = child_id(roots, s + pos);
+      if (lane == 0) write_split(N, node, l, axis, pos, s, e, depth);
+      // stable partition of the other two axis orders by side
+      if (lane < m) sm.lside[sm.idx[axis][lo + lane]] = lane >= pos ? 1 : 0;
+      __syncwarp();
+      for (int q = 1; q < 3; ++q) {
+        int* ix = sm.idx[axis + q < 3 ? axis + q : axis + q - 3] + lo;
+        const int p = lane < m ? ix[lane] : 0;
+        const bool right = lane < m && sm.lside[p] != 0;
+        const unsigned rm = __ballot_sync(0xFFFFFFFFu, right), below = (1u << lane) - 1u;
+        const int rank = __popc(rm & below);
+        if (lane < m) ix[right ? pos + rank : lane - rank] = p;
+      }
+      const int meta = ((depth + 1) << 2) | (axis + 1);
+      if (lane == 0) sm.stack[sp] = make_int4(l + 1, s + pos, e, meta);
+      sp++;
+      en = make_int4(l, s, s + pos, meta);
+      __syncwarp();
+    }
+    // the axis orders back in place: finishing reads a leaf's references in its order axis
+    for (int a = 0; a < 3; ++a)
+      if (lane < M) I.a[a][rs + lane] = sm.gid[sm.idx[a][lane]];
+    __syncwarp();
+  }
+  if (lane == 0 && st.leaves > 0) {
+    atomicAdd(stats + 0, st.leaves);
+    atomicMin(stats + 1, st.min_occ);
+    atomicMax(stats + 2, st.max_occ);
+    atomicMax(stats + 3, st.max_depth);
+  }
+}
+
 __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_subtrees(
-    const Prims P, IdxSet I, Nodes N, const int* roots, const int* root_count, int leaf_size,
-    double traversal, int* node_counter, int* stats, int* slot_of) {
+    const Prims P, IdxSet I, Nodes N, const int* roots_list, const int* root_count, int roots, int leaf_size,
+    double traversal, int* stats, int* slot_of, int4* small, int* small_count) {
   __shared__ SubtreeSmem sm;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if ((int)blockIdx.x >= *root_count) return;
-  const int root = roots[blockIdx.x];
+  const int root = roots_list[blockIdx.x];
   const int rs = N.start[root], re = N.end[root], M = re - rs;
   for (int i = threadIdx.x; i < M; i += kSubtreeThreads) {
     int p = I.a[0][rs + i];
@@ -714,26 +956,28 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
   for (int a = 1; a < 3; ++a)
     for (int i = threadIdx.x; i < M; i += kSubtreeThreads) sm.idx[a][i] = slot_of[I.a[a][rs + i]];
   if (threadIdx.x == 0) {
-    sm.stack[0] = make_int4(root, rs, re, (N.depth[root] << 2) | (N.order_axis[root] + 1));
-    sm.sp = 1;
+    const int4 en = make_int4(root, rs, re, (N.depth[root] << 2) | (N.order_axis[root] + 1));
+    sm.stack[0] = en;
+    sm.sp = M > kWarpNode ? 1 : 0;
+    if (M <= kWarpNode) small[atomicAdd(small_count, 1)] = en;
   }
   // the subtree's statistics, kept by thread 0 and added to the build's once at the end
-  // (one atomic per block instead of four per leaf on the same four words)
-  int leaves = 0, min_occ = 0x7FFFFFFF, max_occ = 0, max_depth = 0;
+  LeafStats st{0, 0x7FFFFFFF, 0, 0};
   __syncthreads();
+  // ---- the block's nodes: warp a sweeps axis a, the block takes the first minimum over the three
+  // axes' winners, and the warps of the two other axes partition their orders.  Every decision is
+  // computed identically by all threads (or broadcast through shared memory), so the block's
+  // barriers are uniform.
   while (sm.sp > 0) {
     const int4 en = sm.stack[sm.sp - 1];
     __syncthreads();
     if (threadIdx.x == 0) sm.sp--;
     const int node = en.x, s = en.y, e = en.z, m = e - s, lo = s - rs;
     const int oa = (en.w & 3) - 1, depth = en.w >> 2;
-    // node bounds (every warp computes the same union): a butterfly over the lanes that hold
-    // positions, then lane 0's union to all
+    // node bounds (every warp computes the same union)
     Box nb = empty_box();
     for (int i = lane; i < m; i += 32) nb = BoxUnion()(nb, sm.lbox[sm.idx[0][lo + i]]);
-    int span = 1;
-    while (span < min(m, 32)) span <<= 1;
-    for (int off = 1; off < span; off <<= 1) {
+    for (int off = 1; off < 32; off <<= 1) {
       Box o;
       for (int k = 0; k < 3; ++k) {
         o.mn[k] = __shfl_xor_sync(0xFFFFFFFFu, nb.mn[k], off);
@@ -741,14 +985,13 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
       }
       nb = BoxUnion()(nb, o);
     }
-    if (span < 32) nb = warp_bcast(nb, 0);
     const double node_a = surface_area(nb) * traversal;
     // this warp's axis
     double best = CUDART_INF;
-    long long best_flat = 0x7FFFFFFFFFFFFFFFLL;
+    int best_flat = 0x7FFFFFFF;
     const int a = warp;
     const int* ix = sm.idx[a] + lo;
-    if (m > 1 && P.cen[a][sm.gid[ix[m - 1]]] - P.cen[a][sm.gid[ix[0]]] > 1.0e-12) {
+    if (box_centroid(sm.lbox[ix[m - 1]], a) - box_centroid(sm.lbox[ix[0]], a) > 1.0e-12) {
       // suffix boxes and weights, from the last position down (GpuScene.java:1476-1480)
       Box carry = empty_box();
       double acc = 0.0;
@@ -778,7 +1021,7 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
           double bl = surface_area(b) * pw;
           double d = sm.sterm[a][lo + i];
           double c = (node_a + bl) + d;
-          long long flat = (long long)a * m + i;
+          const int flat = a * m + i;
           if (lex_less(c, flat, best, best_flat)) {
             best = c;
             best_flat = flat;
@@ -788,7 +1031,7 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
       }
       for (int off = 16; off > 0; off >>= 1) {
         double oc = __shfl_xor_sync(0xFFFFFFFFu, best, off);
-        long long of = __shfl_xor_sync(0xFFFFFFFFu, best_flat, off);
+        int of = __shfl_xor_sync(0xFFFFFFFFu, best_flat, off);
         if (lex_less(oc, of, best, best_flat)) {
           best = oc;
           best_flat = of;
@@ -807,13 +1050,8 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
         best = sm.best_cost[k];
         best_flat = sm.best_flat[k];
       }
-    // leaf rule (GpuScene.java:1435-1441), the weight sum in the node's current order
-    bool leaf = m == 1 || best == CUDART_INF;
-    if (!leaf && m <= leaf_size) {
-      double wsum = 0.0;
-      for (int j = 0; j < m; ++j) wsum = wsum + (oa < 0 ? P.w[s + j] : sm.lw[sm.idx[oa][lo + j]]);
-      if (!(best < surface_area(nb) * wsum)) leaf = true;
-    }
+    bool leaf = best == CUDART_INF;
+    if (!leaf && m <= leaf_size && !(best < surface_area(nb) * order_weight(sm, P, oa, s, lo, m))) leaf = true;
     if (threadIdx.x == 0) {
       N.bounds[node] = nb;
       N.split_axis[node] = -1;
@@ -821,33 +1059,21 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
     if (leaf) {
       if (threadIdx.x == 0) {
         N.leaf[node] = 1;
-        leaves++;
-        min_occ = min(min_occ, m);
-        max_occ = max(max_occ, m);
-        max_depth = max(max_depth, depth);
+        st.add(m, depth);
       }
       __syncthreads();
       continue;
     }
-    const int axis = (int)(best_flat / m), pos = (int)(best_flat % m);
+    const int axis = best_flat / m, pos = best_flat % m;
     if (threadIdx.x == 0) {
-      int l = atomicAdd(node_counter, 2), r = l + 1;
-      N.leaf[node] = 0;
-      N.left[node] = l;
-      N.right[node] = r;
-      N.split_axis[node] = axis;
-      N.split_pos[node] = pos;
-      N.start[l] = s;
-      N.end[l] = s + pos;
-      N.start[r] = s + pos;
-      N.end[r] = e;
-      N.order_axis[l] = N.order_axis[r] = axis;
-      N.depth[l] = N.depth[r] = depth + 1;
-      N.leaf[l] = N.leaf[r] = 0;
+      const int l = child_id(roots, s + pos);
+      write_split(N, node, l, axis, pos, s, e, depth);
       const int meta = ((depth + 1) << 2) | (axis + 1);
-      sm.stack[sm.sp] = make_int4(r, s + pos, e, meta);
-      sm.stack[sm.sp + 1] = make_int4(l, s, s + pos, meta);
-      sm.sp += 2;
+      const int4 kids[2] = {make_int4(l + 1, s + pos, e, meta), make_int4(l, s, s + pos, meta)};
+      for (int h = 0; h < 2; ++h) {
+        if (kids[h].z - kids[h].y > kWarpNode) sm.stack[sm.sp++] = kids[h];
+        else small[atomicAdd(small_count, 1)] = kids[h];
+      }
     }
     // stable partition of the other two axis orders by side
     if (warp == axis)
@@ -855,25 +1081,18 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
     __syncthreads();
     if (warp != axis) {
       int* t = sm.tmp[a];
-      int nl = 0;
+      int nl = 0, nr = 0;
       for (int base = 0; base < m; base += 32) {
         int li = base + lane;
         bool in = li < m;
         int p = in ? sm.idx[a][lo + li] : 0;
-        bool left = in && sm.lside[p] == 0;
-        unsigned bal = __ballot_sync(0xFFFFFFFFu, left);
-        if (left) t[nl + __popc(bal & ((1u << lane) - 1u))] = p;
-        nl += __popc(bal);
-      }
-      int nr = 0;
-      for (int base = 0; base < m; base += 32) {
-        int li = base + lane;
-        bool in = li < m;
-        int p = in ? sm.idx[a][lo + li] : 0;
-        bool right = in && sm.lside[p] != 0;
-        unsigned bal = __ballot_sync(0xFFFFFFFFu, right);
-        if (right) t[pos + nr + __popc(bal & ((1u << lane) - 1u))] = p;
-        nr += __popc(bal);
+        const bool right = in && sm.lside[p] != 0;
+        const unsigned rm = __ballot_sync(0xFFFFFFFFu, right);
+        const unsigned lm = __ballot_sync(0xFFFFFFFFu, in && !right);
+        const unsigned below = (1u << lane) - 1u;
+        if (in) t[right ? pos + nr + __popc(rm & below) : nl + __popc(lm & below)] = p;
+        nl += __popc(lm);
+        nr += __popc(rm);
       }
       __syncwarp();
       for (int i = lane; i < m; i += 32) sm.idx[a][lo + i] = t[i];
@@ -882,18 +1101,18 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
   }
   for (int a = 0; a < 3; ++a)
     for (int i = threadIdx.x; i < M; i += kSubtreeThreads) I.a[a][rs + i] = sm.gid[sm.idx[a][i]];
-  if (threadIdx.x == 0 && leaves > 0) {
-    atomicAdd(stats + 0, leaves);
-    atomicMin(stats + 1, min_occ);
-    atomicMax(stats + 2, max_occ);
-    atomicMax(stats + 3, max_depth);
+  if (threadIdx.x == 0 && st.leaves > 0) {
+    atomicAdd(stats + 0, st.leaves);
+    atomicMin(stats + 1, st.min_occ);
+    atomicMax(stats + 2, st.max_occ);
+    atomicMax(stats + 3, st.max_depth);
   }
 }
 
 // Leaf-or-split decision per active node (GpuScene.java:1424-1447).
 __global__ void k_decide(const Prims P, IdxSet I, Nodes N, const int* active, int k,
                          const double* best_cost, const long long* best_flat, const Box* node_box,
-                         int leaf_size, int* node_counter, int* next_active, int* next_count,
+                         int leaf_size, int roots, int* next_active, int* next_count,
                          int* level_of, int level, int* stats, int* largest_child, int* small_roots,
                          int* small_count) {
   int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -922,8 +1141,7 @@ __global__ void k_decide(const Prims P, IdxSet I, Nodes N, const int* active, in
   long long flat = best_flat[g];
   int axis = (int)(flat / n);
   int pos = (int)(flat % n);
-  int c = atomicAdd(node_counter, 2);
-  int l = c, r = c + 1;
+  const int l = child_id(roots, s + pos), r = l + 1;
   N.leaf[node] = 0;
   N.left[node] = l;
   N.right[node] = r;
@@ -1224,7 +1442,8 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   double* part_cost = W.alloc<double>(max_arg_blocks);
   long long* part_flat = W.alloc<long long>(max_arg_blocks);
   int* part_node = W.alloc<int>(max_arg_blocks);
-  int* counters = W.alloc<int>(8);  // node counter, next count, stats[4]
+  int4* small_list = W.alloc<int4>(n);  // nodes that k_small_subtrees builds
+  int* counters = W.alloc<int>(8);  // their number, next count, stats[4], largest child, subtrees
   int* root_start = W.alloc<int>(4);
   int* root_end = W.alloc<int>(4);
   size_t tmp_bytes = 0, b1 = 0, b3 = 0, b4 = 0;
@@ -1254,7 +1473,7 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   // ---- roots
   int h_rs[4], h_re[4];
   int roots = root_ranges(c, per_type, h_rs, h_re);
-  int h_counters[8] = {roots, 0, 0, 0x7FFFFFFF, 0, 0, 0, 0};
+  int h_counters[8] = {0, 0, 0, 0x7FFFFFFF, 0, 0, 0, 0};
   cudaMemcpyAsync(root_start, h_rs, roots * 4, cudaMemcpyHostToDevice, sm);
   cudaMemcpyAsync(root_end, h_re, roots * 4, cudaMemcpyHostToDevice, sm);
   cudaMemcpyAsync(N.start, h_rs, roots * 4, cudaMemcpyHostToDevice, sm);
@@ -1274,6 +1493,7 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   cudaMemcpyAsync(counters, h_counters, sizeof(h_counters), cudaMemcpyHostToDevice, sm);
   cudaMemsetAsync(N.order_axis, 0xFF, (size_t)roots * 4, sm);  // -1: input order
   cudaMemsetAsync(N.depth, 0, (size_t)roots * 4, sm);
+  cudaMemsetAsync(N.leaf, 0xFF, (size_t)cap * 4, sm);  // -1: no node
   cudaMemcpyAsync(level_of, h_level.data(), roots * 4, cudaMemcpyHostToDevice, sm);
   k_init_keys<<<blocks(n), 256, 0, sm>>>(key, root_start, root_end, roots, n);
 
@@ -1364,7 +1584,7 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
     cudaMemsetAsync(counters + 1, 0, 4, sm);
     cudaMemsetAsync(counters + 6, 0, 4, sm);
     k_decide<<<blocks(k), 256, 0, sm>>>(P, I, N, active, k, best_cost, best_flat, node_box, c.leaf_size,
-                                        counters, next_active, counters + 1, level_of, level,
+                                        roots, next_active, counters + 1, level_of, level,
                                         counters + 2, counters + 6, sub_roots, counters + 7);
     k_sides<<<blocks(n), 256, 0, sm>>>(I, N, key, level_of, level, n, side);
     {
@@ -1391,15 +1611,18 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
     cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, sm);
     cudaError_t e = cudaStreamSynchronize(sm);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "BVH build levels");
-    if (h[7] > 0)
+    if (h[7] > 0) {
       k_subtrees<<<(unsigned)h[7], kSubtreeThreads, 0, sm>>>(
-          P, I, N, sub_roots, counters + 7, c.leaf_size, c.traversal, counters, counters + 2, flags);
+          P, I, N, sub_roots, counters + 7, roots, c.leaf_size, c.traversal, counters + 2, flags, small_list, counters);
+      k_small_subtrees<<<ctx->sm_count * kSmallBlocksPerSm, 32, 0, sm>>>(P, I, N, small_list, counters, roots, c.leaf_size,
+                                                                        c.traversal, counters + 2);
+    }
     cudaMemcpyAsync(h, counters, sizeof(h), cudaMemcpyDeviceToHost, sm);
     e = cudaStreamSynchronize(sm);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "BVH subtrees");
-    total_nodes = h[0];
-    if (total_nodes < 1 || total_nodes > cap) return fail(ctx, RTB_ERR_DEVICE_CHECK, "BVH node count out of range");
+    total_nodes = 2 * h[2] - roots;  // a full binary forest of h[2] leaves
+    if (h[2] < 1 || total_nodes > cap) return fail(ctx, RTB_ERR_DEVICE_CHECK, "BVH node count out of range");
   }
   int rotation_count = 0;
   if (rotate) {
@@ -1436,7 +1659,7 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
     cudaMemcpyAsync(counters + 5, &depth, 4, cudaMemcpyHostToDevice, sm);
     cudaStreamSynchronize(sm);
   }
-  rtb_status fs = finish_build(ctx, desc, cfg, W, c, in, P, I, N, roots, total_nodes, counters, out, stats);
+  rtb_status fs = finish_build(ctx, desc, cfg, W, c, in, P, I, N, roots, cap, total_nodes, counters, out, stats);
   if (fs == RTB_OK && stats) {
     stats->rotation_count = rotation_count;
     stats->sequential_nodes = sequential_nodes;

@@ -129,7 +129,7 @@ struct Nodes {
   int* depth;
   int* left;
   int* right;
-  int* leaf;        // 1 leaf, 0 interior
+  int* leaf;        // 1 leaf, 0 interior, -1 no node of this id
   int* split_axis;  // this level's decision (-1: none)
   int* split_pos;
   Box* bounds;
@@ -195,7 +195,7 @@ __global__ void k_update_keys(const Nodes N, const int* level_of, int level, int
 
 __global__ void k_parents(Nodes N, int count, int roots) {
   int node = blockIdx.x * blockDim.x + threadIdx.x;
-  if (node >= count) return;
+  if (node >= count || N.leaf[node] < 0) return;
   if (node < roots) N.parent[node] = -1;
   N.visits[node] = 0;
   if (N.leaf[node]) return;
@@ -209,7 +209,7 @@ __global__ void k_parents(Nodes N, int count, int roots) {
 // SMs: written before a fence and the visit, read past the L1 cache after it.
 __global__ void k_bottom_up(const Prims P, IdxSet I, Nodes N, int count, double traversal) {
   int node = blockIdx.x * blockDim.x + threadIdx.x;
-  if (node >= count || !N.leaf[node]) return;
+  if (node >= count || N.leaf[node] != 1) return;
   N.size[node] = 1;
   N.rsize[node] = N.end[node] - N.start[node];
   double c0 = 0.0, c1 = 0.0, c2 = 0.0;
@@ -259,7 +259,7 @@ struct BuildResult {
 __global__ void k_flatten(const Prims P, IdxSet I, const Nodes N, int count, int roots, float* node_bounds,
                           int* node_data, int* refs, int* ranks, int* root_out, BuildResult* result) {
   const int node = blockIdx.x * blockDim.x + threadIdx.x;
-  if (node >= count) return;
+  if (node >= count || N.leaf[node] < 0) return;
   int at = 0, f = 0, leaves = 0, c = node;
   for (int p = N.parent[c]; p >= 0; c = p, p = N.parent[c]) {
     const int l = N.left[p];
@@ -449,11 +449,13 @@ inline int root_ranges(const BuildCfg& c, bool per_type, int* rs, int* re) {
   return roots;
 }
 
-// Sizes and SAH statistics, the flattened arrays and the resident scene.  counters + 2 holds
+// Sizes and SAH statistics, the flattened arrays and the resident scene, of total_nodes nodes
+// whose ids lie below `ids`, the roots first.  counters + 2 holds
 // {leaves, min occupancy, max occupancy, max depth}.
 inline rtb_status finish_build(rtb_context* ctx, const rtb_scene_desc* desc, const rtb_build_config* cfg,
                                Workspace& W, const BuildCfg& c, const PrimInputs& in, const Prims& P,
-                               const IdxSet& I, const Nodes& N, int roots, int total_nodes, const int* counters,
+                               const IdxSet& I, const Nodes& N, int roots, int ids, int total_nodes,
+                               const int* counters,
                                rtb_scene** out, rtb_bvh_stats* stats) {
   cudaStream_t sm = ctx->stream;
   const int n = c.total;
@@ -464,9 +466,9 @@ inline rtb_status finish_build(rtb_context* ctx, const rtb_scene_desc* desc, con
   int* o_roots = W.alloc<int>(4);
   BuildResult* o_result = W.alloc<BuildResult>(1);
   if (!W.ok) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "BVH output");
-  k_parents<<<blocks(total_nodes), 256, 0, sm>>>(N, total_nodes, roots);
-  k_bottom_up<<<blocks(total_nodes, 128), 128, 0, sm>>>(P, I, N, total_nodes, c.traversal);
-  k_flatten<<<blocks(total_nodes, 128), 128, 0, sm>>>(P, I, N, total_nodes, roots, o_nb, o_nd, o_refs, o_rank,
+  k_parents<<<blocks(ids), 256, 0, sm>>>(N, ids, roots);
+  k_bottom_up<<<blocks(ids, 128), 128, 0, sm>>>(P, I, N, ids, c.traversal);
+  k_flatten<<<blocks(ids, 128), 128, 0, sm>>>(P, I, N, ids, roots, o_nb, o_nd, o_refs, o_rank,
                                                       o_roots, o_result);
   cudaEventRecord(ctx->ev1, sm);
   // Read back through pinned memory, so that the host goes on; scene_create waits for the stream.
