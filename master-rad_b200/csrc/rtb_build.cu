@@ -50,18 +50,6 @@ __global__ void k_gather_weights(const Prims P, const int* idx, int n, double* w
   if (j < n) wpos[j] = P.w[idx[j]];
 }
 
-// Unit construction weights: prefix / suffix sums are exact integers, one thread per position.
-__global__ void k_weights_unit(const Nodes N, const int* key, const int* level_of, int level, int n,
-                               double* pw, double* sw) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  int node = key[j];
-  if (level_of[node] != level) return;
-  int s = N.start[node], e = N.end[node];
-  pw[j] = (double)(j - s + 1);
-  sw[j] = (double)(e - j);
-}
-
 // Weighted prefix / suffix sums in the reference's sequential order, one warp per
 // (node, axis, direction), all three axes in one launch: the warp loads 32 weights at a
 // time (coalesced, the next chunk prefetched), broadcasts them to every lane with all 32
@@ -172,7 +160,7 @@ struct TypeWeights {
 // such a chunk).  Box unions (min / max) and integer sums are exact, so any association of
 // them gives the sequential result bit for bit.
 #ifndef RTB_SEG_ITEMS
-#define RTB_SEG_ITEMS 4
+#define RTB_SEG_ITEMS 2
 #endif
 constexpr int kSegThreads = 256, kSegItems = RTB_SEG_ITEMS, kSegChunk = kSegThreads * kSegItems;
 constexpr int kSegWarps = kSegThreads / 32, kCarryThreads = 1024;
@@ -330,13 +318,20 @@ __global__ void __launch_bounds__(kCarryThreads) k_seg_carries(int nc, Seg<typen
   }
 }
 
-// Per (chunk, axis): both scans with the carries, each active position handed to `use`.
+// Per (chunk, axis): both scans with the carries; every active position's split cost by `use`, and
+// each node's least cost over the axis's positions.  The minima of a thread's, a warp's and the
+// block's positions of one node meet before the one atomic: the nodes' costs are non-negative,
+// so their bit patterns order like the values.
 template <class L, class U>
-__global__ void __launch_bounds__(kSegThreads) k_seg_apply(const L load, const U use, const int* key, int n,
+__global__ void __launch_bounds__(kSegThreads) k_seg_costs(const L load, const U use, const int* key, int n,
                                                            int nc, const Seg<typename L::V>* fwd,
-                                                           const Seg<typename L::V>* bwd) {
+                                                           const Seg<typename L::V>* bwd,
+                                                           unsigned long long* best_bits) {
   using V = typename L::V;
   __shared__ Seg<V> s_warp[kSegWarps];
+  __shared__ unsigned long long s_best[kSegWarps];
+  __shared__ int s_node[kSegWarps];
+  const unsigned long long inf = 0x7FF0000000000000ULL;
   const int a = blockIdx.y, c = blockIdx.x;
   const int j0 = c * kSegChunk + threadIdx.x * kSegItems;
   int head[kSegItems], tail[kSegItems], node[kSegItems];
@@ -348,9 +343,47 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_apply(const L load, const U
   const V cb = c + 1 < nc ? bwd[slot + 1].v : L::identity();
   seg_scan_block<L, false, kSegItems, kSegWarps>(head, v, cf, fb, fi, s_warp);
   seg_scan_block<L, true, kSegItems, kSegWarps>(tail, v, cb, bb, bi, s_warp);
+  int mine = -1;  // the node of the thread's last active positions and their least cost
+  unsigned long long least = inf;
 #pragma unroll
-  for (int i = 0; i < kSegItems; ++i)
-    if (act >> i & 1) use(a, j0 + i, node[i], tail[i], fb[i], fi[i], bi[i]);
+  for (int i = 0; i < kSegItems; ++i) {
+    if (!(act >> i & 1)) continue;
+    const unsigned long long bits =
+        (unsigned long long)__double_as_longlong(use(a, j0 + i, node[i], tail[i], fb[i], fi[i], bi[i]));
+    if (node[i] != mine) {
+      if (least != inf) atomicMin(best_bits + mine, least);
+      mine = node[i];
+      least = inf;
+    }
+    least = min(least, bits);
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int same = 0;
+  __match_all_sync(0xFFFFFFFFu, mine, &same);
+  if (same) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) least = min(least, __shfl_xor_sync(0xFFFFFFFFu, least, off));
+  } else if (least != inf) {
+    atomicMin(best_bits + mine, least);
+  }
+  if (lane == 0) {
+    s_best[w] = same ? least : inf;
+    s_node[w] = mine;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    mine = -1;
+    least = inf;
+    for (int q = 0; q <= kSegWarps; ++q) {
+      const int node_q = q < kSegWarps ? s_node[q] : -1;
+      if (node_q != mine) {
+        if (least != inf) atomicMin(best_bits + mine, least);
+        mine = node_q;
+        least = inf;
+      }
+      if (q < kSegWarps) least = min(least, s_best[q]);
+    }
+  }
 }
 
 struct BoxOp {
@@ -384,32 +417,41 @@ struct BoxLoad : BoxOp {
   __device__ Box operator()(int a, int j) const { return P.box[I.a[a][j]]; }
 };
 
-// One-hot type counts in each axis order, for the level's nodes above kSeqNodeSize.
-struct CountLoad : CountOp {
-  Prims P;
-  IdxSet I;
-  Nodes N;
-  const int* level_of;
-  int level;
-  __device__ bool active(int node) const {
-    return level_of[node] == level && N.end[node] - N.start[node] > kSeqNodeSize;
+struct BoxCounts {
+  Box box;
+  TypeCounts counts;
+};
+
+struct BoxCountsOp {
+  using V = BoxCounts;
+  __device__ static BoxCounts identity() {
+    BoxCounts r;
+    r.box = BoxOp::identity();
+    r.counts = CountOp::identity();
+    return r;
   }
-  __device__ TypeCounts operator()(int a, int j) const {
-    int t = P.type[I.a[a][j]];
-    unsigned long long one = 1ULL << (32 * (t & 1));
-    return t < 2 ? TypeCounts{one, 0ULL} : TypeCounts{0ULL, one};
+  __device__ static BoxCounts combine(const BoxCounts& x, const BoxCounts& y) {
+    BoxCounts r;
+    r.box = BoxOp::combine(x.box, y.box);
+    r.counts = CountOp::combine(x.counts, y.counts);
+    return r;
   }
 };
 
-// Count-based prefix and suffix weights of every position of a large node.
-struct CountWeights {
-  TypeWeights tw;
-  double* pw[3];
-  double* sw[3];
-  __device__ void operator()(int a, int j, int, int, const TypeCounts&, const TypeCounts& upto,
-                             const TypeCounts& from) const {
-    pw[a][j] = counts_weight(upto, tw.w);
-    sw[a][j] = counts_weight(from, tw.w);
+// Boxes and one-hot type counts in each axis order, for the nodes at the level.
+struct BoxCountsLoad : BoxCountsOp {
+  Prims P;
+  IdxSet I;
+  const int* level_of;
+  int level;
+  __device__ bool active(int node) const { return level_of[node] == level; }
+  __device__ BoxCounts operator()(int a, int j) const {
+    const int p = I.a[a][j], t = P.type[p];
+    const unsigned long long one = 1ULL << (32 * (t & 1));
+    BoxCounts r;
+    r.box = P.box[p];
+    r.counts = t < 2 ? TypeCounts{one, 0ULL} : TypeCounts{0ULL, one};
+    return r;
   }
 };
 
@@ -417,184 +459,123 @@ struct CountWeights {
 // positions [s, j) left; +inf marks positions that are not candidates.  The left bounds
 // are the forward scan before j, the right bounds the backward scan at j, and the node's
 // bounds their union (written once per node, at its last position, for the axis-0 pass).
-// For nodes whose weights came from counts, bound[j] limits |cost[j] - the reference's cost|.
-struct SplitCosts {
+struct CostArgs {
   Prims P;
   IdxSet I;
   Nodes N;
+  double traversal;
+  double* cost[3];
+  Box* node_box;  // node bounds at each node's last position
+  // Bounds, and whether j is a candidate of node (then with its range).
+  __device__ bool candidate(int a, int j, int node, int* s, int* e) const {
+    *s = N.start[node];
+    *e = N.end[node];
+    if (!(j > *s && *e - *s > 1)) return false;
+    const int* idx = I.a[a];
+    return P.cen[a][idx[*e - 1]] - P.cen[a][idx[*s]] > 1.0e-12;
+  }
+  __device__ double split(double an, double al, double ar, double wl, double wr) const {
+    const double b = al * wl;
+    const double d = ar * wr;
+    return (an + b) + d;
+  }
+};
+
+// Unit weights: the sums are exact integers.
+struct UnitCosts : CostArgs {
+  __device__ double operator()(int a, int j, int node, int tail, const Box& left, const Box& upto,
+                               const Box& right) const {
+    if (a == 0 && tail) node_box[j] = upto;
+    int s, e;
+    double c = CUDART_INF;
+    if (candidate(a, j, node, &s, &e))
+      c = split(surface_area(BoxUnion()(left, right)) * traversal, surface_area(left), surface_area(right),
+                (double)(j - s), (double)(e - j));
+    cost[a][j] = c;
+    return c;
+  }
+};
+
+// Other weights: from the counts, with bound[j] limiting |cost[j] - the reference's cost|, or for a
+// node marked in `seq` from its sequential sums.
+struct CountedCosts : CostArgs {
+  TypeWeights tw;
+  const int* seq;
   const double* pw[3];
   const double* sw[3];
-  double traversal;
-  int certified;
-  double* cost[3];
   double* bound[3];
-  Box* node_box;  // node bounds at each node's last position
-  __device__ void operator()(int a, int j, int node, int tail, const Box& left, const Box& upto,
-                             const Box& right) const {
-    if (a == 0 && tail) node_box[j] = upto;
-    int s = N.start[node], e = N.end[node];
+  __device__ double operator()(int a, int j, int node, int tail, const BoxCounts& left, const BoxCounts& upto,
+                               const BoxCounts& right) const {
+    if (a == 0 && tail) node_box[j] = upto.box;
+    int s, e;
     double c = CUDART_INF;
-    if (j > s && e - s > 1) {
-      const int* idx = I.a[a];
-      double ext = P.cen[a][idx[e - 1]] - P.cen[a][idx[s]];
-      if (ext > 1.0e-12) {
-        double an = surface_area(BoxUnion()(left, right)) * traversal;
-        double al = surface_area(left);
-        double ar = surface_area(right);
-        double b = al * pw[a][j - 1];
-        double d = ar * sw[a][j];
-        c = (an + b) + d;
-        if (certified && e - s > kSeqNodeSize) {
-          const double u = 0x1p-53;
-          double kl = (double)(j - s), kr = (double)(e - j);
-          bound[a][j] = 2.0 * (al * pw[a][j - 1] * (kl * u) + ar * sw[a][j] * (kr * u) + 8.0 * u * c);
-        }
+    if (candidate(a, j, node, &s, &e)) {
+      const double an = surface_area(BoxUnion()(left.box, right.box)) * traversal;
+      const double al = surface_area(left.box), ar = surface_area(right.box);
+      if (seq[node]) {
+        c = split(an, al, ar, pw[a][j - 1], sw[a][j]);
+      } else {
+        const double wl = counts_weight(left.counts, tw.w), wr = counts_weight(right.counts, tw.w);
+        c = split(an, al, ar, wl, wr);
+        const double u = 0x1p-53;
+        const double kl = (double)(j - s), kr = (double)(e - j);
+        bound[a][j] = 2.0 * (al * wl * (kl * u) + ar * wr * (kr * u) + 8.0 * u * c);
       }
     }
     cost[a][j] = c;
+    return c;
   }
 };
 
-// Each active node's slot in the level's per-node arrays.
-__global__ void k_node_slots(const int* active, int k, int* g_of_node) {
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < k) g_of_node[active[g]] = g;
+// A node's winner: the first minimum over (axis, position), by node id.
+struct Winners {
+  double* cost;     // least cost, +inf with no candidate
+  long long* flat;  // axis * count + position of the first candidate that has it
+  int* failed;      // the certificate failed
+  int* seq;         // weights from sequential sums
+};
+
+__device__ __forceinline__ void clear_winner(const Winners& W, int node, int seq) {
+  W.cost[node] = CUDART_INF;
+  W.flat[node] = 0x7FFFFFFFFFFFFFFFLL;
+  W.failed[node] = 0;
+  W.seq[node] = seq;
 }
 
-// The winner's bound, and a cleared failure flag, per certified node.
-__global__ void k_best_bound(const Nodes N, const int* active, int k, const double* best_cost,
-                             const long long* best_flat, const double* bnd0, const double* bnd1,
-                             const double* bnd2, double* best_bound, int* failed) {
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= k) return;
-  failed[g] = 0;
-  int node = active[g];
-  int s = N.start[node], len = N.end[node] - s;
-  if (len <= kSeqNodeSize || best_cost[g] == CUDART_INF) return;
-  long long flat = best_flat[g];
-  int axis = (int)(flat / len), pos = (int)(flat % len);
-  const double* b = axis == 0 ? bnd0 : axis == 1 ? bnd1 : bnd2;
-  best_bound[g] = b[s + pos];
+__global__ void k_clear_winners(Winners W, int nodes) {
+  const int node = blockIdx.x * blockDim.x + threadIdx.x;
+  if (node < nodes) clear_winner(W, node, 0);
 }
 
-// A certified node fails when some other candidate could, in the reference's rounding, cost
-// as little as the winner.
-__global__ void k_certify(const Nodes N, const int* key, const int* level_of, int level, int n,
-                          const int* g_of_node, const double* cost0, const double* cost1,
-                          const double* cost2, const double* bound0, const double* bound1,
-                          const double* bound2, const double* best_cost, const long long* best_flat,
-                          const double* best_bound, int* failed) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
+// The strict '<' of the reference's loop keeps the first of equal costs.
+__global__ void k_first_minimum(const Nodes N, const int* key, const int* level_of, int level, int n,
+                                const CostArgs C, Winners W) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
-  const int axis = blockIdx.y;  // one axis per grid row
-  const double* cost = axis == 0 ? cost0 : axis == 1 ? cost1 : cost2;
-  const double* bound = axis == 0 ? bound0 : axis == 1 ? bound1 : bound2;
-  int node = key[j];
+  const int a = blockIdx.y, node = key[j];
   if (level_of[node] != level) return;
-  int s = N.start[node], len = N.end[node] - s;
-  if (len <= kSeqNodeSize) return;
-  double c = cost[j];
+  const double c = C.cost[a][j];
+  if (c == CUDART_INF || c != W.cost[node]) return;
+  const int s = N.start[node], len = N.end[node] - s;
+  atomicMin(W.flat + node, (long long)a * len + (j - s));
+}
+
+// A node with count-based weights fails when some other candidate could, in the reference's
+// rounding, cost as little as the winner; it is listed once.
+__global__ void k_certify(const Nodes N, const int* key, const int* level_of, int level, int n,
+                          const CountedCosts C, Winners W, int* list, int* count) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const int a = blockIdx.y, node = key[j];
+  if (level_of[node] != level || C.seq[node]) return;
+  const double c = C.cost[a][j];
   if (c == CUDART_INF) return;
-  int g = g_of_node[node];
-  if ((long long)axis * len + (j - s) == best_flat[g]) return;
-  if (c - bound[j] <= best_cost[g] + best_bound[g]) failed[g] = 1;
-}
-
-__global__ void k_failed_list(const int* active, int k, const int* failed, int* out, int* count) {
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < k && failed[g]) out[atomicAdd(count, 1)] = active[g];
-}
-
-struct Cand {
-  double cost;
-  long long flat;
-};
-__device__ __forceinline__ Cand better(Cand a, Cand b) {
-  if (b.cost < a.cost || (b.cost == a.cost && b.flat < a.flat)) return b;
-  return a;
-}
-
-// First minimum over (axis, position) for each active node, with a node's positions
-// spread over fixed-size chunks so that the few huge nodes of the top levels use many blocks.  Every chunk reduces its positions
-// (all three axes) to one (cost, flat) candidate; then the node's minimum cost and, among
-// the chunks that reach it, the smallest flat index are taken with atomics.  The minimum
-// of (cost, flat) in lexicographic order does not depend on the reduction order, so the
-// choice is the reference's strict first minimum.
-constexpr int kArgChunk = 4096;
-
-__global__ void k_arg_chunk_counts(const Nodes N, const int* active, int k, int* counts,
-                                   unsigned long long* best_bits, long long* best_flat) {
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= k) return;
-  int node = active[g];
-  int len = N.end[node] - N.start[node] - 1;  // candidate positions s+1 .. e-1
-  counts[g] = len > kArgChunk ? (len + kArgChunk - 1) / kArgChunk : 1;
-  best_bits[g] = 0x7FF0000000000000ULL;  // +inf
-  best_flat[g] = 0x7FFFFFFFFFFFFFFFLL;
-}
-
-__global__ void __launch_bounds__(256) k_argmin_chunks(const Nodes N, const int* active, int k,
-                                                       const int* chunk_end, const double* cost0,
-                                                       const double* cost1, const double* cost2,
-                                                       double* part_cost, long long* part_flat,
-                                                       int* part_node, unsigned long long* best_bits) {
-  int b = blockIdx.x;
-  // the node whose chunk range [chunk_end[g-1], chunk_end[g]) holds block b
-  int lo = 0, hi = k;
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (chunk_end[mid] <= b) lo = mid + 1;
-    else hi = mid;
-  }
-  int g = lo;
-  if (g >= k) {
-    if (threadIdx.x == 0) part_node[b] = -1;
-    return;
-  }
-  int chunk = b - (g ? chunk_end[g - 1] : 0);
-  int node = active[g];
-  int s = N.start[node], e = N.end[node];
-  int n = e - s;
-  int j0 = s + 1 + chunk * kArgChunk;
-  int j1 = min(e, j0 + kArgChunk);
-  Cand m{CUDART_INF, 0x7FFFFFFFFFFFFFFFLL};
-  const double* costs[3] = {cost0, cost1, cost2};
-  for (int a = 0; a < 3; ++a)
-    for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-      double c = costs[a][j];
-      if (c != CUDART_INF) m = better(m, Cand{c, (long long)a * n + (j - s)});
-    }
-  __shared__ double sc[8];
-  __shared__ long long sf[8];
-  for (int off = 16; off > 0; off >>= 1) {
-    double oc = __shfl_down_sync(0xFFFFFFFFu, m.cost, off);
-    long long of = __shfl_down_sync(0xFFFFFFFFu, m.flat, off);
-    m = better(m, Cand{oc, of});
-  }
-  int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    sc[w] = m.cost;
-    sf[w] = m.flat;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    Cand r = Cand{sc[0], sf[0]};
-    for (int q = 1; q < (int)(blockDim.x >> 5); ++q) r = better(r, Cand{sc[q], sf[q]});
-    part_cost[b] = r.cost;
-    part_flat[b] = r.flat;
-    part_node[b] = g;
-    // costs are non-negative: their bit patterns order like the values
-    atomicMin(best_bits + g, (unsigned long long)__double_as_longlong(r.cost));
-  }
-}
-
-__global__ void k_argmin_flat(int blocks_total, const double* part_cost, const long long* part_flat,
-                              const int* part_node, const double* best_cost, long long* best_flat) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= blocks_total) return;
-  int g = part_node[b];
-  if (g < 0) return;
-  if (part_cost[b] == best_cost[g]) atomicMin(best_flat + g, part_flat[b]);
+  const int s = N.start[node], len = N.end[node] - s;
+  const long long flat = W.flat[node];
+  if ((long long)a * len + (j - s) == flat) return;
+  const int wa = (int)(flat / len), wp = (int)(flat - (long long)wa * len);
+  if (c - C.bound[a][j] <= W.cost[node] + C.bound[wa][s + wp] && atomicExch(W.failed + node, 1) == 0)
+    list[atomicAdd(count, 1)] = node;
 }
 
 // ---- node ids
@@ -1109,26 +1090,32 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
   }
 }
 
-// Leaf-or-split decision per active node (GpuScene.java:1424-1447).
-__global__ void k_decide(const Prims P, IdxSet I, Nodes N, const int* active, int k,
-                         const double* best_cost, const long long* best_flat, const Box* node_box,
-                         int leaf_size, int roots, int* next_active, int* next_count,
-                         int* level_of, int level, int* stats, int* largest_child, int* small_roots,
-                         int* small_count) {
+// Leaf-or-split decision per active node (GpuScene.java:1424-1447).  A node whose certificate
+// failed stays for the next round, with sequential weights.
+__global__ void k_decide(const Prims P, IdxSet I, Nodes N, const int* active, int k, Winners W,
+                         const Box* node_box, int leaf_size, int roots, int* next_active, int* next_count,
+                         int* level_of, int level, int* stats, int* small_roots, int* small_count) {
   int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= k) return;
   int node = active[g];
   int s = N.start[node], e = N.end[node];
   int n = e - s;
+  N.split_axis[node] = -1;
+  if (W.failed[node]) {
+    clear_winner(W, node, 1);
+    level_of[node] = level + 1;
+    next_active[atomicAdd(next_count, 1)] = node;
+    return;
+  }
   Box bounds = node_box[e - 1];
   N.bounds[node] = bounds;
-  N.split_axis[node] = -1;
-  bool leaf = n == 1 || best_cost[g] == CUDART_INF;
+  const double best = W.cost[node];
+  bool leaf = n == 1 || best == CUDART_INF;
   if (!leaf && n <= leaf_size) {
     double wsum = 0.0;
     for (int j = s; j < e; ++j) wsum = wsum + P.w[current_prim(I.a, N.order_axis[node], j)];
     double leaf_cost = surface_area(bounds) * wsum;
-    if (!(best_cost[g] < leaf_cost)) leaf = true;
+    if (!(best < leaf_cost)) leaf = true;
   }
   if (leaf) {
     N.leaf[node] = 1;
@@ -1138,41 +1125,30 @@ __global__ void k_decide(const Prims P, IdxSet I, Nodes N, const int* active, in
     atomicMax(stats + 3, N.depth[node]);     // max depth
     return;
   }
-  long long flat = best_flat[g];
-  int axis = (int)(flat / n);
-  int pos = (int)(flat % n);
-  const int l = child_id(roots, s + pos), r = l + 1;
-  N.leaf[node] = 0;
-  N.left[node] = l;
-  N.right[node] = r;
-  N.split_axis[node] = axis;
-  N.split_pos[node] = pos;
-  N.start[l] = s;
-  N.end[l] = s + pos;
-  N.start[r] = s + pos;
-  N.end[r] = e;
-  N.order_axis[l] = N.order_axis[r] = axis;
-  N.depth[l] = N.depth[r] = N.depth[node] + 1;
-  N.leaf[l] = N.leaf[r] = 0;
-  atomicMax(stats + 3, N.depth[node] + 1);
+  const long long flat = W.flat[node];
+  const int axis = (int)(flat / n), pos = (int)(flat % n);
+  const int l = child_id(roots, s + pos);
+  write_split(N, node, l, axis, pos, s, e, N.depth[node]);
   // children of at most kSubtreeSize primitives leave the level loop: k_subtrees builds
   // their whole subtrees later (level_of -1 keeps the level kernels off their positions)
-  int sizes[2] = {pos, n - pos}, kids[2] = {l, r};
+  const int sizes[2] = {pos, n - pos};
   for (int h = 0; h < 2; ++h) {
     if (sizes[h] <= kSubtreeSize) {
-      level_of[kids[h]] = -1;
-      small_roots[atomicAdd(small_count, 1)] = kids[h];
+      level_of[l + h] = -1;
+      small_roots[atomicAdd(small_count, 1)] = l + h;
     } else {
-      level_of[kids[h]] = level + 1;
-      next_active[atomicAdd(next_count, 1)] = kids[h];
-      atomicMax(largest_child, sizes[h]);
+      level_of[l + h] = level + 1;
+      clear_winner(W, l + h, 0);
+      next_active[atomicAdd(next_count, 1)] = l + h;
     }
   }
 }
 
-// Stable partition of the three axis orders of every node split at this level, one axis
-// per blockIdx.y: left flags, one exclusive sum over all 3n flags (a node's left rank is a
-// difference inside its own axis range, so the other axes' counts cancel), then the scatter.
+// Stable partition of the three axis orders of every node split at this level, one axis per
+// blockIdx.y: left flags, one exclusive sum over all 3n of them (a node's left rank is a difference
+// inside its own axis range, so the other axes' counts cancel), then the scatter, which also gives
+// the positions of split nodes their children's keys.  (Flags made as the scan reads them: the
+// scan's few threads wait for the chain of gathers, 1.6 ms for 0.42 + 0.2 at 1M.)
 __global__ void k_left_flags3(IdxSet I, const Nodes N, const int* key, const int* level_of, int level,
                               int n, const unsigned char* side, int* flags) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1183,7 +1159,7 @@ __global__ void k_left_flags3(IdxSet I, const Nodes N, const int* key, const int
   flags[(size_t)a * n + j] = split ? (side[I.a[a][j]] == 0) : 0;
 }
 
-__global__ void k_scatter3(IdxSet I, IdxSet T, const Nodes N, const int* key, const int* level_of,
+__global__ void k_scatter3(IdxSet I, IdxSet T, const Nodes N, const int* key, int* key_out, const int* level_of,
                            int level, int n, const unsigned char* side, const int* lscan) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
@@ -1193,12 +1169,14 @@ __global__ void k_scatter3(IdxSet I, IdxSet T, const Nodes N, const int* key, co
   int* out = T.a[a];
   if (!(level_of[node] == level && N.split_axis[node] >= 0)) {
     out[j] = p;
+    if (a == 0) key_out[j] = node;
     return;
   }
   const int* ls = lscan + (size_t)a * n;
-  const int s = N.start[node];
+  const int s = N.start[node], pos = N.split_pos[node];
   const int lrank = ls[j] - ls[s];
-  out[side[p] == 0 ? s + lrank : s + N.split_pos[node] + ((j - s) - lrank)] = p;
+  out[side[p] == 0 ? s + lrank : s + pos + ((j - s) - lrank)] = p;
+  if (a == 0) key_out[j] = N.left[node] + (j < s + pos ? 0 : 1);
 }
 
 __global__ void k_sides(IdxSet I, const Nodes N, const int* key, const int* level_of, int level, int n,
@@ -1399,30 +1377,25 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   Nodes N = alloc_nodes(W, cap);
   int* level_of = W.alloc<int>(cap);
   int* key = W.alloc<int>(n);
+  int* key2 = W.alloc<int>(n);
   Box* node_box = W.alloc<Box>(n);  // a node's bounds at its last position
   const int nc = (n + kSegChunk - 1) / kSegChunk;
-  Seg<Box>* box_fwd = W.alloc<Seg<Box>>(3 * (size_t)nc);
-  Seg<Box>* box_bwd = W.alloc<Seg<Box>>(3 * (size_t)nc);
-  Seg<TypeCounts>* cnt_fwd = c.weighted ? W.alloc<Seg<TypeCounts>>(3 * (size_t)nc) : nullptr;
-  Seg<TypeCounts>* cnt_bwd = c.weighted ? W.alloc<Seg<TypeCounts>>(3 * (size_t)nc) : nullptr;
+  const size_t seg = c.weighted ? sizeof(Seg<BoxCounts>) : sizeof(Seg<Box>);
+  char* seg_fwd = W.alloc<char>(3 * (size_t)nc * seg);
+  char* seg_bwd = W.alloc<char>(3 * (size_t)nc * seg);
   WeightChains chains;
-  for (int a = 0; a < 3; ++a) {
-    chains.w[a] = W.alloc<double>(n);
-    chains.pw[a] = W.alloc<double>(n);
-    chains.sw[a] = c.weighted || a == 0 ? W.alloc<double>(n) : chains.sw[0];
-    if (!c.weighted && a > 0) chains.pw[a] = chains.pw[0];
-  }
   double* cost[3];
   double* bound[3];
   for (int a = 0; a < 3; ++a) {
+    chains.w[a] = c.weighted ? W.alloc<double>(n) : nullptr;
+    chains.pw[a] = c.weighted ? W.alloc<double>(n) : nullptr;
+    chains.sw[a] = c.weighted ? W.alloc<double>(n) : nullptr;
     cost[a] = W.alloc<double>(n);
     bound[a] = c.weighted ? W.alloc<double>(n) : nullptr;
   }
-  int* g_of_node = W.alloc<int>(cap);
-  int* failed = W.alloc<int>(cap);
+  Winners win{W.alloc<double>(cap), W.alloc<long long>(cap), W.alloc<int>(cap), W.alloc<int>(cap)};
   int* failed_list = W.alloc<int>(cap);
-  double* best_bound = W.alloc<double>(cap);
-  int* lists = W.alloc<int>(2);  // small count, failed count
+  int* lists = W.alloc<int>(2);  // next round's nodes, failed nodes
   int* sub_roots = W.alloc<int>(cap);  // nodes whose subtrees k_subtrees builds
   unsigned char* side = W.alloc<unsigned char>(n);
   int* flags = W.alloc<int>(3 * (size_t)n);  // left flags of the three axis orders
@@ -1434,21 +1407,13 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   int* tkeys2 = W.alloc<int>(n);
   int* active = W.alloc<int>(cap);
   int* next_active = W.alloc<int>(cap);
-  double* best_cost = W.alloc<double>(cap);
-  long long* best_flat = W.alloc<long long>(cap);
-  int* arg_counts = W.alloc<int>(cap);
-  int* arg_ends = W.alloc<int>(cap);
-  long long max_arg_blocks = n / kArgChunk + cap;
-  double* part_cost = W.alloc<double>(max_arg_blocks);
-  long long* part_flat = W.alloc<long long>(max_arg_blocks);
-  int* part_node = W.alloc<int>(max_arg_blocks);
   int4* small_list = W.alloc<int4>(n);  // nodes that k_small_subtrees builds
-  int* counters = W.alloc<int>(8);  // their number, next count, stats[4], largest child, subtrees
+  int* counters = W.alloc<int>(8);  // their number, -, stats[4], -, subtrees
   int* root_start = W.alloc<int>(4);
   int* root_end = W.alloc<int>(4);
   size_t tmp_bytes = 0, b1 = 0, b3 = 0, b4 = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, b1, skeys, skeys2, svals, svals, n);
-  cub::DeviceScan::ExclusiveSum(nullptr, b3, flags, lscan, std::max(3 * n, cap));
+  cub::DeviceScan::ExclusiveSum(nullptr, b3, flags, lscan, 3 * n);
   cub::DeviceRadixSort::SortPairs(nullptr, b4, tkeys, tkeys2, svals, svals, n, 0, 2);
   tmp_bytes = std::max(b1, std::max(b3, b4));
   void* tmp = W.alloc<char>(tmp_bytes);
@@ -1502,106 +1467,75 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   for (int t = 0; t < 4; ++t) tw.w[t] = c.weighted ? 1.0 + c.lambda * (c.measured[t] - 1.0) : 1.0;
   int sequential_nodes = 0;
   int k = (int)h_big.size(), level = 0, total_nodes = roots;
-  const dim3 seg_grid(nc, 3), carry_grid(3, 2);
-  // split costs of every position on all three axes (and the level's node bounds)
-  auto costs = [&](int certified) {
-    BoxLoad L;
-    L.P = P;
-    L.I = I;
-    L.level_of = level_of;
-    L.level = level;
-    SplitCosts U{P, I, N, {chains.pw[0], chains.pw[1], chains.pw[2]},
-                 {chains.sw[0], chains.sw[1], chains.sw[2]}, c.traversal, certified,
-                 {cost[0], cost[1], cost[2]}, {bound[0], bound[1], bound[2]}, node_box};
-    k_seg_chunks<<<seg_grid, kSegThreads, 0, sm>>>(L, key, n, nc, box_fwd, box_bwd);
-    k_seg_carries<BoxOp><<<carry_grid, kCarryThreads, 0, sm>>>(nc, box_fwd, box_bwd);
-    k_seg_apply<<<seg_grid, kSegThreads, 0, sm>>>(L, U, key, n, nc, box_fwd, box_bwd);
-  };
-  auto argmin = [&]() {
-    k_arg_chunk_counts<<<blocks(k), 256, 0, sm>>>(N, active, k, arg_counts,
-                                                  (unsigned long long*)best_cost, best_flat);
-    size_t tb = tmp_bytes;
-    cub::DeviceScan::InclusiveSum(tmp, tb, arg_counts, arg_ends, k, sm);
-    // chunks <= (positions / kArgChunk) + one per node; surplus blocks find no node
-    long long nb = (long long)n / kArgChunk + k + 1;
-    k_argmin_chunks<<<(unsigned)nb, 256, 0, sm>>>(N, active, k, arg_ends, cost[0], cost[1], cost[2],
-                                                  part_cost, part_flat, part_node,
-                                                  (unsigned long long*)best_cost);
-    k_argmin_flat<<<blocks(nb), 256, 0, sm>>>((int)nb, part_cost, part_flat, part_node, best_cost,
-                                              best_flat);
-  };
+  const dim3 seg_grid(nc, 3), carry_grid(3, 2), axes_grid(blocks(n), 3);
+  k_clear_winners<<<1, 32, 0, sm>>>(win, roots);
+  int* round = (int*)pinned(ctx, 2 * sizeof(int));  // next round's nodes, failed nodes
+  if (!round) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "pinned staging");
+  static_assert(kSubtreeSize >= kSeqNodeSize, "level-loop nodes must all be certifiable");
   while (k > 0) {
     // Every node of the level loop holds more than kSubtreeSize >= kSeqNodeSize primitives
-    // (smaller ones go to k_subtrees), so with non-unit weights all of them take the
-    // certified count-based weights; only those whose certificate fails are summed
-    // sequentially, below.
-    static_assert(kSubtreeSize >= kSeqNodeSize, "level-loop nodes must all be certifiable");
-    const bool certify = c.weighted;
+    // (smaller ones go to k_subtrees), so with non-unit weights all of them take the certified
+    // count-based weights; one whose certificate fails comes back in the next round with its
+    // sequential sums.  A round is one wait for the host.
+    CostArgs A{P, I, N, c.traversal, {cost[0], cost[1], cost[2]}, node_box};
+    CountedCosts U;
     if (c.weighted) {
-      cudaMemsetAsync(lists, 0, 2 * sizeof(int), sm);
-      k_node_slots<<<blocks(k), 256, 0, sm>>>(active, k, g_of_node);
-      {
-        CountLoad L;
-        L.P = P;
-        L.I = I;
-        L.N = N;
-        L.level_of = level_of;
-        L.level = level;
-        CountWeights U{tw, {chains.pw[0], chains.pw[1], chains.pw[2]},
-                       {chains.sw[0], chains.sw[1], chains.sw[2]}};
-        k_seg_chunks<<<seg_grid, kSegThreads, 0, sm>>>(L, key, n, nc, cnt_fwd, cnt_bwd);
-        k_seg_carries<CountOp><<<carry_grid, kCarryThreads, 0, sm>>>(nc, cnt_fwd, cnt_bwd);
-        k_seg_apply<<<seg_grid, kSegThreads, 0, sm>>>(L, U, key, n, nc, cnt_fwd, cnt_bwd);
+      static_cast<CostArgs&>(U) = A;
+      U.tw = tw;
+      U.seq = win.seq;
+      for (int a = 0; a < 3; ++a) {
+        U.pw[a] = chains.pw[a];
+        U.sw[a] = chains.sw[a];
+        U.bound[a] = bound[a];
       }
+      BoxCountsLoad L;
+      L.P = P;
+      L.I = I;
+      L.level_of = level_of;
+      L.level = level;
+      auto *fwd = (Seg<BoxCounts>*)seg_fwd, *bwd = (Seg<BoxCounts>*)seg_bwd;
+      k_seg_chunks<<<seg_grid, kSegThreads, 0, sm>>>(L, key, n, nc, fwd, bwd);
+      k_seg_carries<BoxCountsOp><<<carry_grid, kCarryThreads, 0, sm>>>(nc, fwd, bwd);
+      k_seg_costs<<<seg_grid, kSegThreads, 0, sm>>>(L, U, key, n, nc, fwd, bwd, (unsigned long long*)win.cost);
     } else {
-      k_weights_unit<<<blocks(n), 256, 0, sm>>>(N, key, level_of, level, n, chains.pw[0], chains.sw[0]);
+      BoxLoad L;
+      L.P = P;
+      L.I = I;
+      L.level_of = level_of;
+      L.level = level;
+      UnitCosts UU;
+      static_cast<CostArgs&>(UU) = A;
+      auto *fwd = (Seg<Box>*)seg_fwd, *bwd = (Seg<Box>*)seg_bwd;
+      k_seg_chunks<<<seg_grid, kSegThreads, 0, sm>>>(L, key, n, nc, fwd, bwd);
+      k_seg_carries<BoxOp><<<carry_grid, kCarryThreads, 0, sm>>>(nc, fwd, bwd);
+      k_seg_costs<<<seg_grid, kSegThreads, 0, sm>>>(L, UU, key, n, nc, fwd, bwd, (unsigned long long*)win.cost);
     }
-    costs(certify ? 1 : 0);
-    argmin();
-    if (certify) {
-      // large nodes whose winner is not clear of the others' bounds: sequential weights,
-      // their costs again, and the argmin again (unchanged for every other node)
-      k_best_bound<<<blocks(k), 256, 0, sm>>>(N, active, k, best_cost, best_flat, bound[0], bound[1],
-                                              bound[2], best_bound, failed);
-      k_certify<<<dim3(blocks(n), 3), 256, 0, sm>>>(N, key, level_of, level, n, g_of_node, cost[0],
-                                                    cost[1], cost[2], bound[0], bound[1], bound[2],
-                                                    best_cost, best_flat, best_bound, failed);
-      k_failed_list<<<blocks(k), 256, 0, sm>>>(active, k, failed, failed_list, lists + 1);
-      int nfail = 0;
-      cudaMemcpyAsync(&nfail, lists + 1, 4, cudaMemcpyDeviceToHost, sm);
-      cudaError_t e = cudaStreamSynchronize(sm);
-      if (e != cudaSuccess) return cuda_fail(ctx, e, "BVH build level");
-      if (nfail > 0) {
-        for (int a = 0; a < 3; ++a)
-          k_gather_weights<<<blocks(n), 256, 0, sm>>>(P, I.a[a], n, const_cast<double*>(chains.w[a]));
-        k_weights_seq<<<blocks(6LL * 32 * nfail, 128), 128, 0, sm>>>(chains, N, failed_list, nfail,
-                                                                     nullptr);
-        costs(0);
-        argmin();
-        sequential_nodes += nfail;
-      }
-    }
-    cudaMemsetAsync(counters + 1, 0, 4, sm);
-    cudaMemsetAsync(counters + 6, 0, 4, sm);
-    k_decide<<<blocks(k), 256, 0, sm>>>(P, I, N, active, k, best_cost, best_flat, node_box, c.leaf_size,
-                                        roots, next_active, counters + 1, level_of, level,
-                                        counters + 2, counters + 6, sub_roots, counters + 7);
+    cudaMemsetAsync(lists, 0, 2 * sizeof(int), sm);
+    k_first_minimum<<<axes_grid, 256, 0, sm>>>(N, key, level_of, level, n, A, win);
+    if (c.weighted)
+      k_certify<<<axes_grid, 256, 0, sm>>>(N, key, level_of, level, n, U, win, failed_list, lists + 1);
+    k_decide<<<blocks(k), 256, 0, sm>>>(P, I, N, active, k, win, node_box, c.leaf_size, roots, next_active, lists,
+                                        level_of, level, counters + 2, sub_roots, counters + 7);
     k_sides<<<blocks(n), 256, 0, sm>>>(I, N, key, level_of, level, n, side);
     {
-      const dim3 axes_grid(blocks(n), 3);
       k_left_flags3<<<axes_grid, 256, 0, sm>>>(I, N, key, level_of, level, n, side, flags);
       size_t tb = tmp_bytes;
       cub::DeviceScan::ExclusiveSum(tmp, tb, flags, lscan, 3 * n, sm);
-      k_scatter3<<<axes_grid, 256, 0, sm>>>(I, T, N, key, level_of, level, n, side, lscan);
+      k_scatter3<<<axes_grid, 256, 0, sm>>>(I, T, N, key, key2, level_of, level, n, side, lscan);
       for (int a = 0; a < 3; ++a) std::swap(I.a[a], T.a[a]);
+      std::swap(key, key2);
     }
-    k_update_keys<<<blocks(n), 256, 0, sm>>>(N, level_of, level, n, key);
-    int next_info[6] = {0, 0, 0, 0, 0, 0};  // counters[1..6]: next count, ..., largest child
-    cudaMemcpyAsync(next_info, counters + 1, sizeof(next_info), cudaMemcpyDeviceToHost, sm);
+    cudaMemcpyAsync(round, lists, 2 * sizeof(int), cudaMemcpyDeviceToHost, sm);
     cudaError_t e = cudaStreamSynchronize(sm);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "BVH build level");
-    int next = next_info[0];
-    if (next > 0) std::swap(active, next_active);
+    const int next = round[0], nfail = round[1];
+    if (nfail > 0) {
+      for (int a = 0; a < 3; ++a)
+        k_gather_weights<<<blocks(n), 256, 0, sm>>>(P, I.a[a], n, const_cast<double*>(chains.w[a]));
+      k_weights_seq<<<blocks(6LL * 32 * nfail, 128), 128, 0, sm>>>(chains, N, failed_list, nfail, nullptr);
+      sequential_nodes += nfail;
+    }
+    std::swap(active, next_active);
     k = next;
     level++;
   }
@@ -1613,7 +1547,7 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
     if (e != cudaSuccess) return cuda_fail(ctx, e, "BVH build levels");
     if (h[7] > 0) {
       k_subtrees<<<(unsigned)h[7], kSubtreeThreads, 0, sm>>>(
-          P, I, N, sub_roots, counters + 7, roots, c.leaf_size, c.traversal, counters + 2, flags, small_list, counters);
+          P, I, N, sub_roots, counters + 7, roots, c.leaf_size, c.traversal, counters + 2, lscan, small_list, counters);
       k_small_subtrees<<<ctx->sm_count * kSmallBlocksPerSm, 32, 0, sm>>>(P, I, N, small_list, counters, roots, c.leaf_size,
                                                                         c.traversal, counters + 2);
     }
