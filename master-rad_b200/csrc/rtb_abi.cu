@@ -1,6 +1,7 @@
 // The C ABI (include/rtb200.h): contexts, scene residency, render and replay entry points.
 // Every entry point locks the context, makes its device current and returns a status;
 // errors carry a message retrievable with rtb_last_error.
+#include <algorithm>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
@@ -8,6 +9,10 @@
 #include "rtb_internal.h"
 
 namespace rtb {
+
+// Results up to this size come back by way of pinned staging: a 64x36 image (28 KB) or 4,000
+// rays; beyond it the second copy costs what the first saves.
+constexpr size_t kPinnedCopyBytes = 256 << 10;
 
 rtb_status fail(rtb_context* ctx, rtb_status s, const std::string& msg) {
   if (ctx) ctx->last_error = msg;
@@ -33,6 +38,7 @@ void* stage(rtb_context* ctx, size_t bytes) {
 }
 
 void* pinned(rtb_context* ctx, size_t bytes) {
+  bytes = std::max(bytes, kPinnedCopyBytes);  // one allocation serves a context's small uses
   if (bytes > ctx->pinned_bytes) {
     cudaStreamSynchronize(ctx->stream);
     cudaFreeHost(ctx->h_pinned);
@@ -53,10 +59,6 @@ using Clock = std::chrono::steady_clock;
 long long ns_since(Clock::time_point t0) {
   return std::chrono::duration_cast<std::chrono::nanoseconds>(Clock::now() - t0).count();
 }
-
-// Results up to this size come back by way of pinned staging: a 64x36 image (28 KB) or 4,000
-// rays; beyond it the second copy costs what the first saves.
-constexpr size_t kPinnedCopyBytes = 256 << 10;
 
 struct Guard {
   rtb_context* ctx;
