@@ -222,9 +222,14 @@ __device__ __forceinline__ void start_sample(const RenderArgs& a, long long pixe
 // 0.379 / 0.353 and 1024x1024 11.1 / 10.9, four glass spheres 1024x768, 16 spp, 24 segments
 // deep 6.21 / 4.56; but 300 mixed primitives 512x512, 16 spp 2.90 / 3.68, 10k 256x256 at 4 spp
 // 1.121 / 1.125, 8 spp 1.75 / 1.97.  So the phases take frames of kPhaseItems samples per
-// resident thread over a tree of kPhaseNodes nodes.
+// resident thread over a tree of kPhaseNodes nodes, and paths of kPhaseDepth segments: camera rays
+// walk the tree together as neighbours and gain nothing from being taken singly (segments 1 / 2 /
+// 3 / 4 deep, phases / lanes: 120k primitives 1834x219, 6 spp 0.50 / 0.30, 1.38 / 1.46, 2.38 / 2.96,
+// 3.38 / 4.46; 10k 1024x1024, 4 spp 1.20 / 0.93, 2.73 / 2.26, 4.24 / 3.99, 5.77 / 5.90; 1M 2 spp 1.64 /
+// 1.24, 3.35 / 2.82, 5.00 / 4.61, 6.60 / 6.40).  Refilling only whole warps in phases of mostly
+// camera rays took back a tenth of the difference at depth 1 and cost 1 % at depth 8.
 constexpr int kBlock = 1024, kSmallBlock = 128;
-constexpr int kPhaseItems = 2, kPhaseNodes = 64;
+constexpr int kPhaseItems = 2, kPhaseNodes = 64, kPhaseDepth = 3;
 constexpr int kSlotsPerLane = 6;   // 4: 5 % slower (more phases), 8: 2 % (the slots leave L2)
 constexpr int kRefillLanes = 8;    // 4 and 12 within 1 %
 constexpr int kPoolLeafLanes = 8;  // 4 and 12 within 1 %
@@ -390,7 +395,7 @@ inline RenderArgs frame_args(const rtb_scene* scene, const rtb_camera* cam, cons
 
 // Whether the two-phase form is the faster one (see above).
 inline bool use_phases(const RenderArgs& a, int sm_count) {
-  return a.max_depth > 0 && a.S.use_bvh && a.S.node_count >= kPhaseNodes &&
+  return a.max_depth >= kPhaseDepth && a.S.use_bvh && a.S.node_count >= kPhaseNodes &&
          a.pixels * a.spp >= (long long)kPhaseItems * 1024 * sm_count;
 }
 

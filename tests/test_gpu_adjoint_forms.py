@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 
 
 # 2 samples per resident thread of 148 SMs are 303,104
-@pytest.mark.parametrize("width,height,spp,depth", [(552, 550, 1, 3), (69, 69, 64, 4), (333, 457, 2, 1),
+@pytest.mark.parametrize("width,height,spp,depth", [(552, 550, 1, 3), (69, 69, 64, 4), (333, 457, 2, 1), (333, 457, 2, 3),
                                                     (318, 318, 3, 32)])
 def test_adjoint_forms_agree(width, height, spp, depth):
     torch = pytest.importorskip("torch")

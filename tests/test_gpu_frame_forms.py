@@ -41,7 +41,7 @@ def _frame(ctx, fn, res, width, height, spp, depth, use_bvh=1, stack=0):
 # 2 samples per resident thread of 148 SMs are 303,104
 @pytest.mark.parametrize("n,width,height,spp,depth,stack", [
     (600, 551, 550, 1, 3, 0), (600, 552, 550, 1, 3, 0), (600, 317, 319, 3, 5, 8), (600, 318, 318, 3, 5, 16),
-    (600, 69, 69, 64, 4, -1), (600, 1024, 601, 2, 2, 0), (5000, 333, 457, 2, 32, 0), (40, 552, 550, 1, 3, 0),
+    (600, 69, 69, 64, 4, -1), (600, 1024, 601, 2, 2, 0), (600, 1024, 601, 2, 3, 0), (5000, 333, 457, 2, 32, 0), (40, 552, 550, 1, 3, 0),
     (600, 552, 550, 2, 0, 0)])
 def test_frame_forms_equal_the_wavefront(ctx, n, width, height, spp, depth, stack):
     res = ResidentScene.build(ctx, _scene(n))
