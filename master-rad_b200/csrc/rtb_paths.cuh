@@ -224,10 +224,12 @@ __device__ __forceinline__ void start_sample(const RenderArgs& a, long long pixe
 // 1.121 / 1.125, 8 spp 1.75 / 1.97.  So the phases take frames of kPhaseItems samples per
 // resident thread over a tree of kPhaseNodes nodes, and paths of kPhaseDepth segments: camera rays
 // walk the tree together as neighbours and gain nothing from being taken singly (segments 1 / 2 /
-// 3 / 4 deep, phases / lanes: 120k primitives 1834x219, 6 spp 0.50 / 0.30, 1.38 / 1.46, 2.38 / 2.96,
-// 3.38 / 4.46; 10k 1024x1024, 4 spp 1.20 / 0.93, 2.73 / 2.26, 4.24 / 3.99, 5.77 / 5.90; 1M 2 spp 1.64 /
-// 1.24, 3.35 / 2.82, 5.00 / 4.61, 6.60 / 6.40).  Refilling only whole warps in phases of mostly
-// camera rays took back a tenth of the difference at depth 1 and cost 1 % at depth 8.
+// 3 / 4 deep, phases / lanes, ms: 120k primitives 1834x219, 6 spp 0.50 / 0.30, 1.38 / 1.46, 2.38 /
+// 2.96, 3.38 / 4.46; 10k 1024x1024, 4 spp 1.20 / 0.93, 2.73 / 2.26, 4.24 / 3.99, 5.77 / 5.90; 1M
+// 2 spp 1.64 / 1.24, 3.35 / 2.82, 5.00 / 4.61, 6.60 / 6.40).  The form before this walk took
+// 0.35 and 1.74 ms for the first one's one and two segments.  Refilling only whole warps in
+// phases of mostly camera rays took back between none and four tenths of the difference at one
+// segment (0.51, 1.10, 1.60) and cost 1 % at depth 8.
 constexpr int kBlock = 1024, kSmallBlock = 128;
 constexpr int kPhaseItems = 2, kPhaseNodes = 64, kPhaseDepth = 3;
 constexpr int kSlotsPerLane = 6;   // 4: 5 % slower (more phases), 8: 2 % (the slots leave L2)
