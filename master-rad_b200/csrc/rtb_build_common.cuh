@@ -166,22 +166,6 @@ __global__ void k_left_flags(const int* idx, const Nodes N, const int* key, cons
   flags[j] = split ? (side[idx[j]] == 0) : 0;
 }
 
-__global__ void k_scatter(const int* idx, const Nodes N, const int* key, const int* level_of, int level,
-                          int n, const unsigned char* side, const int* lscan, int* out) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  int node = key[j];
-  int p = idx[j];
-  if (!(level_of[node] == level && N.split_axis[node] >= 0)) {
-    out[j] = p;
-    return;
-  }
-  int s = N.start[node];
-  int lrank = lscan[j] - lscan[s];
-  int dst = side[p] == 0 ? s + lrank : s + N.split_pos[node] + ((j - s) - lrank);
-  out[dst] = p;
-}
-
 __global__ void k_update_keys(const Nodes N, const int* level_of, int level, int n, int* key) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
