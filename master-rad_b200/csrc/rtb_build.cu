@@ -599,11 +599,6 @@ __global__ void k_certify(const Nodes N, const int* key, const int* level_of, in
 
 // ---- node ids
 //
-// A split puts a boundary between two positions that no other split of the tree uses, so the
-// children of a node split at position q are nodes roots + 2 q and the next: ids need no counter.
-// They are sparse; N.leaf is -1 where there is no node.
-__device__ __forceinline__ int child_id(int roots, int split) { return roots + 2 * split; }
-
 // ---- whole subtrees of at most kSubtreeSize primitives, one block each
 //
 // The recursion of BvhBuildState.build (GpuScene.java:1424-1447) below such a node, depth first,
@@ -799,33 +794,6 @@ __device__ __forceinline__ double order_weight(const Smem& sm, const Prims& P, i
   return sum;
 }
 
-struct LeafStats {
-  int leaves, min_occ, max_occ, max_depth;
-  __device__ __forceinline__ void add(int m, int depth) {
-    leaves++;
-    min_occ = min(min_occ, m);
-    max_occ = max(max_occ, m);
-    max_depth = max(max_depth, depth);
-  }
-};
-
-// A split node's record and its children's, by one thread.
-__device__ __forceinline__ void write_split(const Nodes& N, int node, int l, int axis, int pos, int s, int e,
-                                            int depth) {
-  const int r = l + 1;
-  N.leaf[node] = 0;
-  N.left[node] = l;
-  N.right[node] = r;
-  N.split_axis[node] = axis;
-  N.split_pos[node] = pos;
-  N.start[l] = s;
-  N.end[l] = s + pos;
-  N.start[r] = s + pos;
-  N.end[r] = e;
-  N.order_axis[l] = N.order_axis[r] = axis;
-  N.depth[l] = N.depth[r] = depth + 1;
-}
-
 // Everything below each listed node of at most kWarpNode primitives, a warp (the block) a node,
 // depth first.
 __global__ void __launch_bounds__(32, kSmallBlocksPerSm) k_small_subtrees(const Prims P, IdxSet I, Nodes N,
@@ -928,12 +896,7 @@ __global__ void __launch_bounds__(32, kSmallBlocksPerSm) k_small_subtrees(const 
       if (lane < M) I.a[a][rs + lane] = sm.gid[sm.idx[a][lane]];
     __syncwarp();
   }
-  if (lane == 0 && st.leaves > 0) {
-    atomicAdd(stats + 0, st.leaves);
-    atomicMin(stats + 1, st.min_occ);
-    atomicMax(stats + 2, st.max_occ);
-    atomicMax(stats + 3, st.max_depth);
-  }
+  if (lane == 0) st.add_to(stats);
 }
 
 __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_subtrees(
@@ -1101,12 +1064,7 @@ __global__ void __launch_bounds__(kSubtreeThreads, RTB_SUBTREE_BLOCKS_PER_SM) k_
   }
   for (int a = 0; a < 3; ++a)
     for (int i = threadIdx.x; i < M; i += kSubtreeThreads) I.a[a][rs + i] = sm.gid[sm.idx[a][i]];
-  if (threadIdx.x == 0 && st.leaves > 0) {
-    atomicAdd(stats + 0, st.leaves);
-    atomicMin(stats + 1, st.min_occ);
-    atomicMax(stats + 2, st.max_occ);
-    atomicMax(stats + 3, st.max_depth);
-  }
+  if (threadIdx.x == 0) st.add_to(stats);
 }
 
 // Leaf-or-split decision per active node (GpuScene.java:1424-1447).  A node whose certificate

@@ -156,22 +156,44 @@ struct IdxSet {
   int* a[3];
 };
 
+// A split puts a boundary between two positions that no other split of the tree uses, so the
+// children of a node split at position q are nodes roots + 2 q and the next: ids need no counter.
+// They are sparse; N.leaf is -1 where there is no node.
+__device__ __forceinline__ int child_id(int roots, int split) { return roots + 2 * split; }
 
-__global__ void k_left_flags(const int* idx, const Nodes N, const int* key, const int* level_of,
-                             int level, int n, const unsigned char* side, int* flags) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  int node = key[j];
-  bool split = level_of[node] == level && N.split_axis[node] >= 0;
-  flags[j] = split ? (side[idx[j]] == 0) : 0;
-}
+// The leaves one thread or warp has made, added to the build's statistics once at its end.
+struct LeafStats {
+  int leaves, min_occ, max_occ, max_depth;
+  __device__ __forceinline__ void add(int m, int depth) {
+    leaves++;
+    min_occ = min(min_occ, m);
+    max_occ = max(max_occ, m);
+    max_depth = max(max_depth, depth);
+  }
+  __device__ __forceinline__ void add_to(int* stats) const {
+    if (leaves == 0) return;
+    atomicAdd(stats + 0, leaves);
+    atomicMin(stats + 1, min_occ);
+    atomicMax(stats + 2, max_occ);
+    atomicMax(stats + 3, max_depth);
+  }
+};
 
-__global__ void k_update_keys(const Nodes N, const int* level_of, int level, int n, int* key) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  int node = key[j];
-  if (level_of[node] != level || N.split_axis[node] < 0) return;
-  key[j] = j < N.start[node] + N.split_pos[node] ? N.left[node] : N.right[node];
+// A split node's record and its children's, by one thread.
+__device__ __forceinline__ void write_split(const Nodes& N, int node, int l, int axis, int pos, int s, int e,
+                                            int depth) {
+  const int r = l + 1;
+  N.leaf[node] = 0;
+  N.left[node] = l;
+  N.right[node] = r;
+  N.split_axis[node] = axis;
+  N.split_pos[node] = pos;
+  N.start[l] = s;
+  N.end[l] = s + pos;
+  N.start[r] = s + pos;
+  N.end[r] = e;
+  N.order_axis[l] = N.order_axis[r] = axis;
+  N.depth[l] = N.depth[r] = depth + 1;
 }
 
 // ---- finishing passes: three launches over all nodes, whatever the tree's depth (a launch per
