@@ -105,7 +105,7 @@ typedef struct {
   long long bytes;
   double build_ms;          /* build time: CUDA events for the device builders, host wall
                                time for the SBVH modes */
-  int sequential_nodes;     /* nodes above 256 primitives whose split the count-based
+  int sequential_nodes;     /* nodes above 512 primitives whose split the count-based
                                weights could not certify, summed in the sequential order */
   int rotation_count;       /* BvhStats.rotationCount of the rotation modes */
   int spatial_split_count;  /* BvhStats.spatialSplitCount of the SBVH modes */

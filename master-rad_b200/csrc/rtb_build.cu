@@ -13,7 +13,7 @@
 //  * Prefix and suffix weights are SEQUENTIAL double sums in the reference; with
 //    non-dyadic weights (1.3, 2.1) their rounding depends on the order.  With unit weights
 //    the sums are exact integers and are written directly.  Otherwise a node of more than
-//    kSeqNodeSize primitives takes its weights from per-type counts (a segmented integer
+//    kSubtreeSize primitives takes its weights from per-type counts (a segmented integer
 //    scan), summed exactly and rounded once, and its costs carry a rigorous bound on how far
 //    the reference's sequentially rounded costs can be from them; its argmin is the
 //    reference's whenever every other candidate's cost minus its bound exceeds the winner's
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128) k_weights_seq(const WeightChains C, const
 
 // ---- certified weights for large nodes
 //
-// Nodes above kSeqNodeSize primitives: prefix weight of positions [s, j] = sum over the four
+// Nodes above kSubtreeSize primitives: prefix weight of positions [s, j] = sum over the four
 // primitive types of (count of that type in [s, j]) x (its construction weight), from a
 // segmented inclusive scan of per-type counts, summed in double-double (each product split
 // exactly with fma) and rounded once.  The reference's sequential sum of the same k weights
@@ -139,8 +139,6 @@ __global__ void __launch_bounds__(128) k_weights_seq(const WeightChains C, const
 // bound for recursive summation), so each cost gets a bound on its distance from the
 // reference's: the weight errors times the areas, plus the cost expression's own roundings
 // in both evaluations, doubled for margin.
-constexpr int kSeqNodeSize = 256;
-
 struct TypeCounts {
   unsigned long long a, b;  // (sphere | box << 32), (affine sphere | affine box << 32)
 };
@@ -1456,9 +1454,8 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   k_clear_winners<<<1, 32, 0, sm>>>(win, roots);
   int* round = (int*)pinned(ctx, 2 * sizeof(int));  // next round's nodes, failed nodes
   if (!round) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "pinned staging");
-  static_assert(kSubtreeSize >= kSeqNodeSize, "level-loop nodes must all be certifiable");
   while (k > 0) {
-    // Every node of the level loop holds more than kSubtreeSize >= kSeqNodeSize primitives
+    // Every node of the level loop holds more than kSubtreeSize primitives
     // (smaller ones go to k_subtrees), so with non-unit weights all of them take the certified
     // count-based weights; one whose certificate fails comes back in the next round with its
     // sequential sums.  A round is one wait for the host.
