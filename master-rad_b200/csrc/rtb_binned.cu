@@ -45,14 +45,6 @@ constexpr int kChunk = 2048;   // positions per block in the large-node passes, 
 constexpr double kMinExtent = 1.0e-12;
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
-// float <-> order-preserving unsigned, so atomicMin / atomicMax order float values.
-__device__ __forceinline__ unsigned f2o(float f) {
-  unsigned b = __float_as_uint(f);
-  return (b >> 31) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float o2f(unsigned o) {
-  return __uint_as_float((o >> 31) ? (o & 0x7FFFFFFFu) : ~o);
-}
 // Inverse of order_key (double -> order-preserving 64-bit).
 __device__ __forceinline__ double k2d(unsigned long long k) {
   return __longlong_as_double((long long)((k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFULL) : ~k));

@@ -54,6 +54,15 @@ __device__ __forceinline__ unsigned long long order_key(double v) {
   return (b >> 63) ? ~b : (b | 0x8000000000000000ULL);
 }
 
+// float <-> order-preserving unsigned, so that integer minima and maxima order float values.
+__device__ __forceinline__ unsigned f2o(float f) {
+  unsigned b = __float_as_uint(f);
+  return (b >> 31) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ float o2f(unsigned o) {
+  return __uint_as_float((o >> 31) ? (o & 0x7FFFFFFFu) : ~o);
+}
+
 struct Prims {
   float* lo[3];
   float* hi[3];
