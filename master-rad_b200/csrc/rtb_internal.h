@@ -147,10 +147,9 @@ rtb_status render_frame_wavefront(rtb_context* ctx, rtb_scene* scene, const rtb_
                                   const rtb_render_params* p, float* d_rgb, cudaStream_t stream);
 // One frame's launch, planned apart from where it runs (the batch's frames mode launches
 // many into one graph).  plan_frame validates and sizes; bind_frame gives it a queue head
-// (zeroed before launch), a sample buffer of frame_tail_bytes (nullptr: no single-sample
-// tail), path slots of frame_path_bytes, the abort flag and 14 counters; launch_frame enqueues
-// its kernels and returns how many.  Frames that may run at the same time need buffers of
-// their own.
+// (zeroed before launch), a sample buffer of frame_tail_bytes, path slots of
+// frame_path_bytes, the abort flag and 14 counters; launch_frame enqueues its kernels and
+// returns how many.  Frames that may run at the same time need buffers of their own.
 struct FramePlan;
 FramePlan* new_frame_plan();
 void delete_frame_plan(FramePlan* f);

@@ -2,6 +2,7 @@
 // in which the frame and adjoint kernels run many of them per lane.
 #pragma once
 #include "rtb_internal.h"
+#include "rtb_plan.h"
 
 namespace rtb {
 namespace {
@@ -230,16 +231,13 @@ __device__ __forceinline__ void start_sample(const RenderArgs& a, long long pixe
 // 0.35 and 1.74 ms for the first one's one and two segments.  Refilling only whole warps in
 // phases of mostly camera rays took back between none and four tenths of the difference at one
 // segment (0.51, 1.10, 1.60) and cost 1 % at depth 8.
-constexpr int kBlock = 1024, kSmallBlock = 128;
 constexpr int kPhaseItems = 2, kPhaseNodes = 64, kPhaseDepth = 3;
-constexpr int kSlotsPerLane = 6;   // 4: 5 % slower (more phases), 8: 2 % (the slots leave L2)
 constexpr int kRefillLanes = 8;    // 4 and 12 within 1 %
 constexpr int kPoolLeafLanes = 8;  // 4 and 12 within 1 %
 
 // A path slot in global memory, by groups of 32 slots: the group's origins, directions,
 // throughputs, radiances, sums (16 bytes a slot), hits and items (8 bytes a slot).  A warp
 // that takes a group reads whole lines, and one base address serves every field.
-constexpr int kGroupBytes = 32 * 96;
 struct Slot {
   char* p;   // the slot's 16-byte column
   char* p8;  // its 8-byte column
@@ -280,9 +278,6 @@ struct SlotLists {
 __device__ __forceinline__ int* slot_list(const RenderArgs& a, char* base, int which) {
   const int padded = (a.slots + 31) / 32 * 32;
   return (int*)(base + (size_t)padded / 32 * kGroupBytes) + which * padded;
-}
-inline __host__ __device__ size_t block_path_bytes(int slots) {
-  return (size_t)((slots + 31) / 32) * (kGroupBytes + 2 * 32 * sizeof(int));
 }
 
 // Between the shade and the trace phase: the block's one thread that calls it sets up the list

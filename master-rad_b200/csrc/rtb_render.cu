@@ -435,32 +435,16 @@ __global__ void __launch_bounds__(256) k_wf_shade(const __grid_constant__ Render
 
 }  // namespace
 
-// One frame's launch: arguments, grid, and how many of its last pixels run one sample per
-// item.  Built by plan_frame; the caller binds the queue, sample buffer and flags.
+// One frame's launch: arguments, and how its pixels become items and blocks.  Built by
+// plan_frame; the caller binds the queue, the buffers and the flags.
 struct FramePlan {
   RenderArgs a;
+  FrameShape shape;
   int metrics = 0;
   int shared_stack = 0;       // k_render's SDEPTH: 0, 8 or kSharedStackDepth
-  int block = 0;              // kBlock: k_render, kSmallBlock: k_render_small
-  int sm_count = 0;
-  long long resident = 0;     // threads of a full-occupancy grid
-  long long tail_pixels = 0;  // the frame's last pixels, queued one sample per item
-  long long grid = 0;
 };
 
 namespace {
-
-// Lanes of each warp that take one of n rays or items.  Few go to few lanes of many warps: a
-// warp walks on until the longest of its rays ends and runs every branch any of them takes, so
-// work for less than 32 lanes in kFewWarpsPerSm warps of every SM waits least when it is spread
-// over those.  257 rays among 4,096 primitives 67 -> 42 us, 64x36 pixels of 10k primitives 204 ->
-// 128 us, of 65 spheres 48 -> 42 us; with 2 / 4 / 16 warps an SM the second takes 164 / 149 / 129,
-// the third 46 / 43 / 45.
-constexpr int kFewWarpsPerSm = 8;
-int lanes_per_warp(long long n, int sm_count) {
-  const long long warps = (long long)sm_count * kFewWarpsPerSm;
-  return (int)std::min<long long>(32, std::max<long long>(1, (n + warps - 1) / warps));
-}
 
 template <bool METRICS, int SDEPTH>
 const void* render_kernel_of(int block) {
@@ -498,25 +482,8 @@ long long traversal_bytes(const DevScene& S) {
          (long long)S.count[kBox] * 32 + ((long long)S.count[kAffineSphere] + S.count[kAffineBox]) * 48;
 }
 
-void set_tail(FramePlan* f, long long tail_pixels) {
-  RenderArgs& a = f->a;
-  f->tail_pixels = tail_pixels;
-  a.split = a.pixels - tail_pixels;
-  a.items = a.split + tail_pixels * a.spp;
-  const long long blocks = f->resident / f->block;
-  if (f->block == kSmallBlock) {
-    a.slots = lanes_per_warp(a.items, f->sm_count);
-    const long long per_block = (long long)a.slots * (kSmallBlock / 32);
-    f->grid = std::min<long long>(blocks, (a.items + per_block - 1) / per_block);
-    return;
-  }
-  // Path slots per block: kSlotsPerLane a lane on large frames; where the frame's items fill
-  // them only a few times, the number that divides them into equal rounds (a last round of a
-  // few slots costs nearly a whole one).
-  const long long most = kSlotsPerLane * kBlock;
-  const long long rounds = (a.items + blocks * most - 1) / (blocks * most);
-  a.slots = (int)std::min(most, std::max<long long>(32, (a.items + blocks * rounds - 1) / (blocks * rounds)));
-  f->grid = std::min<long long>(blocks, (a.items + a.slots - 1) / a.slots);
+long long resident_threads(rtb_context* ctx, const FramePlan* f, int block) {
+  return (long long)ctx->sm_count * frame_blocks_per_sm(ctx, f->metrics, f->shared_stack, block) * block;
 }
 
 }  // namespace
@@ -545,43 +512,46 @@ rtb_status plan_frame(rtb_context* ctx, rtb_scene* scene, const rtb_camera* cam,
     return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "shared_stack_entries must be 0, -1, 8 or 16");
   f->shared_stack = se == 0 ? (traversal_bytes(a.S) > kSharedStackSceneBytes ? kSharedStackDepth : 0)
                   : se < 0 ? 0 : se;
-  f->block = use_phases(a, ctx->sm_count) ? kBlock : kSmallBlock;
-  f->sm_count = ctx->sm_count;
-  f->resident = (long long)ctx->sm_count * frame_blocks_per_sm(ctx, f->metrics, f->shared_stack, f->block) * f->block;
+  FrameShape& shape = f->shape;
+  shape.block = use_phases(a, ctx->sm_count) ? kBlock : kSmallBlock;
+  shape.sm_count = ctx->sm_count;
+  shape.spp = a.spp;
+  shape.pixels = a.pixels;
+  shape.resident = resident_threads(ctx, f, shape.block);
   // Tail: about four pixels per resident thread are split into single samples.
   double per_thread = tail_per_thread > 0 ? (double)tail_per_thread : RTB_TAIL_FACTOR;
-  long long tail_pixels = std::min<long long>(a.pixels, (long long)(per_thread * f->resident));
+  long long tail_pixels = std::min<long long>(a.pixels, (long long)(per_thread * shape.resident));
   // A pixel of one sample is its own item, and a black frame has none.
-  set_tail(f, a.max_depth > 0 && a.spp > 1 ? std::min<long long>(tail_pixels, kMaxTailItems / a.spp) : 0);
+  shape.set_tail(a.max_depth > 0 && a.spp > 1 ? std::min<long long>(tail_pixels, kMaxTailItems / a.spp) : 0);
   return RTB_OK;
 }
 
-size_t frame_tail_bytes(const FramePlan* f) {
-  return (size_t)f->tail_pixels * f->a.spp * 3 * sizeof(float);
-}
+size_t frame_tail_bytes(const FramePlan* f) { return f->shape.tail_bytes(); }
 
-size_t frame_path_bytes(const FramePlan* f) {
-  return f->block == kBlock ? (size_t)f->grid * block_path_bytes(f->a.slots) : 0;
-}
+size_t frame_path_bytes(const FramePlan* f) { return f->shape.path_bytes(); }
 
 void bind_frame(FramePlan* f, unsigned long long* queue, float* tail, void* paths, int* abort_flag,
                 unsigned long long* counters) {
-  if (!tail) set_tail(f, 0);  // no buffer: every pixel keeps its samples in one slot
-  f->a.queue = queue;
-  f->a.tail = tail;
-  f->a.paths = paths;
-  f->a.abort_flag = abort_flag;
-  f->a.counters = counters;
+  RenderArgs& a = f->a;
+  a.split = f->shape.split;
+  a.items = f->shape.items;
+  a.slots = f->shape.slots;
+  a.queue = queue;
+  a.tail = tail;
+  a.paths = paths;
+  a.abort_flag = abort_flag;
+  a.counters = counters;
 }
 
 int launch_frame(const FramePlan* f, cudaStream_t stream) {
   const RenderArgs& a = f->a;
+  const FrameShape& shape = f->shape;
   void* args[] = {const_cast<RenderArgs*>(&a)};
-  cudaLaunchKernel(render_kernel(f->metrics, f->shared_stack, f->block), dim3((unsigned)f->grid), dim3(f->block), args,
-                   stack_smem(f->shared_stack, f->block), stream);
-  if (f->tail_pixels == 0) return 1;
-  k_sum_tail<<<(unsigned)((f->tail_pixels + 255) / 256), 256, 0, stream>>>(
-      a.tail, a.out, a.split, (int)f->tail_pixels, a.spp, a.abort_flag);
+  cudaLaunchKernel(render_kernel(f->metrics, f->shared_stack, shape.block), dim3((unsigned)shape.grid),
+                   dim3(shape.block), args, stack_smem(f->shared_stack, shape.block), stream);
+  if (shape.tail_pixels == 0) return 1;
+  k_sum_tail<<<(unsigned)((shape.tail_pixels + 255) / 256), 256, 0, stream>>>(
+      a.tail, a.out, a.split, (int)shape.tail_pixels, a.spp, a.abort_flag);
   return 2;
 }
 
@@ -594,10 +564,11 @@ rtb_status render_frame(rtb_context* ctx, rtb_scene* scene, const rtb_camera* ca
   FramePlan f;
   rtb_status s = plan_frame(ctx, scene, cam, p, d_rgb, &f, row0, row_stride);
   if (s != RTB_OK) return s;
-  const bool tail_ok = ctx_grow(&ctx->d_tail, &ctx->tail_bytes, frame_tail_bytes(&f), stream);
-  if (!ctx_grow(&ctx->d_paths, &ctx->path_bytes, frame_path_bytes(&f), stream))
-    return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "path slots");
-  bind_frame(&f, ctx->d_work, tail_ok ? ctx->d_tail : nullptr, ctx->d_paths, ctx->d_abort, ctx->d_work + 8);
+  const bool fits = settle_frame(
+      f.shape, [&](size_t bytes) { return ctx_grow(&ctx->d_tail, &ctx->tail_bytes, bytes, stream); },
+      [&](size_t bytes) { return ctx_grow(&ctx->d_paths, &ctx->path_bytes, bytes, stream); });
+  if (!fits) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "path slots");
+  bind_frame(&f, ctx->d_work, ctx->d_tail, ctx->d_paths, ctx->d_abort, ctx->d_work + 8);
   if (timed) cudaEventRecord(ctx->ev0, stream);
   ctx->render_launches = launch_frame(&f, stream);
   if (timed) cudaEventRecord(ctx->ev1, stream);
