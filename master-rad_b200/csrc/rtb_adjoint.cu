@@ -25,7 +25,6 @@ namespace {
 
 constexpr int kTable = 512;       // shared-memory gradient entries per block
 constexpr int kMaxVertices = 32;  // max_depth limit of the renderer
-constexpr long long kMaxVertexBytes = 256LL << 20;  // of the phases' paths
 
 struct AdjointArgs {
   RenderArgs r;          // scene, camera, sizes, queue, path slots
@@ -420,21 +419,18 @@ static rtb_status render_backward(rtb_context* ctx, rtb_scene* scene, const rtb_
   a.samples = a.r.pixels * a.r.spp;
   a.r.queue = ctx->d_work;
   a.r.abort_flag = ctx->d_abort;
-  const bool phases = use_phases(a.r, ctx->sm_count);
+  bool phases = use_phases(a.r, ctx->sm_count);
   long long grid = ctx->sm_count;
   if (phases) {
-    // As many slots as a frame has (set_tail in rtb_render.cu), in equal rounds, but vertices of
-    // kMaxVertexBytes at most.
-    const long long vertex = 2 * sizeof(float4) * a.r.max_depth;
-    const long long most = std::max<long long>(
-        kBlock, std::min<long long>(kSlotsPerLane * kBlock, kMaxVertexBytes / (vertex * grid) / kBlock * kBlock));
-    const long long rounds = (a.samples + grid * most - 1) / (grid * most);
-    a.r.slots = (int)std::min(most, (a.samples + grid * rounds - 1) / (grid * rounds));
-    const size_t path_bytes = ((size_t)grid * block_path_bytes(a.r.slots) + 255) & ~(size_t)255;
-    if (!ctx_grow(&ctx->d_paths, &ctx->path_bytes, path_bytes + (size_t)(grid * a.r.slots * vertex), sm))
-      return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "path slots");
-    a.r.paths = ctx->d_paths;
-    a.vertices = (float4*)((char*)ctx->d_paths + path_bytes);
+    const ReplayShape shape(a.samples, a.r.max_depth, ctx->sm_count);
+    // without the memory, one path a lane
+    phases = ctx_grow(&ctx->d_paths, &ctx->path_bytes, shape.path_bytes + shape.vertex_bytes, sm);
+    if (phases) {
+      grid = shape.grid;
+      a.r.slots = shape.slots;
+      a.r.paths = ctx->d_paths;
+      a.vertices = (float4*)((char*)ctx->d_paths + shape.path_bytes);
+    }
   }
   size_t gbytes = (size_t)scene->dev.material_count * 3 * sizeof(float);
   arm_abort(ctx, sm, true);

@@ -357,21 +357,33 @@ rtb_status plan_frames(rtb_context* ctx, rtb_batch* B, const std::vector<int>& o
     }
     B->frames.push_back(f);
     branch_bytes[i % K] = std::max(branch_bytes[i % K], rtb::frame_tail_bytes(f));
-    path_bytes[i % K] = std::max(path_bytes[i % K], rtb::frame_path_bytes(f));
   }
   std::vector<size_t> off(K, 0), path_off(K, 0);
   size_t total = 0;
-  for (int b = 0; b < K; ++b) {
-    off[b] = total;
-    total += (branch_bytes[b] + 255) & ~(size_t)255;
-    path_off[b] = total;
-    total += (path_bytes[b] + 255) & ~(size_t)255;
-  }
+  auto lay_out = [&] {
+    std::fill(path_bytes.begin(), path_bytes.end(), 0);
+    for (int i = 0; i < n; ++i)
+      path_bytes[i % K] = std::max(path_bytes[i % K], rtb::frame_path_bytes(B->frames[i]));
+    total = 0;
+    for (int b = 0; b < K; ++b) {
+      off[b] = total;
+      total += (branch_bytes[b] + 255) & ~(size_t)255;
+      path_off[b] = total;
+      total += (path_bytes[b] + 255) & ~(size_t)255;
+    }
+  };
+  lay_out();
   if (total > B->frame_tail_bytes) {
     cudaFree(B->d_frame_tails);
     B->d_frame_tails = nullptr;
     B->frame_tail_bytes = 0;
     cudaError_t e = cudaMalloc(&B->d_frame_tails, total);
+    if (e == cudaErrorMemoryAllocation) {  // without path slots, then
+      cudaGetLastError();
+      for (FramePlan* f : B->frames) frame_without_slots(ctx, f);
+      lay_out();
+      e = total > 0 ? cudaMalloc(&B->d_frame_tails, total) : cudaSuccess;
+    }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "batch frame sample buffers");
     B->frame_tail_bytes = total;
   }

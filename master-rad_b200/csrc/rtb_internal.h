@@ -149,7 +149,7 @@ rtb_status render_frame_wavefront(rtb_context* ctx, rtb_scene* scene, const rtb_
 // many into one graph).  plan_frame validates and sizes; bind_frame gives it a queue head
 // (zeroed before launch), a sample buffer of frame_tail_bytes, path slots of
 // frame_path_bytes, the abort flag and 14 counters; launch_frame enqueues its kernels and
-// returns how many.  Frames that may run at the same time need buffers of their own.
+// returns how many.  frame_without_slots: the same frame in the form that needs none.  Frames that may run at the same time need buffers of their own.
 struct FramePlan;
 FramePlan* new_frame_plan();
 void delete_frame_plan(FramePlan* f);
@@ -160,6 +160,7 @@ rtb_status plan_frame(rtb_context* ctx, rtb_scene* scene, const rtb_camera* cam,
                       int row_stride = 1, int tail_per_thread = 0);
 size_t frame_tail_bytes(const FramePlan* f);
 size_t frame_path_bytes(const FramePlan* f);
+void frame_without_slots(rtb_context* ctx, FramePlan* f);
 void bind_frame(FramePlan* f, unsigned long long* queue, float* tail, void* paths, int* abort_flag,
                 unsigned long long* counters);
 int launch_frame(const FramePlan* f, cudaStream_t stream);

@@ -62,17 +62,41 @@ struct FrameShape {
     }
     grid = std::min(blocks, (items + per_block - 1) / per_block);
   }
+  // In k_render_small's form; the tail stays as long as it was.
+  void without_slots(long long small_resident) {
+    block = kSmallBlock;
+    resident = small_resident;
+    set_tail(tail_pixels);
+  }
   size_t tail_bytes() const { return (size_t)tail_pixels * spp * 3 * sizeof(float); }
   size_t path_bytes() const { return block == kBlock ? (size_t)grid * block_path_bytes(slots) : 0; }
 };
 
 // Settles a frame's buffers: grow_tail(bytes) and grow_paths(bytes) say whether the buffer is
-// there.  Without a sample buffer every pixel keeps its samples in one slot.  The slots are asked
+// there.  Without a sample buffer every pixel keeps its samples in one slot; without path slots
+// the frame runs in the form that needs none, of small_resident() threads.  The slots are asked
 // for last: their number depends on the tail, and does not only shrink without it.
-template <class Tail, class Paths>
-inline bool settle_frame(FrameShape& f, Tail&& grow_tail, Paths&& grow_paths) {
+template <class Tail, class Paths, class Small>
+inline void settle_frame(FrameShape& f, Tail&& grow_tail, Paths&& grow_paths, Small&& small_resident) {
   if (!grow_tail(f.tail_bytes())) f.set_tail(0);
-  return grow_paths(f.path_bytes());
+  if (f.block == kBlock && !grow_paths(f.path_bytes())) f.without_slots(small_resident());
 }
+
+// The path slots of a replay in phases, one block an SM: as a frame's, but vertices of
+// kMaxVertexBytes at most.
+constexpr long long kMaxVertexBytes = 256LL << 20;
+struct ReplayShape {
+  long long grid = 0;
+  int slots = 0;
+  size_t path_bytes = 0, vertex_bytes = 0;  // the vertices lie behind the slots
+  ReplayShape(long long samples, int max_depth, int sm_count) : grid(sm_count) {
+    const long long vertex = 2LL * 16 * max_depth;  // two float4 a segment
+    const long long most = std::max<long long>(
+        kBlock, std::min<long long>(kSlotsPerLane * kBlock, kMaxVertexBytes / (vertex * grid) / kBlock * kBlock));
+    slots = slots_in_rounds(samples, grid, most);
+    path_bytes = ((size_t)grid * block_path_bytes(slots) + 255) & ~(size_t)255;
+    vertex_bytes = (size_t)(grid * slots * vertex);
+  }
+};
 
 }  // namespace rtb

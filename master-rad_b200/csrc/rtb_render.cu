@@ -530,6 +530,10 @@ size_t frame_tail_bytes(const FramePlan* f) { return f->shape.tail_bytes(); }
 
 size_t frame_path_bytes(const FramePlan* f) { return f->shape.path_bytes(); }
 
+void frame_without_slots(rtb_context* ctx, FramePlan* f) {
+  if (f->shape.block == kBlock) f->shape.without_slots(resident_threads(ctx, f, kSmallBlock));
+}
+
 void bind_frame(FramePlan* f, unsigned long long* queue, float* tail, void* paths, int* abort_flag,
                 unsigned long long* counters) {
   RenderArgs& a = f->a;
@@ -564,10 +568,10 @@ rtb_status render_frame(rtb_context* ctx, rtb_scene* scene, const rtb_camera* ca
   FramePlan f;
   rtb_status s = plan_frame(ctx, scene, cam, p, d_rgb, &f, row0, row_stride);
   if (s != RTB_OK) return s;
-  const bool fits = settle_frame(
+  settle_frame(
       f.shape, [&](size_t bytes) { return ctx_grow(&ctx->d_tail, &ctx->tail_bytes, bytes, stream); },
-      [&](size_t bytes) { return ctx_grow(&ctx->d_paths, &ctx->path_bytes, bytes, stream); });
-  if (!fits) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "path slots");
+      [&](size_t bytes) { return ctx_grow(&ctx->d_paths, &ctx->path_bytes, bytes, stream); },
+      [&] { return resident_threads(ctx, &f, kSmallBlock); });
   bind_frame(&f, ctx->d_work, ctx->d_tail, ctx->d_paths, ctx->d_abort, ctx->d_work + 8);
   if (timed) cudaEventRecord(ctx->ev0, stream);
   ctx->render_launches = launch_frame(&f, stream);

@@ -1,7 +1,8 @@
-"""The host arithmetic of a frame's launch (csrc/rtb_plan.h, compiled here for the host): over
-frame sizes from one pixel to beyond 4K and 1 to 512 samples, and whichever of the buffers can
-be had, the path slots that the launch uses lie inside the buffer that was asked for last, and
-the queue's items cover every sample once."""
+"""The host arithmetic of a frame's and a replay's launch (csrc/rtb_plan.h, compiled here for the
+host): over frame sizes from one pixel to beyond 4K and 1 to 512 samples, and whichever of the
+buffers can be had, the path slots that the launch uses lie inside the buffer that was asked for
+last, the queue's items cover every sample once, and a frame without slots takes the form that
+needs none."""
 import ctypes as C
 import os
 import subprocess
@@ -13,7 +14,7 @@ SOURCE = r"""
 #include "rtb_plan.h"
 using namespace rtb;
 struct Out { long long block, slots, grid, items, split, tail_pixels, tail_bytes, path_bytes, had_tail, had_paths; };
-extern "C" int settle(int block, int sm_count, long long resident, long long pixels, int spp, long long tail,
+extern "C" void settle(int block, int sm_count, long long resident, long long pixels, int spp, long long tail,
                       long long tail_limit, long long path_limit, Out* o) {
   FrameShape f;
   f.block = block;
@@ -23,9 +24,10 @@ extern "C" int settle(int block, int sm_count, long long resident, long long pix
   f.resident = resident;
   f.set_tail(tail);
   *o = Out{};
-  const bool ok = settle_frame(
+  settle_frame(
       f, [&](size_t n) { return (long long)n <= tail_limit ? (o->had_tail = (long long)n, true) : false; },
-      [&](size_t n) { return (long long)n <= path_limit ? (o->had_paths = (long long)n, true) : false; });
+      [&](size_t n) { return (long long)n <= path_limit ? (o->had_paths = (long long)n, true) : false; },
+      [&] { return resident / 2; });
   o->block = f.block;
   o->slots = f.slots;
   o->grid = f.grid;
@@ -34,7 +36,14 @@ extern "C" int settle(int block, int sm_count, long long resident, long long pix
   o->tail_pixels = f.tail_pixels;
   o->tail_bytes = (long long)f.tail_bytes();
   o->path_bytes = f.block == kBlock ? (long long)(f.grid * block_path_bytes(f.slots)) : 0;
-  return ok;
+}
+extern "C" void replay(long long samples, int max_depth, int sm_count, long long* o) {
+  const ReplayShape r(samples, max_depth, sm_count);
+  o[0] = r.grid;
+  o[1] = r.slots;
+  o[2] = (long long)r.path_bytes;
+  o[3] = (long long)r.vertex_bytes;
+  o[4] = (long long)(r.grid * block_path_bytes(r.slots));
 }
 """
 FIELDS = ("block", "slots", "grid", "items", "split", "tail_pixels", "tail_bytes", "path_bytes", "had_tail",
@@ -46,13 +55,21 @@ class Out(C.Structure):
 
 
 @pytest.fixture(scope="module")
-def settle(tmp_path_factory):
+def plan(tmp_path_factory):
     d = tmp_path_factory.mktemp("plan")
     (d / "plan.cpp").write_text(SOURCE)
     so = str(d / "plan.so")
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, "-o", so, str(d / "plan.cpp")],
                    check=True)
-    fn = C.CDLL(so).settle
+    lib = C.CDLL(so)
+    lib.replay.argtypes = [C.c_longlong, C.c_int, C.c_int, C.POINTER(C.c_longlong)]
+    return lib
+
+
+@pytest.fixture(scope="module")
+def settle(plan):
+    fn = plan.settle
+    fn.restype = None
     fn.argtypes = [C.c_int, C.c_int, C.c_longlong, C.c_longlong, C.c_int, C.c_longlong, C.c_longlong, C.c_longlong,
                    C.POINTER(Out)]
 
@@ -60,8 +77,8 @@ def settle(tmp_path_factory):
         o = Out()
         resident = sms * 1024
         tail = min(pixels, 4 * resident, (1 << 26) // spp) if spp > 1 else 0
-        ok = fn(block, sms, resident, pixels, spp, tail, tail_limit, path_limit, C.byref(o))
-        return ok, o
+        fn(block, sms, resident, pixels, spp, tail, tail_limit, path_limit, C.byref(o))
+        return o
     return call
 
 
@@ -76,8 +93,7 @@ def test_slots_lie_in_the_buffer_asked_for(settle, sms, tail_limit):
     sizes = [w * h for w, h in FRAMES] + [10 ** 5 + 99991 * k for k in range(60)]
     for pixels in sizes:
         for spp in (1, 2, 3, 4, 5, 8, 13, 16, 64, 128, 512):
-            ok, o = settle(1024, sms, pixels, spp, tail_limit, ALL)
-            assert ok
+            o = settle(1024, sms, pixels, spp, tail_limit, ALL)
             what = (pixels, spp, {k: getattr(o, k) for k in FIELDS})
             assert o.path_bytes <= o.had_paths, what
             assert o.tail_bytes <= o.had_tail, what
@@ -85,3 +101,28 @@ def test_slots_lie_in_the_buffer_asked_for(settle, sms, tail_limit):
             # no block without an item, none past the device's
             assert 1 <= o.grid <= sms and (o.grid - 1) * o.slots < o.items, what
             assert 32 <= o.slots <= 6 * 1024 and o.block == 1024, what
+
+
+@pytest.mark.parametrize("tail_limit", [ALL, 0])
+def test_a_frame_without_slots_takes_the_other_form(settle, tail_limit):
+    for pixels in [w * h for w, h in FRAMES]:
+        for spp in (1, 2, 16, 512):
+            o, full = settle(1024, 148, pixels, spp, tail_limit, 0), settle(1024, 148, pixels, spp, tail_limit, ALL)
+            assert (o.block, o.path_bytes, o.had_paths) == (128, 0, 0)
+            assert (o.items, o.split, o.tail_pixels, o.tail_bytes) == (
+                full.items, full.split, full.tail_pixels, full.tail_bytes)
+            assert 1 <= o.slots <= 32 and 1 <= o.grid <= 148 * 4  # half the threads, in blocks of 128
+
+
+@pytest.mark.parametrize("sms", [148, 132])
+def test_replay_slots_and_vertices_lie_in_their_buffer(plan, sms):
+    o = (C.c_longlong * 5)()
+    for samples in [2048 * sms, 2048 * sms + 1, 10 ** 6, 3 * 10 ** 6 + 7, 512 * 512 * 32, 1920 * 1080 * 64, 1 << 33]:
+        for depth in (3, 4, 6, 8, 13, 24, 32):
+            plan.replay(samples, depth, sms, o)
+            grid, slots, paths, vertices, used = o
+            assert grid == sms and 32 <= slots <= 6 * 1024
+            assert used <= paths and paths % 256 == 0
+            assert vertices == grid * slots * depth * 32
+            assert vertices <= (256 << 20) or slots <= 1024
+            assert grid * slots <= samples + grid * 32
