@@ -633,13 +633,14 @@ __global__ void k_first_minimum(const Nodes N, const int* key, const int* level_
 }
 
 // A node with count-based weights fails when some other candidate could, in the reference's
-// rounding, cost as little as the winner; it is listed once.
+// rounding, cost as little as the winner; it is listed once.  A node without a winner (weights
+// whose sums overflow leave no cost but NaN) becomes a leaf; it has no position to compare with.
 __global__ void k_certify(const Nodes N, const int* key, const int* level_of, int level, int n,
                           const CountedCosts C, Winners W, int* list, int* count) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const int a = blockIdx.y, node = key[j];
-  if (level_of[node] != level || C.seq[node]) return;
+  if (level_of[node] != level || C.seq[node] || W.cost[node] == CUDART_INF) return;
   const double c = C.cost[a][j];
   if (c == CUDART_INF) return;
   const int s = N.start[node], len = N.end[node] - s;
