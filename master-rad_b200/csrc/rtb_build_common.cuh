@@ -264,16 +264,28 @@ __global__ void k_bottom_up(const Prims P, IdxSet I, Nodes N, int count, double 
 // What the host reads back of a finished build.
 struct BuildResult {
   double sah[4][3];  // per root
+  int nodes, refs;   // below all roots, by the climb: every node and primitive, if none was lost
 };
 
 // The flattened reference layout (flattenBvh / leafKind, GpuScene.java:772-808).  A node's preorder
 // index and first reference are sums over the path to its root: one for every step down, the
 // left sibling's sizes for every step to the right, the earlier trees' sizes at the root.  A full
 // binary tree of s nodes has (s + 1) / 2 leaves, so the same walk gives an interior node's rank
-// among the interior nodes.
-__global__ void k_flatten(const Prims P, IdxSet I, const Nodes N, int count, int roots, float* node_bounds,
-                          int* node_data, int* refs, int* ranks, int* root_out, BuildResult* result) {
+// among the interior nodes.  The arrays are sized by the leaves that the build counted, not by
+// these sums: nothing is written past total_nodes and total_refs, and the host compares.
+__global__ void k_flatten(const Prims P, IdxSet I, const Nodes N, int count, int roots, int total_nodes,
+                          int total_refs, float* node_bounds, int* node_data, int* refs, int* ranks,
+                          int* root_out, BuildResult* result) {
   const int node = blockIdx.x * blockDim.x + threadIdx.x;
+  if (node == 0) {
+    int nodes = 0, prims = 0;
+    for (int r = 0; r < roots; ++r) {
+      nodes += N.size[r];
+      prims += N.rsize[r];
+    }
+    result->nodes = nodes;
+    result->refs = prims;
+  }
   if (node >= count || N.leaf[node] < 0) return;
   int at = 0, f = 0, leaves = 0, c = node;
   for (int p = N.parent[c]; p >= 0; c = p, p = N.parent[c]) {
@@ -292,6 +304,7 @@ __global__ void k_flatten(const Prims P, IdxSet I, const Nodes N, int count, int
     leaves += (size + 1) >> 1;
     f += N.rsize[r];
   }
+  if ((unsigned)at >= (unsigned)total_nodes) return;
   if (node < roots) {
     root_out[node] = at;
     for (int m = 0; m < 3; ++m) result->sah[node][m] = N.sah[m][node];
@@ -312,6 +325,7 @@ __global__ void k_flatten(const Prims P, IdxSet I, const Nodes N, int count, int
   }
   // references in preorder of the leaves (after rotations that differs from array order)
   int s = N.start[node], e = N.end[node];
+  if (f < 0 || e - s > total_refs - f) return;
   int t0 = -1;
   bool mixed = false;
   for (int j = s; j < e; ++j) {
@@ -483,8 +497,8 @@ inline rtb_status finish_build(rtb_context* ctx, const rtb_scene_desc* desc, con
   if (!W.ok) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "BVH output");
   k_parents<<<blocks(ids), 256, 0, sm>>>(N, ids, roots);
   k_bottom_up<<<blocks(ids, 128), 128, 0, sm>>>(P, I, N, ids, c.traversal);
-  k_flatten<<<blocks(ids, 128), 128, 0, sm>>>(P, I, N, ids, roots, o_nb, o_nd, o_refs, o_rank,
-                                                      o_roots, o_result);
+  k_flatten<<<blocks(ids, 128), 128, 0, sm>>>(P, I, N, ids, roots, total_nodes, n, o_nb, o_nd, o_refs, o_rank,
+                                              o_roots, o_result);
   cudaEventRecord(ctx->ev1, sm);
   // Read back through pinned memory, so that the host goes on; scene_create waits for the stream.
   struct Back {
@@ -502,10 +516,11 @@ inline rtb_status finish_build(rtb_context* ctx, const rtb_scene_desc* desc, con
   const BuildResult& h_result = back->result;
   float ms = 0.0f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-  if (total_nodes != 2 * h_stats[0] - roots) {
+  if (h_result.nodes != total_nodes || h_result.refs != n) {
     scene_free(*out, sm);
     *out = nullptr;
-    return fail(ctx, RTB_ERR_DEVICE_CHECK, "A binary BVH forest must contain 2 * leafCount - rootCount nodes.");
+    return fail(ctx, RTB_ERR_DEVICE_CHECK,
+                "A binary BVH forest must contain 2 * leafCount - rootCount nodes and every primitive.");
   }
   if (stats) {
     stats->node_count = total_nodes;

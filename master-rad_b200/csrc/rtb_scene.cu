@@ -36,11 +36,20 @@ __device__ __forceinline__ int checked_material(float v, int nmat, int* err) {
   return m;
 }
 
+// The insertion index behind storage index s.
+__device__ __forceinline__ int source_index(const int* orig_of_new, int s, int n, int* err) {
+  if (!orig_of_new) return s;
+  const int o = orig_of_new[s];
+  if ((unsigned)o < (unsigned)n) return o;
+  atomicOr(err, 1);
+  return 0;
+}
+
 __global__ void k_pack_spheres(const float* raw, int n, const int* orig_of_new, float4* out,
                                int* mat, int* orig, int nmat, int* err) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
-  int o = orig_of_new ? orig_of_new[s] : s;
+  int o = source_index(orig_of_new, s, n, err);
   const float* r = raw + 5 * (size_t)o;
   out[s] = make_float4(r[0], r[1], r[2], r[3]);
   mat[s] = checked_material(r[4], nmat, err);
@@ -51,7 +60,7 @@ __global__ void k_pack_boxes(const float* raw, int n, const int* orig_of_new, fl
                              int* orig, int nmat, int* err) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
-  int o = orig_of_new ? orig_of_new[s] : s;
+  int o = source_index(orig_of_new, s, n, err);
   const float* r = raw + 7 * (size_t)o;
   out[2 * s] = make_float4(r[0], r[1], r[2], 0.0f);
   out[2 * s + 1] = make_float4(r[3], r[4], r[5], 0.0f);
@@ -63,7 +72,7 @@ __global__ void k_pack_affine(const float* raw, int n, const int* orig_of_new, f
                               float* nm, int* mat, int* orig, int nmat, int* err) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
-  int o = orig_of_new ? orig_of_new[s] : s;
+  int o = source_index(orig_of_new, s, n, err);
   const float* r = raw + 22 * (size_t)o;
   rows[3 * s] = make_float4(r[0], r[1], r[2], r[3]);
   rows[3 * s + 1] = make_float4(r[4], r[5], r[6], r[7]);
@@ -199,11 +208,15 @@ __device__ void write_child(float4* node, int c, int child, const float* bounds,
 }
 
 __global__ void k_convert_nodes(const float* bounds, const int* data, int n, int ref_count,
-                                const int* rank, int synth, float4* nodes, int* err) {
+                                const int* rank, int interior, int synth, float4* nodes, int* err) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int l = data[4 * (size_t)i];
   if (l < 0) return;
+  if ((unsigned)rank[i] >= (unsigned)interior) {
+    atomicOr(err, 4);
+    return;
+  }
   int r = data[4 * (size_t)i + 1];
   float4* node = nodes + 4 * (size_t)(synth + rank[i]);
   write_child(node, 0, l, bounds, data, rank, synth, n, ref_count, err);
@@ -413,7 +426,7 @@ rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* d, const rtb_bvh
   float4* nodes = (float4*)(A + o_nodes);
   if (has_bvh) {
     k_convert_nodes<<<blocks(node_count), 256, 0, sm>>>(d_nb, d_nd, node_count, ref_count, irank,
-                                                         synth, nodes, err);
+                                                         interior, synth, nodes, err);
     k_top_nodes<<<1, 32, 0, sm>>>(d_nb, d_nd, node_count, ref_count, irank, d_roots, root_count,
                                   synth, nodes, err);
     cudaMemcpyAsync(A + o_rnb, d_nb, (size_t)node_count * 24, cudaMemcpyDeviceToDevice, sm);
@@ -450,7 +463,7 @@ rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* d, const rtb_bvh
       }
     }
     // A permutation needs every primitive referenced exactly once (no duplicates), as a builder
-    // does.
+    // does; a builder's tree is refused below if one is not.
     permute = built || (!(herr & 2) && ref_count == nbounded);
     if (permute) {
       // One scan over the four types' flags, one type after the other: a reference's sum is its
@@ -505,7 +518,12 @@ rtb_status scene_create(rtb_context* ctx, const rtb_scene_desc* d, const rtb_bvh
   }
   if (herr & (1 | 4 | 8)) {
     scene_free(s, sm);
-    return fail(ctx, RTB_ERR_INVALID_ARGUMENT, "BVH arrays failed the device range checks");
+    return fail(ctx, built ? RTB_ERR_DEVICE_CHECK : RTB_ERR_INVALID_ARGUMENT,
+                "BVH arrays failed the device range checks");
+  }
+  if (built && (herr & 2)) {
+    scene_free(s, sm);
+    return fail(ctx, RTB_ERR_DEVICE_CHECK, "a built BVH references a primitive twice");
   }
   if (herr & 16) {
     scene_free(s, sm);
