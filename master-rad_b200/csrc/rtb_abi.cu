@@ -1,7 +1,6 @@
 // The C ABI (include/rtb200.h): contexts, scene residency, render and replay entry points.
 // Every entry point locks the context, makes its device current and returns a status;
 // errors carry a message retrievable with rtb_last_error.
-#include <algorithm>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
@@ -9,10 +8,6 @@
 #include "rtb_internal.h"
 
 namespace rtb {
-
-// Results up to this size come back by way of pinned staging: a 64x36 image (28 KB) or 4,000
-// rays; beyond it the second copy costs what the first saves.
-constexpr size_t kPinnedCopyBytes = 256 << 10;
 
 rtb_status fail(rtb_context* ctx, rtb_status s, const std::string& msg) {
   if (ctx) ctx->last_error = msg;
@@ -31,21 +26,20 @@ void* stage(rtb_context* ctx, size_t bytes) {
     ctx->d_stage = nullptr;
     ctx->stage_bytes = 0;
     size_t want = bytes + bytes / 4 + 4096;
-    if (cudaMalloc(&ctx->d_stage, want) != cudaSuccess) return nullptr;
+    if (cudaMalloc(&ctx->d_stage, want) != cudaSuccess) {
+      cudaGetLastError();
+      ctx->d_stage = nullptr;
+      return nullptr;
+    }
     ctx->stage_bytes = want;
   }
   return ctx->d_stage;
 }
 
-void* pinned(rtb_context* ctx, size_t bytes) {
-  bytes = std::max(bytes, kPinnedCopyBytes);  // one allocation serves a context's small uses
-  if (bytes > ctx->pinned_bytes) {
-    cudaStreamSynchronize(ctx->stream);
-    cudaFreeHost(ctx->h_pinned);
+void* pinned(rtb_context* ctx) {
+  if (!ctx->h_pinned && cudaMallocHost(&ctx->h_pinned, kPinnedBytes) != cudaSuccess) {
+    cudaGetLastError();  // the next launch's check is not about this
     ctx->h_pinned = nullptr;
-    ctx->pinned_bytes = 0;
-    if (cudaMallocHost(&ctx->h_pinned, bytes) != cudaSuccess) return nullptr;
-    ctx->pinned_bytes = bytes;
   }
   return ctx->h_pinned;
 }
@@ -308,7 +302,7 @@ rtb_status rtb_trace_replay(rtb_context* ctx, rtb_scene* scene, const float* ray
   // Few rays go through pinned staging, one copy each way: a copy to or from pageable memory
   // costs some 10 us of its own, and there are six.
   const size_t rays_bytes = al(n * 24), hits_bytes = bytes - rays_bytes;
-  char* host = bytes <= kPinnedCopyBytes ? (char*)pinned(ctx, kPinnedCopyBytes) : nullptr;
+  char* host = bytes <= kPinnedBytes ? (char*)pinned(ctx) : nullptr;
   cudaStream_t sm = ctx->stream;
   ctx_acquire(ctx, sm);
   if (host) memcpy(host, rays, n * 24);
@@ -392,23 +386,26 @@ rtb_status rtb_render_sample(rtb_context* ctx, rtb_scene* scene, const rtb_camer
   size_t bytes = (size_t)params->width * params->height * 12;
   float* d_rgb = (float*)stage(ctx, bytes);
   if (!d_rgb) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "output staging");
+  // The stopped word and a small image come back by way of pinned staging in the frame's own
+  // stream, behind it, so that the host waits once; a large image is copied in place.  Taken before
+  // the launch: allocated behind a running frame it would hold up an abort request.
+  char* host = (char*)pinned(ctx);
+  const bool small = host && bytes <= kPinnedBytes - 256;
   cudaStream_t sm = ctx->stream;
   ctx_acquire(ctx, sm);
   arm_abort(ctx, sm, true);
   rtb_status s = render_frame(ctx, scene, camera, params, d_rgb, sm, true);
   ctx_release(ctx, sm);
   if (s != RTB_OK) return s;
-  // The stopped word and a small image come back by way of pinned staging in the frame's own
-  // stream, behind it, so that the host waits once; a large image is copied in place.
-  char* host = (char*)pinned(ctx, kPinnedCopyBytes);
-  const bool small = host && bytes <= kPinnedCopyBytes - 256;
   int aborted = 0;  // abort word [2]: the kernel stopped fetching work
-  cudaMemcpyAsync(host ? (int*)host : &aborted, ctx->d_abort + 2, sizeof(int), cudaMemcpyDeviceToHost, sm);
+  if (host) cudaMemcpyAsync(host, ctx->d_abort + 2, sizeof(int), cudaMemcpyDeviceToHost, sm);
   if (small) cudaMemcpyAsync(host + 256, d_rgb, bytes, cudaMemcpyDeviceToHost, sm);
   cudaError_t e = cudaEventSynchronize(ctx->ev1);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "render");
   auto tc = Clock::now();
-  if (!small) e = cudaMemcpyAsync(rgb, d_rgb, bytes, cudaMemcpyDeviceToHost, sm);
+  // not before the frame is done: a copy to pageable memory waits inside the driver
+  if (!host) e = cudaMemcpyAsync(&aborted, ctx->d_abort + 2, sizeof(int), cudaMemcpyDeviceToHost, sm);
+  if (e == cudaSuccess && !small) e = cudaMemcpyAsync(rgb, d_rgb, bytes, cudaMemcpyDeviceToHost, sm);
   if (e == cudaSuccess) e = cudaStreamSynchronize(sm);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "image read-back");
   if (small) memcpy(rgb, host + 256, bytes);

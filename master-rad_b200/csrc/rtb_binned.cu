@@ -839,8 +839,8 @@ rtb_status build_bvh_binned(rtb_context* ctx, const rtb_scene_desc* desc, const 
     Round round;
     int counters[8];
   };
-  Back* back = (Back*)pinned(ctx, sizeof(Back));
-  if (!back) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "pinned staging");
+  Back local;
+  Back* back = landing(ctx, local);
   back->round = h_round;
   int k = (int)h_active.size(), level = 0;
   while (k > 0) {

@@ -1508,8 +1508,10 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
   int k = (int)h_big.size(), level = 0, total_nodes = roots;
   const dim3 seg_grid(nc, 3), carry_grid(3, 2), axes_grid(blocks(n), 3);
   k_clear_winners<<<1, 32, 0, sm>>>(win, roots);
-  int* round = (int*)pinned(ctx, 2 * sizeof(int));  // next round's nodes, failed nodes
-  if (!round) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "pinned staging");
+  struct Round {
+    int next, failed;  // next round's nodes, this round's failed ones
+  } local;
+  Round* round = landing(ctx, local);
   while (k > 0) {
     // Every node of the level loop holds more than kSubtreeSize primitives
     // (smaller ones go to k_subtrees), so with non-unit weights all of them take the certified
@@ -1563,10 +1565,10 @@ rtb_status build_bvh_options(rtb_context* ctx, const rtb_scene_desc* desc, const
       for (int a = 0; a < 3; ++a) std::swap(I.a[a], T.a[a]);
       std::swap(key, key2);
     }
-    cudaMemcpyAsync(round, lists, 2 * sizeof(int), cudaMemcpyDeviceToHost, sm);
+    cudaMemcpyAsync(round, lists, sizeof(Round), cudaMemcpyDeviceToHost, sm);
     cudaError_t e = cudaStreamSynchronize(sm);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "BVH build level");
-    const int next = round[0], nfail = round[1];
+    const int next = round->next, nfail = round->failed;
     if (nfail > 0) {
       for (int a = 0; a < 3; ++a)
         k_gather_weights<<<blocks(n), 256, 0, sm>>>(P, I.a[a], n, const_cast<double*>(chains.w[a]));

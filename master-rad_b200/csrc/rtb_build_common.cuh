@@ -353,6 +353,7 @@ struct Workspace {
   T* alloc(size_t n) {
     void* p = nullptr;
     if (cudaMallocAsync(&p, std::max<size_t>(n, 1) * sizeof(T), stream) != cudaSuccess) {
+      cudaGetLastError();
       ok = false;
       return nullptr;
     }
@@ -505,8 +506,8 @@ inline rtb_status finish_build(rtb_context* ctx, const rtb_scene_desc* desc, con
     int stats[4];
     BuildResult result;
   };
-  Back* back = (Back*)pinned(ctx, sizeof(Back));
-  if (!back) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "pinned staging");
+  Back local;
+  Back* back = landing(ctx, local);
   cudaMemcpyAsync(back->stats, counters + 2, sizeof(back->stats), cudaMemcpyDeviceToHost, sm);
   cudaMemcpyAsync(&back->result, o_result, sizeof(BuildResult), cudaMemcpyDeviceToHost, sm);
   BuiltTree tree{o_nb, o_nd, total_nodes, o_refs, n, o_roots, roots, o_rank, (total_nodes - roots) / 2, in.sph, in.box};

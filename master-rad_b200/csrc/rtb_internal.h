@@ -36,8 +36,7 @@ struct rtb_context {
   // Replay / output staging reused across calls.
   void* d_stage = nullptr;
   size_t stage_bytes = 0;
-  void* h_pinned = nullptr;
-  size_t pinned_bytes = 0;
+  void* h_pinned = nullptr;  // kPinnedBytes, see pinned()
   // Per-sample radiance of the frame's last pixels (rendered one sample per lane).
   float* d_tail = nullptr;
   size_t tail_bytes = 0;
@@ -111,7 +110,20 @@ inline bool ctx_grow(T** buf, size_t* have, size_t want, cudaStream_t stream) {
 
 // Device staging buffer of at least `bytes` (grown on demand, owned by the context).
 void* stage(rtb_context* ctx, size_t bytes);
-void* pinned(rtb_context* ctx, size_t bytes);
+
+// Results up to this size come back by way of pinned staging: a 64x36 image (28 KB) or 4,000
+// rays; beyond it the second copy costs what the first saves.
+constexpr size_t kPinnedBytes = 256 << 10;
+// kPinnedBytes of page-locked memory for a context's small copies, one at a time.  Null where
+// there is none; every caller can do without.
+void* pinned(rtb_context* ctx);
+// Where a small result lands: page-locked, so that its copy does not stop the host, or `local`.
+template <typename T>
+inline T* landing(rtb_context* ctx, T& local) {
+  static_assert(sizeof(T) <= kPinnedBytes, "a small result");
+  T* p = (T*)pinned(ctx);
+  return p ? p : &local;
+}
 
 // rtb_scene.cu
 // A tree that a builder made on the device, in the reference's flattened layout, with what the
