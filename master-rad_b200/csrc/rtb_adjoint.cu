@@ -486,11 +486,15 @@ rtb_status rtb_render_backward_sample(rtb_context* ctx, rtb_scene* scene, const 
   ctx_release(ctx, sm);
   rtb_status s = render_backward(ctx, scene, cam, p, d_adj, d_ga, d_ge, sm);
   if (s != RTB_OK) return s;
+  // Not before the replay is done: a copy to pageable memory waits inside the driver, where it
+  // holds up an abort request from another thread.
+  cudaError_t e = cudaEventSynchronize(ctx->ev1);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "adjoint");
   ctx_acquire(ctx, sm);
   cudaMemcpyAsync(grad_albedo, d_ga, grads, cudaMemcpyDeviceToHost, sm);
   cudaMemcpyAsync(grad_emission, d_ge, grads, cudaMemcpyDeviceToHost, sm);
   ctx_release(ctx, sm);
-  cudaError_t e = cudaStreamSynchronize(sm);
+  e = cudaStreamSynchronize(sm);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "adjoint");
   int aborted = 0;
   cudaMemcpy(&aborted, ctx->d_abort + 2, sizeof(int), cudaMemcpyDeviceToHost);

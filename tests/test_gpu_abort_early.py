@@ -1,6 +1,6 @@
 """An abort stops a frame at a small fraction of its time, on the frame kernel in phases: also
-the first frame of a context, whose buffers and code are not there yet.  The unaborted
-time is taken from frames of fewer samples on the same device, so that the bound
+the first frame of a context, whose buffers and code are not there yet, and a replay's.  The
+unaborted time is taken from frames of fewer samples on the same device, so that the bound
 follows the kernel's speed."""
 import ctypes as C
 import threading
@@ -15,7 +15,7 @@ from rtb200 import synth
 from rtb200.tracer import Context, ResidentScene, camera_struct
 
 pytestmark = pytest.mark.gpu
-SPP = 2048  # some six seconds at 1024 x 1024
+SPP = 2048  # some six seconds at 1024 x 1024, a replay nine
 
 
 def _params(w, spp, frame):
@@ -27,6 +27,17 @@ def _frame(ctx, res, w, spp, frame=1):
     cam = camera_struct(w.camera)
     t = time.perf_counter()
     st = ctx.lib.rtb_render_sample(ctx.handle, res.handle, C.byref(cam), C.byref(_params(w, spp, frame)), N.fptr(img))
+    return st, time.perf_counter() - t
+
+
+def _backward(ctx, res, w, spp):
+    pixels = w.width * w.height
+    adj = np.ones(3 * pixels, np.float32)
+    grads = [np.zeros(3 * w.scene.material_count(), np.float32) for _ in range(2)]
+    cam = camera_struct(w.camera)
+    t = time.perf_counter()
+    st = ctx.lib.rtb_render_backward_sample(ctx.handle, res.handle, C.byref(cam), C.byref(_params(w, spp, 1)),
+                                            N.fptr(adj), N.fptr(grads[0]), N.fptr(grads[1]))
     return st, time.perf_counter() - t
 
 
@@ -46,7 +57,8 @@ def workload():
 
 
 @pytest.mark.parametrize("first", [True, False])
-def test_abort_stops_early(workload, first, call=_frame):
+@pytest.mark.parametrize("call", [_frame, _backward])
+def test_abort_stops_early(workload, first, call):
     w, bvh = workload
     ctx = Context(0)
     try:
