@@ -36,6 +36,20 @@ void* stage(rtb_context* ctx, size_t bytes) {
   return ctx->d_stage;
 }
 
+bool ctx_grow_paths(rtb_context* ctx, size_t want, cudaStream_t stream) {
+  if (want <= ctx->path_bytes) return true;
+  if (ctx->d_paths) cudaFreeAsync(ctx->d_paths, stream);
+  ctx->d_paths = nullptr;
+  ctx->path_bytes = 0;
+  if (cudaMallocAsync(&ctx->d_paths, want, stream) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->d_paths = nullptr;
+    return false;
+  }
+  ctx->path_bytes = want;
+  return true;
+}
+
 // Page-locked memory comes from the driver in larger pieces, and the first block of one costs 1 to
 // 3 ms, another 2 us, and the last one's return 0.4 ms and more.  So one byte of it stays, unused,
 // for the life of the process: a context's first build takes 3.7 ms without it where no other
@@ -174,12 +188,15 @@ rtb_status rtb_context_destroy(rtb_context* ctx) {
   {
     std::lock_guard<std::mutex> lock(ctx->mu);
     cudaSetDevice(ctx->device);
+    if (ctx->stream && ctx->d_paths) {
+      ctx_acquire(ctx, ctx->stream);  // frames on the caller's streams
+      cudaFreeAsync(ctx->d_paths, ctx->stream);
+    }
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->d_work);
     cudaFree(ctx->d_abort);
     cudaFree(ctx->d_stage);
     cudaFree(ctx->d_tail);
-    cudaFree(ctx->d_paths);
     cudaFree(ctx->d_wave);
     cudaFreeHost(ctx->h_pinned);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);

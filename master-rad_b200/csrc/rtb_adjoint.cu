@@ -424,7 +424,7 @@ static rtb_status render_backward(rtb_context* ctx, rtb_scene* scene, const rtb_
   if (phases) {
     const ReplayShape shape(a.samples, a.r.max_depth, ctx->sm_count);
     // without the memory, one path a lane
-    phases = ctx_grow(&ctx->d_paths, &ctx->path_bytes, shape.path_bytes + shape.vertex_bytes, sm);
+    phases = ctx_grow_paths(ctx, shape.path_bytes + shape.vertex_bytes, sm);
     if (phases) {
       grid = shape.grid;
       a.r.slots = shape.slots;

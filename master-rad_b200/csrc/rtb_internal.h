@@ -40,7 +40,7 @@ struct rtb_context {
   // Per-sample radiance of the frame's last pixels (rendered one sample per lane).
   float* d_tail = nullptr;
   size_t tail_bytes = 0;
-  // Path slots of the frame kernel's blocks.
+  // Path slots of the frame kernel's blocks, from the device's pool (ctx_grow_paths).
   void* d_paths = nullptr;
   size_t path_bytes = 0;
   // Path state of the wavefront form, grown to the largest frame rendered in that form.
@@ -107,6 +107,13 @@ inline bool ctx_grow(T** buf, size_t* have, size_t want, cudaStream_t stream) {
   *have = want;
   return true;
 }
+
+// Grows the path slots, in `stream`'s order between ctx_acquire and ctx_release.  They come from
+// the pool that the builders use, up to 94.6 MB for frames and 256 MB more for a replay: every new
+// context's first frame or replay asks for them, and cudaMalloc and cudaFree of so much take
+// 0.4 to 1 ms, now and then 5, and wait for the device (a rank's rows, a context's first call
+// 4.7 to 6.9 -> 3.8 ms, its second 3.1).
+bool ctx_grow_paths(rtb_context* ctx, size_t want, cudaStream_t stream);
 
 // Device staging buffer of at least `bytes` (grown on demand, owned by the context).
 void* stage(rtb_context* ctx, size_t bytes);

@@ -570,7 +570,7 @@ rtb_status render_frame(rtb_context* ctx, rtb_scene* scene, const rtb_camera* ca
   if (s != RTB_OK) return s;
   settle_frame(
       f.shape, [&](size_t bytes) { return ctx_grow(&ctx->d_tail, &ctx->tail_bytes, bytes, stream); },
-      [&](size_t bytes) { return ctx_grow(&ctx->d_paths, &ctx->path_bytes, bytes, stream); },
+      [&](size_t bytes) { return ctx_grow_paths(ctx, bytes, stream); },
       [&] { return resident_threads(ctx, &f, kSmallBlock); });
   bind_frame(&f, ctx->d_work, ctx->d_tail, ctx->d_paths, ctx->d_abort, ctx->d_work + 8);
   if (timed) cudaEventRecord(ctx->ev0, stream);
