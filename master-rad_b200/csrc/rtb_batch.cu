@@ -492,9 +492,15 @@ rtb_status upload_jobs(rtb_context* ctx, rtb_batch* B) {
   return RTB_OK;
 }
 
-void release_batch(rtb_batch* B) {
+void drop_graph(rtb_batch* B) {
   if (B->exec) cudaGraphExecDestroy(B->exec);
   if (B->graph) cudaGraphDestroy(B->graph);
+  B->exec = nullptr;
+  B->graph = nullptr;
+}
+
+void release_batch(rtb_batch* B) {
+  drop_graph(B);
   free_frames(B);
   cudaFree(B->d_jobs);
   cudaFree(B->d_tail);
@@ -509,10 +515,7 @@ void release_batch(rtb_batch* B) {
 }
 
 rtb_status capture(rtb_context* ctx, rtb_batch* B) {
-  if (B->exec) cudaGraphExecDestroy(B->exec);
-  if (B->graph) cudaGraphDestroy(B->graph);
-  B->exec = nullptr;
-  B->graph = nullptr;
+  drop_graph(B);
   cudaStream_t sm = ctx->stream;
   cudaError_t e = cudaStreamBeginCapture(sm, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "batch graph capture");
@@ -593,6 +596,7 @@ rtb_status rtb_batch_render(rtb_context* ctx, rtb_batch* B, void* stream) {
   if (!ctx || !B) return RTB_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(ctx->mu);
   cudaSetDevice(ctx->device);
+  if (!B->exec) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "the batch lost its buffers in rtb_batch_autotune");
   cudaStream_t sm = stream ? (cudaStream_t)stream : ctx->stream;
   ctx_acquire(ctx, sm);
   arm_abort(ctx, sm);  // outside the graph: its kernels read the words, never write [1]
@@ -671,6 +675,7 @@ rtb_status rtb_batch_autotune(rtb_context* ctx, rtb_batch* B, int repeats, rtb_b
   }
   ctx_release(ctx, sm);
   B->tuning = pick;
+  drop_graph(B);  // it names buffers that the trials may have replaced
   rtb_status s2 = upload_jobs(ctx, B);
   if (s2 == RTB_OK) s2 = capture(ctx, B);
   if (s != RTB_OK) return s;
