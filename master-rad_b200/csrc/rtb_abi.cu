@@ -15,6 +15,7 @@ rtb_status fail(rtb_context* ctx, rtb_status s, const std::string& msg) {
 }
 
 rtb_status cuda_fail(rtb_context* ctx, cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here; the next launch's check is not about it
   if (ctx) ctx->last_error = std::string(what) + ": " + cudaGetErrorString(e);
   return e == cudaErrorMemoryAllocation ? RTB_ERR_OUT_OF_MEMORY : RTB_ERR_CUDA;
 }
