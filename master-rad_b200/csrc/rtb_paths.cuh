@@ -142,7 +142,7 @@ __device__ __forceinline__ bool shade_segment(const DevScene& S, bool hit, const
 }
 
 // The camera ray of sample `so` of pixel (x, y) and its random stream (renderKernel
-// prologue, K:1251-1264), for the wavefront kernels (k_render's prologue is inline).
+// prologue, K:1251-1264), for every form of the frame and the replay.
 __device__ __forceinline__ void camera_sample(const RenderArgs& a, int x, int y, int so, uint32_t& rng,
                                               float3& o, float3& d) {
   uint32_t seed = pixel_base_seed(a.frame_hash, (uint32_t)y * (uint32_t)a.width + (uint32_t)x) ^ hash_u32((uint32_t)so);
@@ -224,13 +224,20 @@ __device__ __forceinline__ void start_sample(const RenderArgs& a, long long pixe
 // deep 6.21 / 4.56; but 300 mixed primitives 512x512, 16 spp 2.90 / 3.68, 10k 256x256 at 4 spp
 // 1.121 / 1.125, 8 spp 1.75 / 1.97.  So the phases take frames of kPhaseItems samples per
 // resident thread over a tree of kPhaseNodes nodes, and paths of kPhaseDepth segments: camera rays
-// walk the tree together as neighbours and gain nothing from being taken singly (segments 1 / 2 /
-// 3 / 4 deep, phases / lanes, ms: 120k primitives 1834x219, 6 spp 0.50 / 0.30, 1.38 / 1.46, 2.38 /
-// 2.96, 3.38 / 4.46; 10k 1024x1024, 4 spp 1.20 / 0.93, 2.73 / 2.26, 4.24 / 3.99, 5.77 / 5.90; 1M
-// 2 spp 1.64 / 1.24, 3.35 / 2.82, 5.00 / 4.61, 6.60 / 6.40).  The form before this walk took
-// 0.35 and 1.74 ms for the first one's one and two segments.  Refilling only whole warps in
-// phases of mostly camera rays took back between none and four tenths of the difference at one
-// segment (0.51, 1.10, 1.60) and cost 1 % at depth 8.
+// walk the tree together as neighbours and gain nothing from being taken singly.  Three segments
+// is where the forms meet.  Phases' time over lanes', 15 whole frames (300 to 1M primitives,
+// 400x401 to 1024x1024, 1 / 4 / 16 spp) and 12 ranks' rows of 10k and 120k primitives:
+//
+//   segments        2                 3                 4              5
+//   whole frames    1.00-1.25         0.95-1.11         0.90-1.07      0.84-1.02
+//   rows            0.96-1.29         0.82-1.10         0.76-1.02      -
+//   at 3, by samples a pixel (means): 1 spp 1.05, 4 spp 1.05, 16 spp 1.00; rows 0.99
+//
+// Wide frames, whose camera rays are far apart (1834x219: 0.82 and 0.87), gain most at three, square
+// ones of few samples lose most (10k 1024x1024, 1 spp: 1.22 / 1.10 ms), so neither side of the line
+// has three segments to itself; from three on both are faster than the form before this walk in
+// every cell.  Refilling only whole warps in phases of mostly camera rays took back between none and
+// four tenths of the difference at one segment and cost 1 % at depth 8.
 constexpr int kPhaseItems = 2, kPhaseNodes = 64, kPhaseDepth = 3;
 constexpr int kRefillLanes = 8;    // 4 and 12 within 1 %
 constexpr int kPoolLeafLanes = 8;  // 4 and 12 within 1 %
