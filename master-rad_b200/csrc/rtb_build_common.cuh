@@ -64,7 +64,9 @@ __device__ __forceinline__ float o2f(unsigned o) {
 }
 
 struct Prims {
-  Box* box;          // bounds, one 24-byte record per primitive (gathers)
+  float* lo[3];
+  float* hi[3];
+  Box* box;          // the same bounds, one 24-byte record per primitive (gathers)
   double* cen[3];
   double* w;         // construction weight q = 1 + lambda (c - 1), or 1
   double* measured;  // c
@@ -114,6 +116,8 @@ __global__ void k_prims(const float* spheres, const float* boxes, const float* a
   }
   Box bx;
   for (int k = 0; k < 3; ++k) {
+    P.lo[k][p] = lo[k];
+    P.hi[k][p] = hi[k];
     P.cen[k][p] = ((double)lo[k] + (double)hi[k]) * 0.5;
     bx.mn[k] = lo[k];
     bx.mx[k] = hi[k];
@@ -402,6 +406,8 @@ inline rtb_status build_setup(rtb_context* ctx, const rtb_scene_desc* desc, cons
 inline Prims alloc_prims(Workspace& W, int n) {
   Prims P;
   for (int k = 0; k < 3; ++k) {
+    P.lo[k] = W.alloc<float>(n);
+    P.hi[k] = W.alloc<float>(n);
     P.cen[k] = W.alloc<double>(n);
   }
   P.box = W.alloc<Box>(n);

@@ -455,20 +455,16 @@ rtb_status build_bvh_sbvh(rtb_context* ctx, const rtb_scene_desc* desc, const rt
     Prims P = alloc_prims(W, n);
     if (!W.ok) return fail(ctx, RTB_ERR_OUT_OF_MEMORY, "SBVH primitive bounds");
     upload_prims(desc, c, in, P, sm);
-    std::vector<Box> box(n);
-    cudaMemcpyAsync(box.data(), P.box, (size_t)n * sizeof(Box), cudaMemcpyDeviceToHost, sm);
+    for (int k = 0; k < 3; ++k) {
+      lo[k].resize(n);
+      hi[k].resize(n);
+      cudaMemcpyAsync(lo[k].data(), P.lo[k], (size_t)n * 4, cudaMemcpyDeviceToHost, sm);
+      cudaMemcpyAsync(hi[k].data(), P.hi[k], (size_t)n * 4, cudaMemcpyDeviceToHost, sm);
+    }
     cudaMemcpyAsync(refs.data(), P.ref, (size_t)n * 4, cudaMemcpyDeviceToHost, sm);
     cudaMemcpyAsync(types.data(), P.type, (size_t)n * 4, cudaMemcpyDeviceToHost, sm);
     cudaError_t e = cudaStreamSynchronize(sm);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "SBVH primitive bounds");
-    for (int k = 0; k < 3; ++k) {
-      lo[k].resize(n);
-      hi[k].resize(n);
-      for (int i = 0; i < n; ++i) {
-        lo[k][i] = box[i].mn[k];
-        hi[k][i] = box[i].mx[k];
-      }
-    }
   }
   double w[4], measured[4];
   for (int t = 0; t < 4; ++t) {
