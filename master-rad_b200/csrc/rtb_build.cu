@@ -642,14 +642,14 @@ __global__ void k_certify(const Nodes N, const int* key, const int* level_of, in
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const int a = blockIdx.y, node = key[j];
-  if (level_of[node] != level || C.seq[node] || W.cost[node] == CUDART_INF) return;
-  const double c = C.cost[a][j];
-  if (c == CUDART_INF) return;
+  if (level_of[node] != level || C.seq[node]) return;
+  const double c = C.cost[a][j], best = W.cost[node];
+  if (c == CUDART_INF || best == CUDART_INF) return;
   const int s = N.start[node], len = N.end[node] - s;
   const long long flat = W.flat[node];
   if ((long long)a * len + (j - s) == flat) return;
   const int wa = (int)(flat / len), wp = (int)(flat - (long long)wa * len);
-  if (c - C.bound[a][j] <= W.cost[node] + C.bound[wa][s + wp] && atomicExch(W.failed + node, 1) == 0)
+  if (c - C.bound[a][j] <= best + C.bound[wa][s + wp] && atomicExch(W.failed + node, 1) == 0)
     list[atomicAdd(count, 1)] = node;
 }
 
